@@ -172,6 +172,8 @@ class _State:
         self.__dict__.update(kw)
 
     def __del__(self):
+        if torch is None:  # the interpreter is shutting down
+            return
         # an lhs is freed before the context it borrows from
         for k in ("F", "ms", "elm"):
             obj = self.__dict__.get(k)
