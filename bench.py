@@ -65,10 +65,12 @@ REFINE_TOL = 0.0      # mixed precision: FP64 defect target (0: the NSSOLVER tol
 TRAFFIC_PER_ALG_F32 = 0.765
 TRAFFIC_PER_ALG_F64 = 0.850
 TRAFFIC_SOURCE = "ncu --set full, k_cg_persistent, 2.07M-tet cylinder, 50 iterations/launch, scaled by blocks"
-# The same ratio for the CG on the explicit FP32 Schur operator (k_cg_schur);
-# 1.0 until an ncu capture of that kernel replaces it.
-TRAFFIC_PER_ALG_S2 = 1.0
-TRAFFIC_SOURCE_S2 = "not yet captured: algorithmic bytes"
+# The same ratio for the CG on the explicit Schur operator (k_cg_schur), from
+# captures of the same case: FP32 142.7 MB per iteration of 158.0 algorithmic,
+# FP64 236 MB of 249.
+TRAFFIC_PER_ALG_S2 = 0.90
+TRAFFIC_PER_ALG_S2_F64 = 0.95
+TRAFFIC_SOURCE_S2 = "ncu, k_cg_schur, 2.11M-tet cylinder, 50 iterations/launch, scaled by entries"
 
 
 def _inflow(t: float) -> float:
@@ -350,14 +352,13 @@ def cg_iter_bytes(nnz: int, n: int, mbytes: int, nface: int, resident: bool = Fa
     return nnz * ((0 if resident else 8) + 7 * mbytes) + n * (16 + 8 * mbytes + 24 + 16 + 16 + 16 + 16 * nface)
 
 
-def cg_schur_iter_bytes(nnz2: int, n: int, nface: int) -> int:
-    """Algorithmic HBM bytes of one iteration of the CG on the explicit FP32
-    Schur operator: per 2-ring entry the FP32 value and its int16 column
-    offset (6); per row, once: {R, P_prev} FP64 read in both phases and
-    written (3 x 16), its FP32 copy written and gathered (2 x 8), S P written
-    and read (2 x 8), X read and written (16), and w_f, z_f (phase 1) and z_f
-    (phase 2) per coupled face (3 x 8)."""
-    return nnz2 * 6 + n * (48 + 16 + 16 + 16 + 24 * nface)
+def cg_schur_iter_bytes(nnz2: int, n: int, nface: int, mbytes: int) -> int:
+    """Algorithmic HBM bytes of one iteration of the CG on the explicit Schur
+    operator: per 2-ring entry the value (mbytes) and its int16 column offset
+    (2); per row, once: R gathered, read and written (3 x 8), P and S P read
+    and written in phase 1 and read in phase 2 (6 x 8), X read and written
+    (16), and w_f, z_f (phase 1) and z_f (phase 2) per coupled face (3 x 8)."""
+    return nnz2 * (mbytes + 2) + n * (24 + 48 + 16 + 24 * nface)
 
 
 def run_ours(args):
@@ -472,19 +473,22 @@ def run_ours(args):
     nface = len(P.rcr)
     res64, res32, rbytes = ctypes.c_int(), ctypes.c_int(), ctypes.c_longlong()
     N.check(L.crimson_memls_cg_layout(F64.memls.lhs, ctypes.byref(res64), None, None), "crimson_memls_cg_layout")
-    if L.crimson_memls_cg_layout(FM.memls.lhs, None, ctypes.byref(res32), ctypes.byref(rbytes)) != 0:
-        res32.value = 0   # the mixed solve ran only the explicit-Schur CG
-    s2_state, s2_nnz, s2_npad, s2_form_ms = FM.memls.schur_info()
-    if s2_state == 1:
-        cg_bytes = cg_schur_iter_bytes(s2_nnz, n, nface)
-        cg_kernel = ("k_cg_schur<1> (one CGRAD iteration on the explicit FP32 Schur operator: S P, "
+    N.check(L.crimson_memls_cg_layout(FM.memls.lhs, None, ctypes.byref(res32), ctypes.byref(rbytes)), "crimson_memls_cg_layout")
+    s2_nnz, s2_npad, s2_form_ms = FM.memls.schur_info()[1:]
+    if s2_nnz:
+        cg_bytes = cg_schur_iter_bytes(s2_nnz, n, nface, 4)
+        cg_kernel = ("k_cg_schur<float> (one CGRAD iteration on the explicit FP32 Schur operator: S R, "
                      "coupled-face term, updates)")
     else:
         cg_bytes = cg_iter_bytes(nnz, n, 4, nface, bool(res32.value))
         cg_kernel = "k_cg_persistent<float> (one CGRAD iteration: G P, L P - Gt G P, updates)"
+    s2_nnz64 = F64.memls.schur_info()[1]
+    cg_bytes64 = (cg_schur_iter_bytes(s2_nnz64, n, nface, 8) if s2_nnz64 else
+                  cg_iter_bytes(nnz, n, 8, nface, bool(res64.value)))
     achieved = cg_bytes / (kt["cg_iter_f32"] / 1e3) / 1e9 if kt["cg_iter_f32"] else None
-    cg_bytes64 = cg_iter_bytes(nnz, n, 8, nface, bool(res64.value))
     achieved64 = cg_bytes64 / (kt["cg_iter_f64"] / 1e3) / 1e9 if kt["cg_iter_f64"] else None
+    traffic_f32 = TRAFFIC_PER_ALG_S2 if s2_nnz else TRAFFIC_PER_ALG_F32
+    traffic_f64 = TRAFFIC_PER_ALG_S2_F64 if s2_nnz64 else TRAFFIC_PER_ALG_F64
     line = {
         "metric": METRIC, "value": value, "unit": "s/timestep", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": tm_ms / args.steps, "higher_is_better": False, "scaling": "weak",
@@ -494,7 +498,7 @@ def run_ours(args):
                    "parallelism": "replicas" if ws > 1 else "single GPU",
                    "epstol_ns": P.epstol_ns, "epstol_gmres_cg": [P.epstol_mom, P.epstol_cont],
                    "mixed_refine_tol": Pm.refine_tol if Pm.refine_tol > 0 else P.epstol_ns,
-                   "l2": "inputs larger than L2 (sliced FP32 matrices 0.66 GB, FP64 1.33 GB per solve)"},
+                   "l2": "inputs larger than L2 (sliced FP32 matrices 0.66 GB, FP64 K and Schur operator 1.2 GB per solve)"},
         "fp64": {"value": v64, "unit": "s/timestep", "ms_per_step": t64_ms / args.steps,
                  "e2e": {"value": e2e64, "unit": "s/timestep", "h2d_bytes_per_step": 2 * 4 * n * 8,
                          "d2h_bytes_per_step": 2 * 4 * n * 8},
@@ -509,16 +513,16 @@ def run_ours(args):
         "roofline": {"kernel": cg_kernel,
                      "bound": "hbm", "achieved": achieved, "peak": peaks[0], "unit": "GB/s",
                      "frac": achieved / peaks[0] if achieved else None,
-                     "traffic": (TRAFFIC_PER_ALG_S2 if s2_state == 1 else TRAFFIC_PER_ALG_F32) * cg_bytes,
-                     "traffic_source": TRAFFIC_SOURCE_S2 if s2_state == 1 else TRAFFIC_SOURCE,
+                     "traffic": traffic_f32 * cg_bytes,
+                     "traffic_source": TRAFFIC_SOURCE_S2 if s2_nnz else TRAFFIC_SOURCE,
                      "algorithmic_bytes_per_iter": cg_bytes, "peak_source": peaks[1],
-                     "schur_operator": {"state": s2_state, "nnz": s2_nnz, "sliced_positions": s2_npad,
+                     "schur_operator": {"nnz": s2_nnz, "sliced_positions": s2_npad,
                                         "formation_ms": s2_form_ms},
-                     "columns": ("int16 offsets streamed with the FP32 values" if s2_state == 1 else
+                     "columns": ("int16 offsets streamed with the FP32 values" if s2_nnz else
                                  ("block-resident in shared memory" if res32.value else "read per phase")),
                      "fp64_kernel": {"achieved": achieved64, "frac": achieved64 / peaks[0] if achieved64 else None,
                                      "algorithmic_bytes_per_iter": cg_bytes64,
-                                     "traffic": TRAFFIC_PER_ALG_F64 * cg_bytes64 if TRAFFIC_PER_ALG_F64 else None}},
+                                     "traffic": traffic_f64 * cg_bytes64}},
         "e2e": {"value": e2e, "unit": "s/timestep", "h2d_bytes_per_step": 2 * 4 * n * 8,
                 "d2h_bytes_per_step": 2 * 4 * n * 8},
         "gpu_launches": lm,

@@ -17,7 +17,8 @@
 // blocks per lane issued together; dot products and norms use a single-pass
 // grid reduction whose last block sums the per-block partials in a fixed
 // order (deterministic).  CGRAD runs as one persistent cooperative kernel per
-// call.  The Krylov control flow (Givens rotations, back substitution, the
+// call: in FP64 on the explicitly formed Schur operator (schur.cu) where the
+// pattern allows, else on the two-product kernel below.  The Krylov control flow (Givens rotations, back substitution, the
 // 2i x 2i Gram system solved by GE) runs on the host in FP64 on scalars
 // copied back per step, as the reference's serial code does.
 //
@@ -451,8 +452,8 @@ __global__ void k_max_offset(const int* __restrict__ rowptr, const int* __restri
 }
 
 // Scaled split matrices (CSR, type M) -> sliced copies: K as two 4-vector
-// arrays and one scalar array (npad each), G (3, npad) per component,
-// {Gt0, Gt1, Gt2, L} (npad).
+// arrays and one scalar array (npad each), and for the two-product CG (Gs not
+// null) G (3, npad) per component, {Gt0, Gt1, Gt2, L} (npad).
 template <typename M>
 __global__ void k_to_sell(const int* __restrict__ rowptr, const int* __restrict__ sp, int n,
                           const double* __restrict__ mK, const double* __restrict__ mG, const double* __restrict__ Gt,
@@ -469,6 +470,7 @@ __global__ void k_to_sell(const int* __restrict__ rowptr, const int* __restrict_
             reinterpret_cast<typename V4<M>::type*>(Ks + 4 * npad)[pos] =
                 mk4<M>((M)mK[9 * jj + 4], (M)mK[9 * jj + 5], (M)mK[9 * jj + 6], (M)mK[9 * jj + 7]);
             Ks[8 * npad + pos] = (M)mK[9 * jj + 8];
+            if (!Gs) continue;
 #pragma unroll
             for (int q = 0; q < 3; ++q) Gs[q * npad + pos] = (M)mG[3 * jj + q];
             GLs[pos] = mk4<M>((M)Gt[3 * jj], (M)Gt[3 * jj + 1], (M)Gt[3 * jj + 2], (M)mL[jj]);
@@ -477,7 +479,8 @@ __global__ void k_to_sell(const int* __restrict__ rowptr, const int* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// CGRAD as one persistent cooperative kernel (memLS.f90:367-430).
+// CGRAD as one persistent cooperative kernel (memLS.f90:367-430): the mixed
+// solve, and FP64 on patterns that the explicit operator (schur.cu) excludes.
 //
 // Per iteration three grid-wide barriers: (A) P = R + beta P formed on the
 // fly while computing GP = G P, plus the coupled-face dots w_f . P; (B)
@@ -1668,55 +1671,10 @@ static int cg_resident_bytes(crimson_lhs* L, size_t* bytes) {
     return CRIMSON_OK;
 }
 
-// CGRAD (memLS.f90:367-430) on the Schur-like operator L P - Gt G P; R in/out (n).
-// Gs / GLs: sliced G and {Gt, L} of this NSSOLVER call.
+// Launch form of the two-product CG kernel on this lhs (kernel family and
+// grid), decided once per precision.
 template <typename M>
-static int cgrad(Ctx& C, crimson_subls& ls, const M* Gs, const typename V4<M>::type* GLs,
-                 double* R, int nface,
-                 const double* coef, bool use_s2 = false) {
-    crimson_lhs* L = C.L;
-    cudaStream_t s = C.s;
-    const int n = L->nNo;
-    const double time = now_s();
-    ls.suc = 0;
-    C.dot((const double*)R, (const double*)R, n, kSlotErr);
-    CR_CHECK(C.sync_scal(kSlotErr, 1));
-    double errO = std::sqrt(L->hscal[kSlotErr]);
-    ls.iNorm = errO;
-    double eps = std::max(ls.absTol, ls.relTol * errO);
-    eps = eps * eps;
-    double err = errO;
-    err = err * err;
-    if (use_s2) {
-        // the same CGRAD on the explicit FP32 Schur operator (schur.cu)
-        CR_CUDA(cudaEventRecord(L->ev0, s));
-        CR_CHECK(cg_schur_launch(L, R, nface, coef, L->cgW.p, L->cgZ.p, eps, err, ls.mItr, C.sc(kSlotCg)));
-        CR_CUDA(cudaEventRecord(L->ev1, s));
-        CR_CHECK(C.sync_scal(kSlotCg, 4));
-        err = L->hscal[kSlotCg + 0];
-        errO = L->hscal[kSlotCg + 1];
-        const int i = (int)L->hscal[kSlotCg + 2];
-        ls.suc = (int)L->hscal[kSlotCg + 3];
-        float ms = 0.f;
-        CR_CUDA(cudaEventElapsedTime(&ms, L->ev0, L->ev1));
-        L->cg_acc32.ms += ms;
-        L->cg_acc32.iters += i - 1;
-        L->cg_acc32.launches += 1;
-        if (L->s2_form_pending) {
-            float fm = 0.f;
-            CR_CUDA(cudaEventElapsedTime(&fm, L->s2_ev0, L->s2_ev1));
-            L->s2_form_ms += fm;
-            L->s2_forms += 1;
-            L->s2_form_pending = false;
-        }
-        CR_CUDA(cudaMemcpyAsync(R, L->cgX.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-        CR_CUDA(cudaStreamSynchronize(s));
-        ls.fNorm = std::sqrt(err);
-        ls.callD = now_s() - time + ls.callD;
-        ls.dB = 5.0 * std::log(err / errO);
-        ls.itr = ls.itr + i - 1;
-        return CRIMSON_OK;
-    }
+static int cg_layout(crimson_lhs* L, size_t* rbytes_out) {
     const void* kres[3] = {(const void*)k_cg_persistent<0, M, true>, (const void*)k_cg_persistent<1, M, true>,
                            (const void*)k_cg_persistent<kMaxCoupled, M, true>};
     const void* kglb[3] = {(const void*)k_cg_persistent<0, M, false>, (const void*)k_cg_persistent<1, M, false>,
@@ -1752,13 +1710,91 @@ static int cgrad(Ctx& C, crimson_subls& ls, const M* Gs, const typename V4<M>::t
             grid = sm_count() * std::min(nb, 8);
         }
     }
+    *rbytes_out = rbytes;
+    return CRIMSON_OK;
+}
+
+// Diagnostics: what cg_layout decides for the precisions CGRAD has run in.
+int memls_cg_layout(crimson_lhs* L, int* resident64, int* resident32, long long* smem_bytes) {
+    if (!L->cg_used64 && !L->cg_used32) return CRIMSON_ERR_STATE;
+    size_t rb = 0;
+    if (L->cg_used64) CR_CHECK(cg_layout<double>(L, &rb));
+    if (L->cg_used32) CR_CHECK(cg_layout<float>(L, &rb));
+    if (resident64) *resident64 = L->cg_used64 ? L->cg_res64 : 0;
+    if (resident32) *resident32 = L->cg_used32 ? L->cg_res32 : 0;
+    if (smem_bytes) *smem_bytes = L->cg_res_bytes;
+    return CRIMSON_OK;
+}
+
+// CGRAD (memLS.f90:367-430) on the Schur-like operator L P - Gt G P; R in/out (n).
+// use_s2: on the explicit operator (schur.cu), else with two products on
+// Gs / GLs, the sliced G and {Gt, L} of this NSSOLVER call.
+template <typename M>
+static int cgrad(Ctx& C, crimson_subls& ls, const M* Gs, const typename V4<M>::type* GLs, double* R, int nface,
+                 const double* coef, bool use_s2) {
+    crimson_lhs* L = C.L;
+    cudaStream_t s = C.s;
+    const int n = L->nNo;
+    const double time = now_s();
+    ls.suc = 0;
+    (std::is_same<M, float>::value ? L->cg_used32 : L->cg_used64) = true;
+    auto& acc = std::is_same<M, float>::value ? L->cg_acc32 : L->cg_acc64;
+    if (use_s2) {
+        CR_CUDA(cudaEventRecord(L->ev0, s));
+        CR_CHECK(cg_schur_launch<M>(L, R, nface, coef, ls.relTol, ls.absTol, ls.mItr, C.sc(kSlotCg)));
+        CR_CUDA(cudaEventRecord(L->ev1, s));
+        CR_CHECK(C.sync_scal(kSlotCg, 5));
+        const double err = L->hscal[kSlotCg + 0], errO = L->hscal[kSlotCg + 1];
+        const int i = (int)L->hscal[kSlotCg + 2];
+        if (L->hscal[kSlotCg + 3] < 0.0) {
+            set_last_error("CGRAD: a wait of the persistent kernel ran out");
+            return CRIMSON_ERR_CUDA;
+        }
+        ls.suc = (int)L->hscal[kSlotCg + 3];
+        ls.iNorm = L->hscal[kSlotCg + 4];
+        float ms = 0.f;
+        CR_CUDA(cudaEventElapsedTime(&ms, L->ev0, L->ev1));
+        acc.ms += ms;
+        acc.iters += i - 1;
+        acc.launches += 1;
+        if (L->s2_form_pending) {
+            float fm = 0.f;
+            CR_CUDA(cudaEventElapsedTime(&fm, L->s2_ev0, L->s2_ev1));
+            L->s2_form_ms += fm;
+            L->s2_forms += 1;
+            L->s2_form_pending = false;
+        }
+        ls.fNorm = std::sqrt(err);
+        ls.callD = now_s() - time + ls.callD;
+        ls.dB = 5.0 * std::log(err / errO);
+        ls.itr = ls.itr + i - 1;
+        return CRIMSON_OK;
+    }
+    C.dot((const double*)R, (const double*)R, n, kSlotErr);
+    CR_CHECK(C.sync_scal(kSlotErr, 1));
+    double errO = std::sqrt(L->hscal[kSlotErr]);
+    ls.iNorm = errO;
+    double eps = std::max(ls.absTol, ls.relTol * errO);
+    eps = eps * eps;
+    double err = errO;
+    err = err * err;
+    size_t rbytes = 0;
+    CR_CHECK(cg_layout<M>(L, &rbytes));
+    const int grid = std::is_same<M, float>::value ? L->cg_grid32 : L->cg_grid;
+    const int mode = std::is_same<M, float>::value ? L->cg_res32 : L->cg_res64;
     const int fi = nface == 0 ? 0 : (nface == 1 ? 1 : 2);
-    const void* kfn = mode ? kres[fi] : kglb[fi];
+    const void* kfns[2][3] = {{(const void*)k_cg_persistent<0, M, false>, (const void*)k_cg_persistent<1, M, false>,
+                               (const void*)k_cg_persistent<kMaxCoupled, M, false>},
+                              {(const void*)k_cg_persistent<0, M, true>, (const void*)k_cg_persistent<1, M, true>,
+                               (const void*)k_cg_persistent<kMaxCoupled, M, true>}};
+    const void* kfn = kfns[mode ? 1 : 0][fi];
     const size_t dyn = mode ? rbytes : 0;
     CR_CHECK(L->cgPart.alloc(3 * (size_t)kCgPartStride * std::max(L->cg_grid, L->cg_grid32)));
     CR_CHECK(L->cgRecA.alloc(2 * (size_t)n));
     CR_CHECK(L->cgRecB.alloc(4 * (size_t)n));
     CR_CHECK(L->cgPd.alloc((size_t)n));
+    CR_CHECK(L->cgX.alloc((size_t)n));
+    CR_CHECK(L->cgSP.alloc((size_t)n));
     CR_CUDA(cudaMemsetAsync(L->cgX.p, 0, sizeof(double) * n, s));
     launch(k_cg_init, grid_for(n, 256), 256, 0, s, (const double*)R, reinterpret_cast<double2*>(L->cgRecA.p), n);
     CgArgs<M> a;
@@ -1794,7 +1830,6 @@ static int cgrad(Ctx& C, crimson_subls& ls, const M* Gs, const typename V4<M>::t
     ls.suc = (int)L->hscal[kSlotCg + 3];
     float ms = 0.f;
     CR_CUDA(cudaEventElapsedTime(&ms, L->ev0, L->ev1));
-    auto& acc = std::is_same<M, float>::value ? L->cg_acc32 : L->cg_acc64;
     acc.ms += ms;
     acc.iters += i - 1;
     acc.launches += 1;
@@ -1850,26 +1885,30 @@ static int ge_solve(int N, const double* A, double* B) {
 // Sliced matrix buffers of one precision (zeroed at allocation, so the
 // padding entries stay zero: conversions only write real entries).
 template <typename M>
-static int sell_alloc(crimson_lhs* L, DBuf<M>& K, DBuf<M>& G, DBuf<M>& GL) {
+static int sell_alloc(crimson_lhs* L, DBuf<M>& K, DBuf<M>& G, DBuf<M>& GL, bool two_product) {
     const size_t np = (size_t)L->npad + (size_t)kSlice * kSellUnroll;
-    if (K.n == 9 * np && G.n == 3 * np && GL.n == 4 * np) return CRIMSON_OK;
-    CR_CHECK(K.alloc(9 * np));
-    CR_CHECK(G.alloc(3 * np));
-    CR_CHECK(GL.alloc(4 * np));
-    CR_CUDA(cudaMemsetAsync(K.p, 0, sizeof(M) * K.n, L->stream));
-    CR_CUDA(cudaMemsetAsync(G.p, 0, sizeof(M) * G.n, L->stream));
-    CR_CUDA(cudaMemsetAsync(GL.p, 0, sizeof(M) * GL.n, L->stream));
+    auto zeroed = [&](DBuf<M>& b, size_t n) {
+        if (b.n == n) return CRIMSON_OK;
+        CR_CHECK(b.alloc(n));
+        CR_CUDA(cudaMemsetAsync(b.p, 0, sizeof(M) * n, L->stream));
+        return CRIMSON_OK;
+    };
+    CR_CHECK(zeroed(K, 9 * np));
+    if (two_product) {
+        CR_CHECK(zeroed(G, 3 * np));
+        CR_CHECK(zeroed(GL, 4 * np));
+    }
     return CRIMSON_OK;
 }
-static int sell_mats(crimson_lhs* L, double** K, double** G, double4** GL) {
-    CR_CHECK(sell_alloc(L, L->Ks64, L->Gs64, L->GLs64));
+static int sell_mats(crimson_lhs* L, double** K, double** G, double4** GL, bool two_product) {
+    CR_CHECK(sell_alloc(L, L->Ks64, L->Gs64, L->GLs64, two_product));
     *K = L->Ks64.p;
     *G = L->Gs64.p;
     *GL = reinterpret_cast<double4*>(L->GLs64.p);
     return CRIMSON_OK;
 }
-static int sell_mats(crimson_lhs* L, float** K, float** G, float4** GL) {
-    CR_CHECK(sell_alloc(L, L->Ks32, L->Gs32, L->GLs32));
+static int sell_mats(crimson_lhs* L, float** K, float** G, float4** GL, bool two_product) {
+    CR_CHECK(sell_alloc(L, L->Ks32, L->Gs32, L->GLs32, two_product));
     *K = L->Ks32.p;
     *G = L->Gs32.p;
     *GL = reinterpret_cast<float4*>(L->GLs32.p);
@@ -1975,18 +2014,20 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
     M* Ks = nullptr;
     M* Gs = nullptr;
     typename V4<M>::type* GLs = nullptr;
-    CR_CHECK(sell_mats(L, &Ks, &Gs, &GLs));
-    launch(k_to_sell<M>, grid_for(nNo, 256), 256, 0, s, L->rowptr, (const int*)L->sell_ptr.p, nNo, mK, mG, Gt, mL,
-           L->npad, Ks, Gs, GLs);
-    // mixed precision: the CG runs on the explicit FP32 Schur operator
-    bool use_s2 = false;
-    if (std::is_same<M, float>::value && ls->schur && cg_nface <= kMaxCoupled) {
-        CR_CHECK(schur_pattern(L));
-        if (L->s2_state == 1) {
-            CR_CHECK(schur_form(L, mG, Gt, mL));
-            use_s2 = true;
-        }
+    // CGRAD's operator: in FP64 formed explicitly where the pattern allows
+    // (schur.cu); in the mixed solve only on request, since rounding S
+    // instead of G, Gt and L moves its result by up to 1e-9.
+    const bool want_s2 = std::is_same<M, double>::value || ls->schur;
+    if (want_s2) CR_CHECK(schur_pattern(L));
+    const bool use_s2 = want_s2 && L->s2_state == 1;
+    if (ls->schur) L->s2_asked = true;
+    if (use_s2) {
+        CR_CHECK(schur_form<M>(L, mG, Gt, mL));
+        if (cg_nface > 0) CR_CHECK(schur_faces(L, cg_nface));
     }
+    CR_CHECK(sell_mats(L, &Ks, &Gs, &GLs, !use_s2));
+    launch(k_to_sell<M>, grid_for(nNo, 256), 256, 0, s, L->rowptr, (const int*)L->sell_ptr.p, nNo, mK, mG, Gt, mL,
+           L->npad, Ks, use_s2 ? nullptr : Gs, GLs);
     int i, iBB = 0;
     for (i = 1; i <= ls->RI.mItr; ++i) {
         iB = 2 * i - 1;
@@ -1996,9 +2037,8 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
         C.vs3(mD, (const double*)Ucol(i - 1), Pcol(i - 1));
         launch(k_sub<double, double, double>, grid_for(nNo, 256), 256, 0, s, (const double*)L->Rc.p,
                (const double*)Pcol(i - 1), Pcol(i - 1), (long long)nNo);
-        CR_CHECK(cgrad<M>(C, ls->CG, (const M*)Gs, (const typename V4<M>::type*)GLs, Pcol(i - 1),
-                          cg_nface,
-                          cg_coef, use_s2));
+        CR_CHECK(cgrad<M>(C, ls->CG, (const M*)Gs, (const typename V4<M>::type*)GLs, Pcol(i - 1), cg_nface, cg_coef,
+                          use_s2));
         C.sv3(mG, (const double*)Pcol(i - 1), MUc(iB - 1));
         launch(k_sub<double, double, double>, grid_for(nv, 256), 256, 0, s, (const double*)L->Rm.p,
                (const double*)MUc(iB - 1), MUc(iBB - 1), nv);
@@ -2117,8 +2157,6 @@ static int lhs_work_alloc(crimson_lhs* L, const crimson_ls* ls) {
     CR_CHECK(L->MP.alloc((size_t)nNo * 2 * iB));
     CR_CHECK(L->basis.alloc(3 * (size_t)nNo * (sD + 1)));
     CR_CHECK(L->w3.alloc(3 * (size_t)nNo));
-    CR_CHECK(L->cgX.alloc((size_t)nNo));
-    CR_CHECK(L->cgSP.alloc((size_t)nNo));
     CR_CHECK(sell_pattern(L));
     if (!L->scal.p) {
         CR_CHECK(L->scal.alloc(kScalTotal));
@@ -2415,7 +2453,7 @@ int memls_kernel_time(crimson_lhs* L, int which, int reps, double* ms) {
         switch (which) {
             case 0: C.vv3s((const double*)L->Ks64.p, (const double*)L->basis.p, L->basis.p + n3); break;
             case 6: C.vv3((const double*)L->mK.p, (const double*)L->basis.p, L->basis.p + n3); break;
-            case 2: C.sv3((const double*)L->mG.p, (const double*)L->cgX.p, L->w3.p); break;
+            case 2: C.sv3((const double*)L->mG.p, (const double*)L->P.p, L->w3.p); break;
             case 5: C.vv3s((const float*)L->Ks32.p, (const double*)L->basis.p, L->basis.p + n3); break;
             default:
                 launch(k_mgs<double>, red_grid(n3), 256, 0, s, L->basis.p + 2 * n3, (const double*)L->basis.p,

@@ -24,9 +24,13 @@ struct RedScratch {
 };
 
 int schur_pattern(crimson_lhs* L);
+template <typename M>
 int schur_form(crimson_lhs* L, const double* mG, const double* Gt, const double* mL);
-int cg_schur_launch(crimson_lhs* L, const double* R, int nface, const double* coef, const double* w, const double* z,
-                    double eps, double err0, int mItr, double* out);
+int schur_faces(crimson_lhs* L, int nface);
+template <typename M>
+int cg_schur_launch(crimson_lhs* L, double* R, int nface, const double* coef, double relTol, double absTol, int mItr,
+                    double* out);
+int memls_cg_layout(crimson_lhs* L, int* resident64, int* resident32, long long* smem_bytes);
 
 }  // namespace crimson
 
@@ -67,6 +71,7 @@ struct crimson_lhs {
     DBuf<int> sell_ptr, sell_col;
     DBuf<double> Ks64, Gs64, GLs64;
     DBuf<float> Ks32, Gs32, GLs32;
+    bool cg_used64 = false, cg_used32 = false;   // a CGRAD ran in this precision
     int cg_grid = 0, cg_grid32 = 0;
     int cg_res64 = 0, cg_res32 = 0;    // CG kernel with block-resident columns (per matrix type)
     long long cg_res_bytes = -1;       // its shared memory per block (0: offsets exceed 16 bits); -1 unknown
@@ -90,16 +95,22 @@ struct crimson_lhs {
         long long iters = 0, launches = 0;
     } cg_acc64, cg_acc32;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // explicit FP32 Schur operator S = L - Gt G of the mixed-precision CG
-    // (schur.cu): 2-ring pattern (CSR and sliced int16 offsets), FP32 values
+    // explicit Schur operator S = L - Gt G of CGRAD (schur.cu): slices of the
+    // 2-ring pattern, chunk descriptors, the blocks' ranges, and the operator
+    // (values and int16 column offsets by chunk) per storage precision
     int s2_state = 0;       // 0: pattern not built, 1: usable, -1: not usable on this pattern
-    DBuf<int> s2_rowptr, s2_col, s2_sp;
-    DBuf<short> s2_off;
-    DBuf<float> s2_val;
-    DBuf<float2> s2_recF;
-    DBuf<double> s2_part;
+    bool s2_asked = false;  // a solve asked for it through crimson_memls_ls_set_schur
+    DBuf<int> s2_len, s2_sc;
+    DBuf<uint2> s2_desc;
+    DBuf<int4> s2_wl;
+    DBuf<int2> s2_blk;
+    DBuf<unsigned> s2_mask;
+    DBuf<unsigned char> s2_op64, s2_op32;
+    DBuf<double> s2_R;
+    DBuf<ulonglong2> s2_pk;
+    unsigned long long s2_epoch = 0;
     long long s2_nnz = 0, s2_npad = 0;
-    int s2_nslice = 0, s2_grid = 0;
+    int s2_nslice = 0, s2_grid = 0, s2_max_rows = 0, s2_max_cols = 0, s2_max_chunks = 0, s2_warps = 0;
     cudaEvent_t s2_ev0 = nullptr, s2_ev1 = nullptr;
     bool s2_form_pending = false;   // a formation was recorded between s2_ev0 and s2_ev1
     double s2_form_ms = 0.0;
@@ -116,7 +127,7 @@ struct crimson_ls {
     int precision = CRIMSON_FP64;  // CRIMSON_FP64, CRIMSON_MIXED or CRIMSON_MIXED_F32_TANGENT
     int max_refine = 4;            // FP64 refinement sweeps of the mixed solve
     double refine_tol = 0.0;       // target |R - A x| / |R|; <= 0: RI.relTol
-    int schur = 0;                 // mixed precision: 1 = CG on the explicit FP32 Schur operator when the pattern allows
+    int schur = 0;                 // 1: the mixed solve's CG runs on the explicit Schur operator too, where the pattern allows
     std::string log_path;          // per-solve log (memLS_NS.log format); empty: off
 };
 

@@ -1,220 +1,324 @@
-// Explicit FP32 Schur operator for the mixed-precision CGRAD.
+// Explicit Schur operator of memLS's CGRAD.
 //
 // memLS's CGRAD (flowsolver/src/memLS.f90:367-430) iterates on the
 // continuity Schur complement without forming it: every iteration computes
-// SP = L P - Gt (G P) - (coupled-face terms) as two sparse products, which
-// costs two neighbour-gather phases and three grid barriers per iteration in
-// the persistent kernel.  In the mixed-precision solve the inner CG only has
-// to shape search directions (the FP64 NSSOLVER Gram system and the
-// iterative refinement decide the accuracy), so there the operator
-// S = L - Gt G is formed once per NSSOLVER call in FP64 (on the 2-ring
-// pattern of the node graph) and stored in FP32:
+// SP = L P - Gt (G P) - (coupled-face terms) as two sparse products.  Here
+// S = L - Gt G is formed once per NSSOLVER call, in FP64 and in a fixed
+// order, on the 2-ring pattern of the node graph, stored in FP64 or, for the
+// mixed-precision solve, rounded once to FP32; an iteration is then one
+// sparse product.  Against the two products the stream per row is smaller
+// (about 62 entries of 8 + 2 B against 14.7 blocks of 7 values: 620 / 823 B
+// in FP64, 372 / 412 B in FP32), and an iteration has two grid-wide barriers
+// instead of three.  (The two-product kernel stays for patterns that do not
+// qualify: rows of more than kS2Cap entries, or column offsets past 16 bits
+// -- a numbering without locality, where four times as many gathers would
+// each cost a sector of their own.)
 //
-//   * pattern (once per lhs): the 2-ring of every row, sorted, as a sliced
-//     ELL layout (slices of 32 rows, column-major) with int16 column offsets
-//     col - row (the layout requires |col - row| <= 32767 and at most
-//     kS2Cap entries per row; otherwise the two-product kernel is used);
-//   * values (per NSSOLVER call): S_ij = L_ij - sum_k Gt_ik . G_kj summed in
-//     FP64 in a fixed order (L first, then k in CSR order) -- deterministic --
-//     and rounded once to FP32;
-//   * CG iteration (persistent cooperative kernel, two grid barriers):
-//     phase 1 SP_raw = S P with P = R + beta P_prev formed on the fly from
-//     an FP32 copy {R, P_prev} of the neighbours, plus <P, SP_raw>, w_f . P
-//     and z_f . P; phase 2 the coupled-face (Sherman-Morrison) correction
-//     SP = SP_raw - sum_f coef_f (w_f . P) z_f, X += alpha P, R -= alpha SP,
-//     |R|^2.  Every product accumulates in FP64; X, R, P and all dot
-//     products are FP64, reduced per block and summed in block order.
+// Layout.  Rows in slices of 32 (one warp), a slice as wide as its longest
+// row, cut into chunks of up to kS2Chunk columns.  A chunk is contiguous: its
+// values column by column (32 rows each), then its int16 column offsets
+// col - row: one bulk copy brings it into shared memory.
 //
-// The coupled-face term is the same exact rank-one form the two-product
-// kernel uses: Gt (G P + c valM (valM . G P)) = Gt G P + c (w . P) z with
-// w = G^T valM, z = Gt valM built once per NSSOLVER call.
-#include <cooperative_groups.h>
-#include <cub/cub.cuh>
-
+// CG kernel (persistent, one block per SM).  A block owns a contiguous range
+// of slices.  Its warps take them in turn, so that at any time they gather
+// from neighbouring rows and find them in the L1 (contiguous ranges per warp
+// instead: 107 us against 97 per FP32 iteration on the 4M-tet cylinder); the
+// slices left after the last full turn are split chunk by chunk, partial rows
+// summed through shared memory in warp order.  Two forms:
+//   * resident: where the block's chunks fit in shared memory (meshes up to
+//     about 300,000 tets in FP64, 500,000 in FP32) they are loaded once per
+//     call and no iteration touches the operator in memory again; bound by
+//     the two barriers (1.3 and 2.3 us) and one gather latency;
+//   * streaming: every warp runs its chunks through a ring of two
+//     shared-memory stages filled by cp.async.bulk, so the stream does not
+//     stop at slice ends, barriers or iteration ends; bound by HBM (the
+//     product phase reads 6.7 TB/s in FP64, 5.8 in FP32).
+// Per iteration, before (two-product kernel) and now, B200: 4M-tet cylinder
+// 118 / 80 us FP64, 74 / 56 FP32; 452k-tet bifurcation 24.6 / 16 FP32;
+// 108k-tet cylinder 20 / 9.2 FP64; 1152 tets 15 / 5.5 FP64.
+//
+// Iteration.  S P is kept by the recurrence S P = S R + beta S P_prev, so the
+// product gathers only R (8 B per entry) and does not wait for P:
+//   phase 1  SP = S R + beta SP, P = R + beta P, <P, SP>, w_f . P, z_f . P
+//   barrier  alpha, and the coupled-face coefficients
+//   phase 2  X += alpha P, R -= alpha (SP - sum_f coef_f (w_f . P) z_f), |R|^2
+//   barrier  beta; orders R's new values before the next gathers
+// The coupled-face term is exact: Gt (G P + c valM (valM . G P)) =
+// Gt G P + c (w . P) z with w = G^T valM, z = Gt valM built once per NSSOLVER
+// call; w and z vanish outside the faces' neighbourhoods, so a bit per slice
+// says where they are read.
 #include <algorithm>
-#include <atomic>
 #include <climits>
 #include <vector>
 
 #include "common.cuh"
+#include "gridred.cuh"
 #include "memls.cuh"
 
 namespace crimson {
 
-constexpr int kS2Cap = 256;        // 2-ring entries per row the formation kernel holds
-constexpr int kS2Threads = 1024;   // formation: one warp per row of a 32-row slice
-constexpr int kS2U = 8;            // entries per software-pipelined stage of the CG rows
-constexpr int kS2CgThreads = 512;
+constexpr int kS2Cap = 256;        // 2-ring entries per row
+constexpr int kS2Hash = 1024;      // slots of the pattern kernel's per-row set
+constexpr int kS2Chunk = 8;        // columns of a chunk
+constexpr int kS2FormWarps = 16;   // formation: rows in flight per block
+constexpr int kS2CgWarps = 24;     // most warps of a CG block (80 registers a thread)
 constexpr int kS2MaxFaces = 8;
-constexpr int kS2PartStride = 2 * kS2MaxFaces + 1;
+constexpr int kS2Vals = 1 + 2 * kS2MaxFaces;   // reductions of one barrier
+
+// Bytes of one column of a chunk (32 values and offsets).
+template <typename M>
+__host__ __device__ constexpr int s2_col_bytes() {
+    return 32 * (int)(sizeof(M) + sizeof(short));
+}
+
+// Byte offset of entry e of a row (lane = row & 31) in the operator, and of
+// its column offset; c0 = the slice's first column, w its width.
+template <typename M>
+__device__ __forceinline__ size_t s2_val_pos(int c0, int w, int e, int lane) {
+    const int k0 = e & ~(kS2Chunk - 1), k = e - k0;
+    constexpr int V = 16 / (int)sizeof(M);
+    const size_t base = (size_t)(c0 + k0) * s2_col_bytes<M>();
+    if (w - k0 >= kS2Chunk) return base + (size_t)((k / V) * 32 + lane) * 16 + (size_t)(k % V) * sizeof(M);
+    return base + (size_t)(k * 32 + lane) * sizeof(M);
+}
+template <typename M>
+__device__ __forceinline__ size_t s2_off_pos(int c0, int w, int e, int lane) {
+    const int k0 = e & ~(kS2Chunk - 1), k = e - k0, kc = min(kS2Chunk, w - k0);
+    const size_t base = (size_t)(c0 + k0) * s2_col_bytes<M>() + (size_t)kc * 32 * sizeof(M);
+    if (kc == kS2Chunk) return base + (size_t)lane * 16 + (size_t)k * sizeof(short);
+    return base + (size_t)(k * 32 + lane) * sizeof(short);
+}
 
 // ---------------------------------------------------------------------------
-// Pattern
+// Pattern: the sorted 2-ring of every row, one warp per row.  The distinct
+// columns are collected in a shared-memory hash set and sorted by counting.
+// Returns the row length (> kS2Cap: the row overflows).
 // ---------------------------------------------------------------------------
-__global__ void k_s2_count(const int* __restrict__ rowptr, const int* __restrict__ col, int n,
-                           long long* __restrict__ cnt) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        long long c = 0;
-        for (int t = rowptr[i]; t < rowptr[i + 1]; ++t) {
-            const int k = col[t];
-            c += rowptr[k + 1] - rowptr[k];
+__device__ int s2_ring2(const int* __restrict__ rowptr, const int* __restrict__ col, int r, int* set, int* list) {
+    const int lane = threadIdx.x & 31;
+    for (int q = lane; q < kS2Hash; q += 32) set[q] = -1;
+    __syncwarp();
+    const int rs = rowptr[r], re = rowptr[r + 1];
+    int mine = 0;
+    for (int t = rs; t < re; ++t) {
+        const int k = col[t], ks = rowptr[k], ke = rowptr[k + 1];
+        for (int u = ks + lane; u < ke; u += 32) {
+            const int j = col[u];
+            unsigned h = ((unsigned)j * 2654435761u) >> 22;   // kS2Hash slots
+            for (int probe = 0; probe < kS2Hash; ++probe) {
+                const int old = atomicCAS(set + h, -1, j);
+                if (old == -1) ++mine;
+                if (old == -1 || old == j) break;
+                h = (h + 1) & (kS2Hash - 1);
+            }
         }
-        cnt[i] = c;
+        __syncwarp();
+        // stop before the set can fill up: the row is over the cap anyway
+        int tot = mine;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        if (tot > kS2Cap) return tot;
     }
+    int len = mine;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) len += __shfl_xor_sync(0xffffffffu, len, o);
+    if (!list) return len;
+    // compact, then place every column at the number of smaller ones
+    int base = 0;
+    for (int q0 = 0; q0 < kS2Hash; q0 += 32) {
+        const int j = set[q0 + lane];
+        const unsigned m = __ballot_sync(0xffffffffu, j >= 0);
+        __syncwarp();
+        if (j >= 0) set[base + __popc(m & ((1u << lane) - 1u))] = j;   // at or before q0 + lane
+        base += __popc(m);
+        __syncwarp();
+    }
+    for (int e = lane; e < len; e += 32) {
+        const int j = set[e];
+        int rank = 0;
+        for (int q = 0; q < len; ++q) rank += set[q] < j ? 1 : 0;
+        list[rank] = j;
+    }
+    __syncwarp();
+    return len;
 }
 
-__global__ void k_s2_fill(const int* __restrict__ rowptr, const int* __restrict__ col, int n,
-                          const long long* __restrict__ off, unsigned long long* __restrict__ keys) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        long long p = off[i];
-        for (int t = rowptr[i]; t < rowptr[i + 1]; ++t) {
-            const int k = col[t];
-            for (int u = rowptr[k]; u < rowptr[k + 1]; ++u)
-                keys[p++] = (unsigned long long)i * (unsigned long long)n + (unsigned long long)col[u];
-        }
-    }
-}
-
-__device__ __forceinline__ long long s2_lower_bound(const unsigned long long* a, long long m, unsigned long long v) {
-    long long lo = 0, hi = m;
-    while (lo < hi) {
-        const long long mid = (lo + hi) >> 1;
-        if (a[mid] < v)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
-__global__ void k_s2_csr(const unsigned long long* __restrict__ ukeys, long long m, int n, int* __restrict__ rowptr2,
-                         int* __restrict__ col2, int* __restrict__ maxoff) {
-    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long st = (long long)gridDim.x * blockDim.x;
-    for (long long i = t0; i <= n; i += st)
-        rowptr2[i] = (int)s2_lower_bound(ukeys, m, (unsigned long long)i * (unsigned long long)n);
-    int mo = 0;
-    for (long long j = t0; j < m; j += st) {
-        const int r = (int)(ukeys[j] / (unsigned long long)n);
-        const int c = (int)(ukeys[j] % (unsigned long long)n);
-        col2[j] = c;
-        mo = max(mo, abs(c - r));
+// Row lengths; stat[0] the longest, stat[1] the largest |col - row|.
+__global__ void __launch_bounds__(256) k_s2_len(const int* __restrict__ rowptr, const int* __restrict__ col, int n,
+                                                int* __restrict__ len, int* __restrict__ stat) {
+    __shared__ int sets[8][kS2Hash];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int* set = sets[wid];
+    int mlen = 0, moff = 0;
+    for (int r = blockIdx.x * 8 + wid; r < n; r += gridDim.x * 8) {
+        const int l = s2_ring2(rowptr, col, r, set, nullptr);
+        if (lane == 0) len[r] = l;
+        mlen = max(mlen, l);
+        for (int q = lane; q < kS2Hash; q += 32)
+            if (set[q] >= 0) moff = max(moff, abs(set[q] - r));
+        __syncwarp();
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mo = max(mo, __shfl_xor_sync(0xffffffffu, mo, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(maxoff, mo);
-}
-
-// int16 offsets col - row at every sliced position (pads: 0, the row itself)
-__global__ void k_s2_offsets(const int* __restrict__ rowptr2, const int* __restrict__ col2, const int* __restrict__ sp,
-                             int n, int nrows_pad, short* __restrict__ soff) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows_pad; r += gridDim.x * blockDim.x) {
-        const int s = r >> 5;
-        const int w = (sp[s + 1] - sp[s]) >> 5;
-        const int base = sp[s] + (r & 31);
-        const int rs = r < n ? rowptr2[r] : 0;
-        const int len = r < n ? rowptr2[r + 1] - rs : 0;
-        for (int k = 0; k < w; ++k) soff[base + 32 * k] = k < len ? (short)(col2[rs + k] - r) : (short)0;
+    for (int o = 16; o > 0; o >>= 1) moff = max(moff, __shfl_xor_sync(0xffffffffu, moff, o));
+    if (lane == 0) {
+        atomicMax(stat, mlen);
+        atomicMax(stat + 1, moff);
     }
 }
 
+// Column offsets of every row into the operator's layout (pads: 0, the row
+// itself; their values stay zero).  One warp per row, pad rows of the last
+// slice included.
+template <typename M>
+__global__ void __launch_bounds__(256) k_s2_offsets(const int* __restrict__ rowptr, const int* __restrict__ col, int n,
+                                                    int nrows_pad, const int* __restrict__ sc,
+                                                    unsigned char* __restrict__ op) {
+    __shared__ int sets[8][kS2Hash];
+    __shared__ int lists[8][kS2Cap];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int r = blockIdx.x * 8 + wid; r < nrows_pad; r += gridDim.x * 8) {
+        const int len = r < n ? s2_ring2(rowptr, col, r, sets[wid], lists[wid]) : 0;
+        const int c0 = sc[r >> 5], w = sc[(r >> 5) + 1] - c0;
+        for (int e = lane; e < w; e += 32)
+            *reinterpret_cast<short*>(op + s2_off_pos<M>(c0, w, e, r & 31)) =
+                e < len ? (short)(lists[wid][e] - r) : (short)0;
+        __syncwarp();
+    }
+}
+
+// Per lhs, once: row lengths, slices, chunks, the blocks' slice ranges.
+// s2_state 1: usable, -1: the pattern does not qualify.
 int schur_pattern(crimson_lhs* L) {
     if (L->s2_state != 0) return CRIMSON_OK;
     cudaStream_t s = L->stream;
     const int n = L->nNo;
     L->s2_state = -1;   // unusable unless every step below succeeds
-    DBuf<long long> cnt, koff;
-    CR_CHECK(cnt.alloc((size_t)n + 1));
-    CR_CHECK(koff.alloc((size_t)n + 1));
-    CR_CUDA(cudaMemsetAsync(cnt.p + n, 0, sizeof(long long), s));
-    launch(k_s2_count, grid_for(n, 256), 256, 0, s, L->rowptr, L->col, n, cnt.p);
-    size_t tb = 0;
-    CR_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.p, koff.p, n + 1, s));
-    DBuf<unsigned char> tmp;
-    CR_CHECK(tmp.alloc(tb));
-    CR_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, cnt.p, koff.p, n + 1, s));
-    long long total = 0;
-    CR_CUDA(cudaMemcpyAsync(&total, koff.p + n, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    CR_CUDA(cudaStreamSynchronize(s));
-    if (total <= 0 || total > (long long)INT_MAX) return CRIMSON_OK;
-    const int m = (int)total;
-    DBuf<unsigned long long> keys, keys2, ukeys;
-    DBuf<int> dcount, dmax;
-    CR_CHECK(keys.alloc((size_t)m));
-    CR_CHECK(keys2.alloc((size_t)m));
-    launch(k_s2_fill, grid_for(n, 256), 256, 0, s, L->rowptr, L->col, n, (const long long*)koff.p, keys.p);
-    unsigned long long maxkey = (unsigned long long)n * (unsigned long long)n;
-    int end_bit = 1;
-    while (end_bit < 64 && (1ull << end_bit) <= maxkey) ++end_bit;
-    cub::DoubleBuffer<unsigned long long> dk(keys.p, keys2.p);
-    size_t tb_sort = 0, tb_uniq = 0;
-    CR_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb_sort, dk, m, 0, end_bit, s));
-    CR_CHECK(dcount.alloc(1));
-    CR_CHECK(ukeys.alloc((size_t)m));
-    CR_CUDA(cub::DeviceSelect::Unique(nullptr, tb_uniq, keys.p, ukeys.p, dcount.p, m, s));
-    CR_CHECK(tmp.alloc(std::max(tb_sort, tb_uniq)));
-    CR_CUDA(cub::DeviceRadixSort::SortKeys(tmp.p, tb_sort, dk, m, 0, end_bit, s));
-    CR_CUDA(cub::DeviceSelect::Unique(tmp.p, tb_uniq, dk.Current(), ukeys.p, dcount.p, m, s));
-    int nnz2 = 0;
-    CR_CUDA(cudaMemcpyAsync(&nnz2, dcount.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CR_CUDA(cudaStreamSynchronize(s));
-    keys.release();
-    keys2.release();
-    DBuf<int> rowptr2, col2;
-    CR_CHECK(rowptr2.alloc((size_t)n + 1));
-    CR_CHECK(col2.alloc((size_t)nnz2));
-    CR_CHECK(dmax.alloc(1));
-    CR_CUDA(cudaMemsetAsync(dmax.p, 0, sizeof(int), s));
-    launch(k_s2_csr, grid_for((long long)nnz2 + n + 1, 256), 256, 0, s, (const unsigned long long*)ukeys.p,
-           (long long)nnz2, n, rowptr2.p, col2.p, dmax.p);
-    std::vector<int> rp((size_t)n + 1);
-    int maxoff = 0;
-    CR_CUDA(cudaMemcpyAsync(rp.data(), rowptr2.p, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost, s));
-    CR_CUDA(cudaMemcpyAsync(&maxoff, dmax.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CR_CUDA(cudaStreamSynchronize(s));
-    ukeys.release();
-    int maxlen = 0;
-    for (int i = 0; i < n; ++i) maxlen = std::max(maxlen, rp[i + 1] - rp[i]);
-    if (maxoff > 32767 || maxlen > kS2Cap) return CRIMSON_OK;
-    // sliced layout
-    const int ns = (n + 31) / 32;
-    std::vector<int> sp((size_t)ns + 1, 0);
-    long long pos = 0;
-    for (int q = 0; q < ns; ++q) {
-        int w = 0;
-        for (int r = q * 32; r < std::min(n, (q + 1) * 32); ++r) w = std::max(w, rp[r + 1] - rp[r]);
-        sp[q] = (int)pos;
-        pos += 32LL * w;
-        if (pos + 64LL * kS2U > (long long)INT_MAX) return CRIMSON_OK;
-    }
-    sp[ns] = (int)pos;
-    // the CG row loop loads one stage ahead: up to 32 (2 kS2U - 1) entries past
-    // the last slice, so the arrays carry 64 kS2U zero entries there
-    const size_t np = (size_t)pos + 64 * (size_t)kS2U;
-    CR_CHECK(L->s2_sp.upload(sp.data(), sp.size(), s));
-    CR_CHECK(L->s2_off.alloc(np));
-    CR_CHECK(L->s2_val.alloc(np));
-    CR_CUDA(cudaMemsetAsync(L->s2_off.p, 0, sizeof(short) * np, s));
-    CR_CUDA(cudaMemsetAsync(L->s2_val.p, 0, sizeof(float) * np, s));
-    launch(k_s2_offsets, grid_for((long long)ns * 32, 256), 256, 0, s, (const int*)rowptr2.p, (const int*)col2.p,
-           (const int*)L->s2_sp.p, n, ns * 32, L->s2_off.p);
+    CR_CHECK(L->s2_len.alloc((size_t)n));
+    DBuf<int> stat;
+    CR_CHECK(stat.alloc(2));
+    CR_CUDA(cudaMemsetAsync(stat.p, 0, 2 * sizeof(int), s));
+    launch(k_s2_len, grid_for(n, 8, 16), 256, 0, s, L->rowptr, L->col, n, L->s2_len.p, stat.p);
+    std::vector<int> len((size_t)n);
+    int hs[2] = {0, 0};
+    CR_CUDA(cudaMemcpyAsync(hs, stat.p, sizeof(hs), cudaMemcpyDeviceToHost, s));
+    CR_CUDA(cudaMemcpyAsync(len.data(), L->s2_len.p, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, s));
     CR_CUDA(cudaStreamSynchronize(s));
     CR_CUDA(cudaGetLastError());
-    L->s2_rowptr = std::move(rowptr2);
-    L->s2_col = std::move(col2);
+    if (hs[0] > kS2Cap || hs[1] > 32767) return CRIMSON_OK;
+    const int ns = (n + 31) / 32;
+    std::vector<int> sc((size_t)ns + 1, 0);
+    std::vector<long long> cp((size_t)ns + 1, 0);   // chunks before each slice
+    long long cols = 0, nnz2 = 0;
+    for (int q = 0; q < ns; ++q) {
+        int w = 1;
+        for (int r = q * 32; r < std::min(n, (q + 1) * 32); ++r) {
+            w = std::max(w, len[r]);
+            nnz2 += len[r];
+        }
+        sc[q] = (int)cols;
+        cols += w;
+        cp[q + 1] = cp[q] + (w + kS2Chunk - 1) / kS2Chunk;
+        if (32 * cols > (long long)INT_MAX) return CRIMSON_OK;
+    }
+    sc[ns] = (int)cols;
+    // Blocks: one per SM, contiguous slice ranges with equal shares of the
+    // work: chunks, and the per-row updates of a slice, which cost about as
+    // much as one more chunk.  On small meshes fewer blocks, so that every
+    // block has a chunk for each of four warps (fewer packets per barrier).
+    const int sms = std::min(sm_count(), kGrMaxBlocks);
+    const int grid = (int)std::max(1LL, std::min<long long>({(long long)sms, (long long)ns, (cp[ns] + 3) / 4}));
+    std::vector<int2> blk((size_t)grid + 1);   // first slice, first chunk
+    int q = 0;
+    L->s2_max_rows = 0;
+    int max_chunks = 0;
+    for (int b = 0; b <= grid; ++b) {
+        auto cost = [&](int sl) { return cp[sl] + sl; };
+        const long long want = cost(ns) * b / grid;
+        while (q < ns && cost(q) < want && (cost(q + 1) <= want || want - cost(q) > cost(q + 1) - want)) ++q;
+        if (b == grid) q = ns;
+        blk[b] = make_int2(q, (int)cp[q]);
+        if (b > 0) {
+            L->s2_max_rows = std::max(L->s2_max_rows, 32 * (blk[b].x - blk[b - 1].x));
+            max_chunks = std::max(max_chunks, blk[b].y - blk[b - 1].y);
+            L->s2_max_cols = std::max(L->s2_max_cols, sc[blk[b].x] - sc[blk[b - 1].x]);
+        }
+    }
+    // Per warp its chunks in order.  A block's warps take its slices in turn,
+    // so that at any time they work on neighbouring rows, whose gathers meet
+    // in the L1; the slices left over after the last full turn are cut into
+    // equal shares of chunks.
+    L->s2_max_chunks = max_chunks;
+    const int nw = std::min(kS2CgWarps, std::max(4, max_chunks));
+    // chunk: first column, then slice << 6 | last << 5 | first << 4 | columns
+    std::vector<uint2> desc;
+    desc.reserve((size_t)cp[ns]);
+    std::vector<int4> wl((size_t)grid * nw);   // begin, chunks, last warp that continues this one's last slice
+    auto put = [&](int sl, int k) {
+        const int w = sc[sl + 1] - sc[sl], k0 = k * kS2Chunk, kc = std::min(kS2Chunk, w - k0);
+        desc.push_back(make_uint2((unsigned)(sc[sl] + k0), (unsigned)sl << 6 | (k0 + kc == w ? 32u : 0u) |
+                                                               (k0 == 0 ? 16u : 0u) | (unsigned)kc));
+    };
+    for (int b = 0; b < grid; ++b) {
+        const int s0 = blk[b].x, s1 = blk[b + 1].x;
+        const int full = (s1 - s0) / nw * nw;
+        const long long c0 = cp[s0 + full], tail = cp[s1] - c0;
+        for (int w = 0; w < nw; ++w) {
+            const int begin = (int)desc.size();
+            for (int sl = s0 + w; sl < s0 + full; sl += nw)
+                for (int k = 0; k < cp[sl + 1] - cp[sl]; ++k) put(sl, k);
+            const long long t0 = tail * w / nw, t1 = tail * (w + 1) / nw;
+            int sl = s0 + full;
+            for (long long t = t0; t < t1; ++t) {
+                while (cp[sl + 1] - c0 <= t) ++sl;
+                put(sl, (int)(t - (cp[sl] - c0)));
+            }
+            int wlast = w;
+            if (t1 > t0)   // sl is the slice of chunk t1 - 1
+                while (wlast + 1 < nw && tail * (wlast + 1) / nw < cp[sl + 1] - c0) ++wlast;
+            wl[(size_t)b * nw + w] = make_int4(begin, (int)desc.size() - begin, wlast, t1 > t0 ? 1 : 0);
+        }
+    }
+    L->s2_warps = nw;
+    CR_CHECK(L->s2_wl.upload(wl.data(), wl.size(), s));
+    CR_CHECK(L->s2_sc.upload(sc.data(), sc.size(), s));
+    CR_CHECK(L->s2_desc.upload(desc.data(), desc.size(), s));
+    CR_CHECK(L->s2_blk.upload(blk.data(), blk.size(), s));
+    CR_CHECK(L->s2_mask.alloc((size_t)ns + (size_t)grid));
+    CR_CHECK(L->s2_pk.alloc(2 * (size_t)kS2Vals * grid));
+    CR_CUDA(cudaMemsetAsync(L->s2_pk.p, 0, sizeof(ulonglong2) * L->s2_pk.n, s));
+    CR_CUDA(cudaStreamSynchronize(s));
+    L->s2_epoch = 0;
+    L->s2_grid = grid;
     L->s2_nnz = nnz2;
-    L->s2_npad = pos;
+    L->s2_npad = 32 * cols;
     L->s2_nslice = ns;
     L->s2_state = 1;
     return CRIMSON_OK;
 }
 
+// The operator's buffer in storage type M with its column offsets, on the
+// first solve that uses it.
+template <typename M>
+static int s2_buffer(crimson_lhs* L, DBuf<unsigned char>& op) {
+    const size_t bytes = (size_t)(L->s2_npad / 32) * s2_col_bytes<M>();
+    if (op.p && op.n == bytes) return CRIMSON_OK;
+    cudaStream_t s = L->stream;
+    CR_CHECK(op.alloc(bytes));
+    const int rows = 32 * L->s2_nslice;
+    launch(k_s2_offsets<M>, grid_for(rows, 8, 16), 256, 0, s, L->rowptr, L->col, L->nNo, rows, (const int*)L->s2_sc.p,
+           op.p);
+    CR_CUDA(cudaGetLastError());
+    return CRIMSON_OK;
+}
+static DBuf<unsigned char>& s2_op(crimson_lhs* L, const double*) { return L->s2_op64; }
+static DBuf<unsigned char>& s2_op(crimson_lhs* L, const float*) { return L->s2_op32; }
+
 // ---------------------------------------------------------------------------
-// Values: S = L - Gt G in FP64, rounded to FP32.  One block per 32-row slice,
-// one warp per row; the row's 2-ring columns and FP64 accumulators sit in
-// shared memory.  Within a warp the lanes add distinct columns, and the
-// contributions are added in a fixed order (L, then k in CSR order), so the
-// result is deterministic.  The slice is written back coalesced.
+// Values: S = L - Gt G in FP64, rounded to FP32 for M = float.  One warp per
+// row; the row's 2-ring columns and FP64 accumulators sit in shared memory.
+// Within a warp the lanes add distinct columns, and the contributions are
+// added in a fixed order (L, then k in CSR order): deterministic.  16 rows
+// (half a slice) per block pass, so the write-back fills whole sectors.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int s2_find(const int* cols, int len, int j) {
     int lo = 0, hi = len;
@@ -228,28 +332,26 @@ __device__ __forceinline__ int s2_find(const int* cols, int len, int j) {
     return lo;
 }
 
-__global__ void __launch_bounds__(kS2Threads) k_s2_form(const int* __restrict__ rowptr, const int* __restrict__ col,
-                                                        const double* __restrict__ mG, const double* __restrict__ Gt,
-                                                        const double* __restrict__ mL, const int* __restrict__ rowptr2,
-                                                        const int* __restrict__ col2, const int* __restrict__ sp,
-                                                        int n, int nslice, float* __restrict__ val) {
+template <typename M>
+__global__ void __launch_bounds__(32 * kS2FormWarps) k_s2_form(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                              const double* __restrict__ mG,
+                                                              const double* __restrict__ Gt,
+                                                              const double* __restrict__ mL,
+                                                              const int* __restrict__ len2, const int* __restrict__ sc,
+                                                              int n, int nrows_pad, unsigned char* __restrict__ op) {
     extern __shared__ double s2_smem[];
-    double* acc = s2_smem;                                                 // [32][kS2Cap]
-    int* cols = reinterpret_cast<int*>(s2_smem + 32 * kS2Cap);            // [32][kS2Cap]
-    __shared__ int lens[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double* a = acc + wid * kS2Cap;
-    int* cw = cols + wid * kS2Cap;
-    for (int sl = blockIdx.x; sl < nslice; sl += gridDim.x) {
-        const int r = sl * 32 + wid;
-        int len = 0;
-        if (r < n) {
-            const int rs2 = rowptr2[r];
-            len = rowptr2[r + 1] - rs2;
-            for (int e = lane; e < len; e += 32) {
-                cw[e] = col2[rs2 + e];
-                a[e] = 0.0;
-            }
+    // odd row stride: the write-back reads one column of 16 rows at a time
+    double* a = s2_smem + wid * (kS2Cap + 1);
+    int* cw = reinterpret_cast<int*>(s2_smem + kS2FormWarps * (kS2Cap + 1)) + wid * kS2Cap;
+    __shared__ int lens[kS2FormWarps];
+    for (int r0 = blockIdx.x * kS2FormWarps; r0 < nrows_pad; r0 += gridDim.x * kS2FormWarps) {
+        const int r = r0 + wid;
+        const int c0 = sc[r0 >> 5], w = sc[(r0 >> 5) + 1] - c0;
+        const int len = r < n ? len2[r] : 0;
+        for (int e = lane; e < len; e += 32) {
+            cw[e] = r + (int)*reinterpret_cast<const short*>(op + s2_off_pos<M>(c0, w, e, r & 31));
+            a[e] = 0.0;
         }
         if (lane == 0) lens[wid] = len;
         __syncwarp();
@@ -275,248 +377,550 @@ __global__ void __launch_bounds__(kS2Threads) k_s2_form(const int* __restrict__ 
             }
         }
         __syncthreads();
-        const int p0 = sp[sl], w = (sp[sl + 1] - p0) >> 5;
-        for (int p = threadIdx.x; p < 32 * w; p += blockDim.x) {
-            const int row = p & 31, e = p >> 5;
-            val[p0 + p] = e < lens[row] ? (float)acc[row * kS2Cap + e] : 0.0f;
+        for (int p = threadIdx.x; p < kS2FormWarps * w; p += blockDim.x) {
+            const int row = p % kS2FormWarps, e = p / kS2FormWarps;
+            *reinterpret_cast<M*>(op + s2_val_pos<M>(c0, w, e, (r0 + row) & 31)) =
+                e < lens[row] ? (M)s2_smem[row * (kS2Cap + 1) + e] : M(0);
         }
         __syncthreads();
     }
 }
 
+template <typename M>
 int schur_form(crimson_lhs* L, const double* mG, const double* Gt, const double* mL) {
     if (L->s2_state != 1) return CRIMSON_ERR_STATE;
     cudaStream_t s = L->stream;
-    const size_t smem = 32 * (size_t)kS2Cap * (sizeof(double) + sizeof(int));
-    // the attribute is per device; setting it again (two host threads racing
-    // on the first call) is harmless, so a relaxed flag is enough
-    static std::atomic<bool> attr_set[256];
-    int dev = 0;
-    CR_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 256) return CRIMSON_ERR_UNSUPPORTED;
-    if (!attr_set[dev].load(std::memory_order_relaxed)) {
-        CR_CUDA(cudaFuncSetAttribute(k_s2_form, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set[dev].store(true, std::memory_order_relaxed);
-    }
+    DBuf<unsigned char>& op = s2_op(L, (const M*)nullptr);
+    CR_CHECK(s2_buffer<M>(L, op));
+    const size_t smem = kS2FormWarps * ((kS2Cap + 1) * sizeof(double) + kS2Cap * sizeof(int));
+    CR_CUDA(cudaFuncSetAttribute(k_s2_form<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CR_CUDA(cudaEventRecord(L->s2_ev0, s));
-    launch(k_s2_form, std::min(L->s2_nslice, 2 * sm_count()), kS2Threads, smem, s, L->rowptr, L->col, mG, Gt, mL,
-           (const int*)L->s2_rowptr.p, (const int*)L->s2_col.p, (const int*)L->s2_sp.p, L->nNo, L->s2_nslice,
-           L->s2_val.p);
+    const int rows = 32 * L->s2_nslice;
+    launch(k_s2_form<M>, grid_for(rows, kS2FormWarps, 4), 32 * kS2FormWarps, smem, s, L->rowptr, L->col, mG, Gt, mL,
+           (const int*)L->s2_len.p, (const int*)L->s2_sc.p, L->nNo, rows, op.p);
     CR_CUDA(cudaEventRecord(L->s2_ev1, s));
     CR_CUDA(cudaGetLastError());
     L->s2_form_pending = true;
     return CRIMSON_OK;
 }
+template int schur_form<double>(crimson_lhs*, const double*, const double*, const double*);
+template int schur_form<float>(crimson_lhs*, const double*, const double*, const double*);
+
+// Bit f of mask[slice]: w_f or z_f is not zero on some row of the slice.
+__global__ void k_s2_mask(const double* __restrict__ w, const double* __restrict__ z, int nface, int n, int nslice,
+                          unsigned* __restrict__ mask) {
+    const int lane = threadIdx.x & 31;
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslice; s += (gridDim.x * blockDim.x) >> 5) {
+        const int r = 32 * s + lane;
+        unsigned m = 0;
+        for (int f = 0; f < nface; ++f) {
+            const bool nz = r < n && (w[(size_t)f * n + r] != 0.0 || z[(size_t)f * n + r] != 0.0);
+            if (__any_sync(0xffffffffu, nz)) m |= 1u << f;
+        }
+        if (lane == 0) mask[s] = m;
+    }
+}
+
+// The blocks' face bits: OR over their slices.
+__global__ void k_s2_blkmask(const int2* __restrict__ blk, const unsigned* __restrict__ mask, int nblk,
+                             unsigned* __restrict__ bmask) {
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nblk; b += (gridDim.x * blockDim.x) >> 5) {
+        unsigned m = 0;
+        for (int s = blk[b].x + (threadIdx.x & 31); s < blk[b + 1].x; s += 32) m |= mask[s];
+        m = __reduce_or_sync(0xffffffffu, m);
+        if ((threadIdx.x & 31) == 0) bmask[b] = m;
+    }
+}
+
+int schur_faces(crimson_lhs* L, int nface) {
+    launch(k_s2_mask, grid_for(32LL * L->s2_nslice, 256), 256, 0, L->stream, (const double*)L->cgW.p,
+           (const double*)L->cgZ.p, nface, L->nNo, L->s2_nslice, L->s2_mask.p);
+    launch(k_s2_blkmask, grid_for(32LL * L->s2_grid, 256), 256, 0, L->stream, (const int2*)L->s2_blk.p,
+           (const unsigned*)L->s2_mask.p, L->s2_grid, L->s2_mask.p + L->s2_nslice);
+    CR_CUDA(cudaGetLastError());
+    return CRIMSON_OK;
+}
 
 // ---------------------------------------------------------------------------
-// CGRAD on the explicit FP32 operator: one persistent cooperative launch per
-// call, two grid barriers per iteration.
+// CGRAD: one persistent cooperative launch per call.
 // ---------------------------------------------------------------------------
 struct CgS2Args {
-    const int* sp;
-    const short* off;
-    const float* val;
-    int n;
-    double* X;
-    double2* recA;   // (n) {R, P_prev}, FP64
-    float2* recF;    // (n) {R, P_prev} rounded to FP32: the gathered copy
-    double* SPr;     // (n) S P of this iteration, before the coupled-face term
+    const unsigned char* op;
+    const uint2* desc;
+    const int4* wl;
+    const int2* blk;
+    const unsigned* mask;   // face bits of the slices, then of the blocks
+    int nslice;
+    const int* sc;           // first column of every slice
+    int n, stages, nvec;     // nvec: vectors over the block's rows in shared memory
+    int max_rows, max_cols;  // of a block
+    int evict_first;         // the operator exceeds the L2: its lines go first
+    double* rhs;             // in: right side; out: solution
+    double* R;               // (2 n) the gathered residual, two alternating buffers
+    double* Pg;              // (n) P, SP, X when they do not fit in shared memory
+    double* SPg;
+    double* Xg;
     int nface;
     const double* w;  // (nface, n)
     const double* z;  // (nface, n)
     double coef[kS2MaxFaces];
-    double eps;
-    double err0;
+    double relTol, absTol;
     int mItr;
-    double* part;  // 2 regions of kS2PartStride * gridDim
-    double* out;   // err, errO, i, suc
+    ulonglong2* pk;   // 2 regions of kS2Vals packets per block
+    unsigned long long epoch;
+    double* out;      // err, errO, i, suc (-1: a wait ran out), initial norm
 };
 
-__device__ __forceinline__ double s2_sum_partials(const double* part, int k, double* sm) {
-    double v = 0.0;
-    for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) v += __ldcg(part + (size_t)b * kS2PartStride + k);
-    return block_sum(v, sm);
+__device__ __forceinline__ unsigned s2_smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ bool s2_try_wait(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded wait for a stage's copy.
+__device__ __forceinline__ bool s2_wait(unsigned bar, unsigned parity) {
+    if (s2_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (clock64() - t0 < kGrWaitClocks)
+        if (s2_try_wait(bar, parity)) return true;
+    return false;
 }
 
-template <int NF>
-__global__ void __launch_bounds__(kS2CgThreads, 2) k_cg_schur(CgS2Args a) {
-    namespace cgrp = cooperative_groups;
-    cgrp::grid_group grid = cgrp::this_grid();
-    __shared__ double sm[32];
-    const int n = a.n;
-    double* part1 = a.part;
-    double* part2 = a.part + (size_t)gridDim.x * kS2PartStride;
-    double err = a.err0, errO = a.err0;
+// One lane's share of a full chunk in shared memory.
+template <typename M>
+struct S2Lane;
+template <>
+struct S2Lane<double> {
+    double x[kS2Chunk];
+    __device__ __forceinline__ void load(const unsigned char* p) {
+#pragma unroll
+        for (int j = 0; j < kS2Chunk / 2; ++j) {
+            const double2 q = *reinterpret_cast<const double2*>(p + 512 * j);
+            x[2 * j] = q.x;
+            x[2 * j + 1] = q.y;
+        }
+    }
+};
+template <>
+struct S2Lane<float> {
+    float x[kS2Chunk];
+    __device__ __forceinline__ void load(const unsigned char* p) {
+#pragma unroll
+        for (int j = 0; j < kS2Chunk / 4; ++j) {
+            const float4 q = *reinterpret_cast<const float4*>(p + 512 * j);
+            x[4 * j] = q.x;
+            x[4 * j + 1] = q.y;
+            x[4 * j + 2] = q.z;
+            x[4 * j + 3] = q.w;
+        }
+    }
+};
+
+// The reductions of one barrier.  red[32 k + w]: warp w's partial of value k;
+// tot[k] (shared) receives the sums.  Value 0 comes from every block (and is
+// the barrier); values 1 + 2 f, 2 + 2 f of face f only from the blocks whose
+// slices touch the face (fpend: per lane, as gr_all_blocks), the others'
+// being zero.  data: the block's global writes before the call are visible to
+// all blocks after it.
+__device__ __noinline__ bool s2_reduce(const CgS2Args& a, const double* red, int nface, unsigned own_faces,
+                                       const unsigned char* fpend, unsigned long long ep, bool data, double* tot,
+                                       bool failed) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, nv = 1 + 2 * nface;
+    ulonglong2* pk = a.pk + (size_t)(ep & 1) * kS2Vals * gridDim.x;
+    bool fail = failed;
+    __syncthreads();
+    for (int k = wid; k < nv; k += nw)
+        if (k == 0 || ((own_faces >> ((k - 1) / 2)) & 1)) {
+            const double v = warp_sum(lane < nw ? red[32 * k + lane] : 0.0);
+            if (lane == 0) {
+                if (data) gr_release();
+                gr_publish(pk + (size_t)k * gridDim.x + blockIdx.x, v, ep);
+            }
+        }
+    for (int k = wid; k < nv; k += nw) {
+        const unsigned pend = k == 0 ? gr_all_blocks() : fpend[32 * ((k - 1) / 2) + lane];
+        const double v = gr_collect(pk + (size_t)k * gridDim.x, pend, ep, &fail);
+        if (data) gr_acquire();
+        if (lane == 0) tot[k] = v;
+    }
+    return __syncthreads_or(fail) != 0;
+}
+
+// kRes: the block's chunks stay in shared memory (loaded once), else they
+// stream through the warps' rings.
+template <typename M, bool kRes>
+__global__ void __launch_bounds__(32 * kS2CgWarps, 1) k_cg_schur(const __grid_constant__ CgS2Args a) {
+    extern __shared__ __align__(128) unsigned char s2_dyn[];
+    __shared__ double red[32 * kS2Vals], tot[kS2Vals];
+    __shared__ unsigned char fpend[32 * kS2MaxFaces];
+    // kept out of the registers of the inner loop: the places of P, SP, X and
+    // of the staged w, z; |R|^2 now and before, eps, |R_0|, beta
+    __shared__ double* vp[5];
+    __shared__ double scal[5];
+    constexpr int COL = s2_col_bytes<M>();
+    constexpr int CB = kS2Chunk * COL;   // bytes of a stage
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int n = a.n, S = a.stages;
+    const int2 b0 = a.blk[blockIdx.x], b1 = a.blk[blockIdx.x + 1];
+    const int row0 = 32 * b0.x, nsl = b1.x - b0.x;
+    const int4 wl = a.wl[blockIdx.x * nw + wid];   // this warp's chunks
+    const int nck = wl.y;
+
+    // shared memory: the chunks (all of the block's, or the warps' rings with
+    // their mbarriers), partial rows of slices begun by an earlier warp, the
+    // vectors, the face bits of the block's slices, descriptors
+    const int c0 = a.sc[b0.x];
+    const unsigned ring = kRes ? 0u : (unsigned)(wid * S * CB);
+    const unsigned o_bars = kRes ? (unsigned)a.max_cols * COL : (unsigned)(nw * S * CB);
+    const unsigned o_carry = o_bars + (kRes ? 0u : 8u * nw * S);
+    const unsigned o_vec = o_carry + 256u * nw;
+    const unsigned o_mask = o_vec + 8u * a.nvec * a.max_rows;
+    const unsigned o_desc = o_mask + (unsigned)(a.max_rows / 8) + (a.max_rows / 8 & 4);
+    unsigned long long* const bars = reinterpret_cast<unsigned long long*>(s2_dyn + o_bars) + wid * S;
+    double* const carry = reinterpret_cast<double*>(s2_dyn + o_carry);
+    unsigned* const mask = reinterpret_cast<unsigned*>(s2_dyn + o_mask);
+    // ring: word 1 of the staged chunks' descriptors; kRes: the warp's descriptors
+    unsigned* const sdesc =
+        reinterpret_cast<unsigned*>(s2_dyn + o_desc) + (kRes ? 2 * (wl.x - a.wl[blockIdx.x * nw].x) : wid * S);
+    const bool wz_local = kRes && a.nvec > 3;   // w_f, z_f of the block's rows in shared memory
+    const size_t ldw = wz_local ? (size_t)a.max_rows : (size_t)n;
+    if (threadIdx.x == 0) {
+        double* vec = reinterpret_cast<double*>(s2_dyn + o_vec);
+        vp[0] = a.nvec > 0 ? vec : a.Pg + row0;
+        vp[1] = a.nvec > 0 ? vec + a.max_rows : a.SPg + row0;
+        vp[2] = kRes ? vec + 2 * (size_t)a.max_rows : a.Xg + row0;
+        vp[3] = wz_local ? vec + 3 * (size_t)a.max_rows : const_cast<double*>(a.w) + row0;
+        vp[4] = wz_local ? vec + (3 + a.nface) * (size_t)a.max_rows : const_cast<double*>(a.z) + row0;
+    }
+    __syncthreads();
+
+    int qi = wl.x;           // ring: list entry lane 0 issues next, and its descriptor
+    uint2 dq = make_uint2(0u, 0u);
+    auto issue = [&](int st) {   // lane 0
+        unsigned long long policy;
+        if (a.evict_first)
+            asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+        else
+            asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(policy));
+        const unsigned bar = s2_smem_u32(bars + st), bytes = (dq.y & 15u) * COL;
+        sdesc[st] = dq.y;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::
+                "r"(s2_smem_u32(s2_dyn + ring + st * CB)), "l"(a.op + (size_t)dq.x * COL), "r"(bytes), "r"(bar), "l"(policy)
+            : "memory");
+        if (++qi == wl.x + nck) qi = wl.x;
+        dq = a.desc[qi];
+    };
+    const int nload = kRes ? 0 : min(S, nck);
+    if (kRes) {
+        const size_t beg = (size_t)c0 * COL, bytes = (size_t)(a.sc[b1.x] - c0) * COL;
+        for (size_t p = 16 * (size_t)threadIdx.x; p < bytes; p += 16 * (size_t)blockDim.x)
+            *reinterpret_cast<uint4*>(s2_dyn + p) = *reinterpret_cast<const uint4*>(a.op + beg + p);
+        for (int q = lane; q < nck; q += 32) reinterpret_cast<uint2*>(sdesc)[q] = a.desc[wl.x + q];
+    } else if (lane == 0 && nck > 0) {
+        for (int q = 0; q < S; ++q)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s2_smem_u32(bars + q)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        dq = a.desc[qi];
+        for (int st = 0; st < nload; ++st) issue(st);
+    }
+    unsigned cont = 0;   // warps whose partial rows complete this warp's last slice
+    for (int w = wid + 1; w <= wl.z; ++w)
+        if (a.wl[blockIdx.x * nw + w].w) cont |= 1u << w;
+    const unsigned* bmask = a.mask + a.nslice;
+    const unsigned own_faces = a.nface > 0 ? bmask[blockIdx.x] : 0u;
+    for (int t = threadIdx.x; t < nsl; t += blockDim.x) mask[t] = a.nface > 0 ? a.mask[b0.x + t] : 0u;
+    for (int f = wid; f < a.nface; f += nw) {
+        unsigned m = gr_all_blocks();
+#pragma unroll
+        for (int j = 0; j < kGrPolls; ++j)
+            if (((m >> j) & 1) && !((bmask[lane + 32 * j] >> f) & 1)) m &= ~(1u << j);
+        fpend[32 * f + lane] = (unsigned char)m;
+    }
+
+    // ---- initial residual: |rhs|^2 over the block's rows; P = SP = X = 0 ----
+    unsigned long long ep = a.epoch;
+    double part = 0.0;
+    for (int t = threadIdx.x; t < 32 * nsl; t += blockDim.x)
+        if (row0 + t < n) {
+            const double v = a.rhs[row0 + t];
+            vp[0][t] = 0.0;
+            vp[1][t] = 0.0;
+            vp[2][t] = 0.0;
+            a.R[row0 + t] = v;
+            if (wz_local)
+                for (int f = 0; f < a.nface; ++f) {
+                    vp[3][f * ldw + t] = a.w[(size_t)f * n + row0 + t];
+                    vp[4][f * ldw + t] = a.z[(size_t)f * n + row0 + t];
+                }
+            part += v * v;
+        }
+    part = warp_sum(part);
+    if (lane == 0) red[wid] = part;
+    bool fail = s2_reduce(a, red, 0, 0u, fpend, ++ep, true, tot, false);
+    if (threadIdx.x == 0) {
+        const double e = sqrt(tot[0]), eps = fmax(a.absTol, a.relTol * e);
+        scal[0] = e * e;
+        scal[1] = e;
+        scal[2] = eps * eps;
+        scal[3] = e;
+        scal[4] = 0.0;
+    }
+    __syncthreads();
+
     int suc = 0, i;
-    for (i = 1; i <= a.mItr; ++i) {
-        if (err < a.eps) {
+    int gs = 0;              // ring: stage of the next chunk, its mbarrier phase
+    unsigned parity = 0;
+    bool ok = true;          // no copy of this warp timed out
+    for (i = 1; i <= a.mItr && !fail; ++i) {
+        if (scal[0] < scal[2]) {
             suc = 1;
             break;
         }
-        const bool first = (i == 1);
-        const double beta = first ? 0.0 : err / errO;
-        errO = err;
-        // ---- phase 1: SP_raw = S P (P on the fly), <P, SP_raw>, w_f . P, z_f . P ----
-        double dps = 0.0, wp[NF > 0 ? NF : 1], zp[NF > 0 ? NF : 1];
-#pragma unroll
-        for (int f = 0; f < (NF > 0 ? NF : 1); ++f) wp[f] = zp[f] = 0.0;
-        for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-            const int p0 = __ldg(a.sp + (r >> 5));
-            const int w = (__ldg(a.sp + (r >> 5) + 1) - p0) >> 5;
-            const int base = p0 + (r & 31);
-            float v[kS2U];
-            short o[kS2U];
-#pragma unroll
-            for (int u = 0; u < kS2U; ++u) {
-                v[u] = __ldcs(a.val + base + 32 * u);
-                o[u] = __ldcs(a.off + base + 32 * u);
+        // R alternates between two buffers: phase 2 writes the one that no
+        // block has gathered from since the last barrier that ordered data
+        const double* Rc = a.R + (size_t)((i - 1) & 1) * n;
+        // ---- phase 1 ----
+        double dps = 0.0;
+        double acc0 = 0.0, acc1 = 0.0;
+        bool owner = false, open = false;   // owner: this warp began the slice; open: it is not complete
+        int slice = 0;
+        // completes a slice: SP = S R + beta SP, P = R + beta P, <P, SP>
+        auto finish = [&](double acc) {
+            const int t = 32 * (slice - b0.x) + lane;
+            if (row0 + t < n) {
+                const double beta = scal[4];
+                const double sv = acc + beta * vp[1][t];
+                const double pr = Rc[row0 + t] + beta * vp[0][t];
+                vp[1][t] = sv;
+                vp[0][t] = pr;
+                dps += pr * sv;
             }
-            double acc = 0.0;
-            for (int k0 = 0; k0 < w; k0 += kS2U) {
-                float vn[kS2U];
-                short on[kS2U];
+        };
+#pragma unroll 1
+        for (int q = 0; q < nck; ++q) {
+            unsigned d, p;
+            if (kRes) {
+                const uint2 e = reinterpret_cast<const uint2*>(sdesc)[q];
+                d = e.y;
+                p = (e.x - (unsigned)c0) * COL;
+            } else {
+                if (!s2_wait(s2_smem_u32(bars + gs), parity)) ok = false;
+                d = sdesc[gs];
+                p = ring + gs * CB;
+            }
+            const int kc = (int)(d & 15u);
+            slice = (int)(d >> 6);
+            const double* Rr = Rc + min(32 * slice + lane, n - 1);
+            if (d & 16u) owner = true;
+            open = true;
+            if (kc == kS2Chunk) {
+                const uint4 o = *reinterpret_cast<const uint4*>(s2_dyn + p + kS2Chunk * 32 * sizeof(M) + 16 * lane);
+                const unsigned w[4] = {o.x, o.y, o.z, o.w};
+                double g[kS2Chunk];
 #pragma unroll
-                for (int u = 0; u < kS2U; ++u) {
-                    // the arrays carry 64 kS2U zero entries past the last slice
-                    vn[u] = __ldcs(a.val + base + 32 * (k0 + kS2U + u));
-                    on[u] = __ldcs(a.off + base + 32 * (k0 + kS2U + u));
+                for (int u = 0; u < kS2Chunk; ++u) g[u] = Rr[u % 2 ? (int)w[u / 2] >> 16 : (int)(short)(w[u / 2] & 0xffffu)];
+                S2Lane<M> c;
+                c.load(s2_dyn + p + 16 * lane);
+                if (!kRes) {
+                    // the values are in registers: the stage takes the chunk one ring ahead
+                    __syncwarp();
+                    if (lane == 0) issue(gs);
                 }
 #pragma unroll
-                for (int u = 0; u < kS2U; ++u) {
-                    if (k0 + u < w) {
-                        const float2 q = a.recF[r + (int)o[u]];
-                        const double pj = first ? (double)q.x : (double)q.x + beta * (double)q.y;
-                        acc = acc + (double)v[u] * pj;
+                for (int u = 0; u < kS2Chunk; u += 2) {
+                    acc0 = acc0 + (double)c.x[u] * g[u];
+                    acc1 = acc1 + (double)c.x[u + 1] * g[u + 1];
+                }
+            } else {
+                const short* o = reinterpret_cast<const short*>(s2_dyn + p + kc * 32 * (int)sizeof(M)) + lane;
+                const M* v = reinterpret_cast<const M*>(s2_dyn + p) + lane;
+#pragma unroll 1
+                for (int u = 0; u < kc; ++u) acc0 = acc0 + (double)v[32 * u] * Rr[(int)o[32 * u]];
+                if (!kRes) {
+                    __syncwarp();
+                    if (lane == 0) issue(gs);
+                }
+            }
+            if (!kRes && ++gs == nload) {
+                gs = 0;
+                parity ^= 1u;
+            }
+            if (d & 32u) {
+                const double acc = acc0 + acc1;
+                acc0 = acc1 = 0.0;
+                if (owner)
+                    finish(acc);
+                else
+                    carry[32 * wid + lane] = acc;
+                owner = open = false;
+            }
+        }
+        const double acc = acc0 + acc1;
+        if (open && !owner) carry[32 * wid + lane] = acc;
+        __syncthreads();
+        if (open && owner) {
+            double t = acc;
+            for (unsigned m = cont; m; m &= m - 1) t = t + carry[32 * (__ffs(m) - 1) + lane];
+            finish(t);
+        }
+        // coupled faces: w_f . P and z_f . P over the slices that touch them
+        if (own_faces) {
+            __syncthreads();
+            for (unsigned m = own_faces; m; m &= m - 1) {
+                const int f = __ffs(m) - 1;
+                double wv = 0.0, zv = 0.0;
+                for (int sl = wid; sl < nsl; sl += nw)
+                    if ((mask[sl] >> f) & 1) {
+                        const int t = 32 * sl + lane;
+                        if (row0 + t < n) {
+                            const double pr = vp[0][t];
+                            wv += vp[3][f * ldw + t] * pr;
+                            zv += vp[4][f * ldw + t] * pr;
+                        }
                     }
-                }
-#pragma unroll
-                for (int u = 0; u < kS2U; ++u) {
-                    v[u] = vn[u];
-                    o[u] = on[u];
-                }
-            }
-            const double2 ra = a.recA[r];
-            const double pr = first ? ra.x : ra.x + beta * ra.y;
-            a.SPr[r] = acc;
-            dps += pr * acc;
-#pragma unroll
-            for (int f = 0; f < NF; ++f)
-                if (f < a.nface) {
-                    wp[f] += a.w[(size_t)f * n + r] * pr;
-                    zp[f] += a.z[(size_t)f * n + r] * pr;
-                }
-        }
-        dps = block_sum(dps, sm);
-        if (threadIdx.x == 0) part1[(size_t)blockIdx.x * kS2PartStride] = dps;
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            if (f < a.nface) {
-                const double tw = block_sum(wp[f], sm);
-                const double tz = block_sum(zp[f], sm);
-                if (threadIdx.x == 0) {
-                    part1[(size_t)blockIdx.x * kS2PartStride + 1 + f] = tw;
-                    part1[(size_t)blockIdx.x * kS2PartStride + 1 + kS2MaxFaces + f] = tz;
+                wv = warp_sum(wv);
+                zv = warp_sum(zv);
+                if (lane == 0) {
+                    red[32 * (1 + 2 * f) + wid] = wv;
+                    red[32 * (2 + 2 * f) + wid] = zv;
                 }
             }
         }
-        grid.sync();
-        double cS[NF > 0 ? NF : 1];
-        double den = s2_sum_partials(part1, 0, sm);
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            cS[f] = 0.0;
-            if (f < a.nface) {
-                cS[f] = a.coef[f] * s2_sum_partials(part1, 1 + f, sm);
-                den = den - cS[f] * s2_sum_partials(part1, 1 + kS2MaxFaces + f, sm);
-            }
-        }
-        const double alpha = errO / den;
-        // ---- phase 2: SP = SP_raw - sum_f cS_f z_f; X += alpha P, R -= alpha SP, |R|^2 ----
+        dps = warp_sum(dps);
+        if (lane == 0) red[wid] = dps;
+        fail = s2_reduce(a, red, a.nface, own_faces, fpend, ++ep, false, tot, !ok || fail);
+        double den = tot[0];
+        for (int f = 0; f < a.nface; ++f) den = den - a.coef[f] * tot[1 + 2 * f] * tot[2 + 2 * f];
+        const double alpha = scal[0] / den;
+        // ---- phase 2 ----
+        double* Rw = a.R + (size_t)(i & 1) * n;
         double rs = 0.0;
-        for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-            const double2 ra = a.recA[r];
-            const double pr = first ? ra.x : ra.x + beta * ra.y;
-            double sp = a.SPr[r];
-#pragma unroll
-            for (int f = 0; f < NF; ++f)
-                if (f < a.nface) sp = sp - cS[f] * a.z[(size_t)f * n + r];
-            a.X[r] = a.X[r] + alpha * pr;
-            const double rv = ra.x - alpha * sp;
-            a.recA[r] = make_double2(rv, pr);
-            a.recF[r] = make_float2((float)rv, (float)pr);
+        for (int sl = wid; sl < nsl; sl += nw) {
+            const int t = 32 * sl + lane, r = row0 + t;
+            if (r >= n) continue;
+            double sv = vp[1][t];
+            for (unsigned m = mask[sl]; m; m &= m - 1) {
+                const int f = __ffs(m) - 1;
+                sv = sv - a.coef[f] * tot[1 + 2 * f] * vp[4][f * ldw + t];
+            }
+            vp[2][t] = vp[2][t] + alpha * vp[0][t];
+            const double rv = Rc[r] - alpha * sv;
+            Rw[r] = rv;
             rs += rv * rv;
         }
-        rs = block_sum(rs, sm);
-        if (threadIdx.x == 0) part2[(size_t)blockIdx.x * kS2PartStride] = rs;
-        grid.sync();
-        const double e2 = sqrt(s2_sum_partials(part2, 0, sm));
-        err = e2 * e2;
+        rs = warp_sum(rs);
+        if (lane == 0) red[wid] = rs;
+        fail = s2_reduce(a, red, 0, 0u, fpend, ++ep, true, tot, fail);
+        if (threadIdx.x == 0) {
+            const double e2 = sqrt(tot[0]), err = e2 * e2;
+            scal[4] = err / scal[0];
+            scal[1] = scal[0];
+            scal[0] = err;
+        }
+        __syncthreads();
     }
+    // the copies still under way, one per stage
+    for (int q = 0; q < nload && ok; ++q) {
+        ok = s2_wait(s2_smem_u32(bars + gs), parity);
+        if (++gs == nload) {
+            gs = 0;
+            parity ^= 1u;
+        }
+    }
+    for (int t = threadIdx.x; t < 32 * nsl; t += blockDim.x)
+        if (row0 + t < n) a.rhs[row0 + t] = vp[2][t];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.out[0] = err;
-        a.out[1] = errO;
+        a.out[0] = scal[0];
+        a.out[1] = scal[1];
         a.out[2] = (double)i;
-        a.out[3] = (double)suc;
+        a.out[3] = fail ? -1.0 : (double)suc;
+        a.out[4] = scal[3];
     }
 }
 
-// recA = {R, 0}, recF = {R, 0}
-__global__ void k_s2_init(const double* __restrict__ R, double2* __restrict__ recA, float2* __restrict__ recF, int n) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        recA[t] = make_double2(R[t], 0.0);
-        recF[t] = make_float2((float)R[t], 0.0f);
-    }
-}
-
-// One CGRAD call on the explicit operator: R (n) holds the right side and
-// receives nothing (the solution is left in L->cgX); out (4 doubles, device)
-// receives err, errO, the iteration index and the success flag.
-int cg_schur_launch(crimson_lhs* L, const double* R, int nface, const double* coef, const double* w, const double* z,
-                    double eps, double err0, int mItr, double* out) {
+// One CGRAD call: R (n) holds the right side and receives the solution; out
+// (5 doubles, device) receives err, errO, the iteration index, the success
+// flag and the initial norm.
+template <typename M>
+int cg_schur_launch(crimson_lhs* L, double* R, int nface, const double* coef, double relTol, double absTol, int mItr,
+                    double* out) {
     if (L->s2_state != 1 || nface > kS2MaxFaces) return CRIMSON_ERR_STATE;
     cudaStream_t s = L->stream;
-    const int n = L->nNo;
-    const void* kfn[3] = {(const void*)k_cg_schur<0>, (const void*)k_cg_schur<1>,
-                          (const void*)k_cg_schur<kS2MaxFaces>};
-    const int fi = nface == 0 ? 0 : (nface == 1 ? 1 : 2);
-    if (L->s2_grid == 0) {
-        int nb = 1 << 30;
-        for (const void* f : kfn) {
-            int b = 0;
-            CR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kS2CgThreads, 0));
-            nb = std::min(nb, b);
-        }
-        if (nb < 1) return CRIMSON_ERR_UNSUPPORTED;
-        L->s2_grid = sm_count() * std::min(nb, 2);
+    const size_t n = (size_t)L->nNo;
+    constexpr size_t kStatic = 8 * 1024;   // static shared memory (red, tot) and the driver's reserve
+    const size_t budget = 227 * 1024 - kStatic;
+    const int nw = L->s2_warps;
+    const size_t cb = (size_t)kS2Chunk * s2_col_bytes<M>();
+    const size_t vec1 = sizeof(double) * (size_t)L->s2_max_rows;
+    const size_t fixed = sizeof(double) * 32 * (size_t)nw + sizeof(unsigned) * (size_t)(L->s2_max_rows / 32) + 16;
+    const size_t own = (size_t)L->s2_max_cols * s2_col_bytes<M>() + sizeof(uint2) * (size_t)L->s2_max_chunks;
+    // everything in shared memory, or a ring per warp
+    const bool res = fixed + 3 * vec1 + own <= budget;
+    // two stages per warp: more of them take the L1 from the gathers (4M-tet
+    // cylinder, two / three stages: 80.7 / 85 us per FP64 iteration)
+    constexpr int stages = 2;
+    const size_t ring = (cb + sizeof(unsigned long long) + sizeof(unsigned)) * nw * stages;
+    // vectors in shared memory.  Resident: P, SP, X and the faces' w and z.
+    // Streaming: P and SP where that leaves at least 64 KB of L1 (4M-tet
+    // cylinder, with / without: 56.6 / 58.1 us FP32, 82.3 / 80.7 us FP64,
+    // where it would not).
+    int nvec = res ? 3 + 2 * nface : 2;
+    if (res && fixed + nvec * vec1 + own > budget) nvec = 3;
+    if (!res && fixed + ring + 2 * vec1 > (size_t)160 * 1024) nvec = 0;
+    const size_t smem = fixed + nvec * vec1 + (res ? own : ring);
+    const void* kfn = res ? (const void*)k_cg_schur<M, true> : (const void*)k_cg_schur<M, false>;
+    // the same value for every lhs: host threads that launch side by side set it alike
+    CR_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
+    CR_CHECK(L->s2_R.alloc(2 * n));
+    if (nvec < 2) {
+        CR_CHECK(L->cgPd.alloc(n));
+        CR_CHECK(L->cgSP.alloc(n));
     }
-    CR_CHECK(L->s2_part.alloc(2 * (size_t)kS2PartStride * L->s2_grid));
-    CR_CHECK(L->cgRecA.alloc(2 * (size_t)n));
-    CR_CHECK(L->s2_recF.alloc((size_t)n));
-    CR_CHECK(L->cgSP.alloc((size_t)n));
-    CR_CUDA(cudaMemsetAsync(L->cgX.p, 0, sizeof(double) * n, s));
-    launch(k_s2_init, grid_for(n, 256), 256, 0, s, R, reinterpret_cast<double2*>(L->cgRecA.p), L->s2_recF.p, n);
+    if (nvec < 3) CR_CHECK(L->cgX.alloc(n));
     CgS2Args a;
-    a.sp = L->s2_sp.p;
-    a.off = L->s2_off.p;
-    a.val = L->s2_val.p;
-    a.n = n;
-    a.X = L->cgX.p;
-    a.recA = reinterpret_cast<double2*>(L->cgRecA.p);
-    a.recF = L->s2_recF.p;
-    a.SPr = L->cgSP.p;
+    a.op = s2_op(L, (const M*)nullptr).p;
+    a.desc = L->s2_desc.p;
+    a.wl = L->s2_wl.p;
+    a.blk = L->s2_blk.p;
+    a.mask = L->s2_mask.p;
+    a.nslice = L->s2_nslice;
+    a.n = L->nNo;
+    a.sc = L->s2_sc.p;
+    a.stages = stages;
+    a.max_cols = L->s2_max_cols;
+    a.nvec = nvec;
+    a.max_rows = L->s2_max_rows;
+    a.evict_first = s2_op(L, (const M*)nullptr).n > (size_t)80 << 20;
+    a.rhs = R;
+    a.R = L->s2_R.p;
+    a.Pg = L->cgPd.p;
+    a.SPg = L->cgSP.p;
+    a.Xg = L->cgX.p;
     a.nface = nface;
-    a.w = w;
-    a.z = z;
+    a.w = L->cgW.p;
+    a.z = L->cgZ.p;
     for (int f = 0; f < kS2MaxFaces; ++f) a.coef[f] = f < nface ? coef[f] : 0.0;
-    a.eps = eps;
-    a.err0 = err0;
+    a.relTol = relTol;
+    a.absTol = absTol;
     a.mItr = mItr;
-    a.part = L->s2_part.p;
+    a.pk = L->s2_pk.p;
+    a.epoch = L->s2_epoch;
     a.out = out;
+    L->s2_epoch += 2ull * (unsigned long long)std::max(mItr, 0) + 2;
     void* kargs[] = {&a};
     note_launch();
-    CR_CUDA(cudaLaunchCooperativeKernel(kfn[fi], dim3(L->s2_grid), dim3(kS2CgThreads), kargs, 0, s));
+    CR_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(L->s2_grid), dim3(32 * nw), kargs, smem, s));
     return CRIMSON_OK;
 }
+template int cg_schur_launch<double>(crimson_lhs*, double*, int, const double*, double, double, int, double*);
+template int cg_schur_launch<float>(crimson_lhs*, double*, int, const double*, double, double, int, double*);
 
 }  // namespace crimson

@@ -142,9 +142,8 @@ class FlowParams:
     max_refine: int = 4
     refine_tol: float = 0.0
     # Mixed precision only: 1 runs the inner CG on the explicit FP32 Schur
-    # operator S = L - Gt G formed once per NS solve, 0 (default: measured
-    # faster on the 4M-tet cylinder, 0.0739 vs 0.0765 ms per CG iteration) on
-    # the two FP32 products L P and Gt (G P) (crimson_memls_ls_set_schur).
+    # operator S = L - Gt G formed once per NS solve, 0 (default) on the two
+    # FP32 products L P and Gt (G P) (crimson_memls_ls_set_schur).
     explicit_schur: int = 0
 
     def outlets(self) -> list:

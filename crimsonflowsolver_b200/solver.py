@@ -241,8 +241,9 @@ class MemLS:
 
     def schur_info(self):
         """(state, nnz, sliced positions, average formation ms) of the explicit
-        FP32 Schur operator on this lhs (state 1: in use, 0: not built, -1:
-        the pattern does not allow it)."""
+        Schur operator on this lhs (state 1: in use, -1: the pattern does not
+        allow it, 0: no solve with explicit_schur = 1 has run; entries 0: no
+        solve uses it)."""
         st, nnz, npad, fm = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_longlong(), ctypes.c_double()
         N.check(N.lib().crimson_memls_schur_info(self.lhs, ctypes.byref(st), ctypes.byref(nnz), ctypes.byref(npad),
                                                  ctypes.byref(fm)), "crimson_memls_schur_info")

@@ -163,18 +163,15 @@ int crimson_memls_ls_free(crimson_ls* ls);
  * (on a small cylinder after 2 steps of 3 iterations: 1e-6 velocity, 4e-5
  * pressure relative to the FP64 tangent). */
 int crimson_memls_ls_set_precision(crimson_ls* ls, int precision, int max_refine, double refine_tol);
-/* Inner CG form of the mixed-precision solve (no counterpart in the
- * reference, which has only FP64).  explicit_schur = 1: each
- * NSSOLVER call forms the continuity Schur operator S = L - Gt G in FP64 on
- * the 2-ring pattern, rounds it to FP32, and CGRAD multiplies by S (one
- * sparse product and two grid barriers per iteration); the pattern is built
- * on the first mixed solve of an lhs and is used when every |col - row| of
- * the 2-ring fits 16 bits and no row has more than 256 entries.
- * explicit_schur = 0 (the default): CGRAD multiplies by L and Gt G as two
- * FP32 products, as memLS does in FP64.  On the 4M-tet cylinder one CG
- * iteration takes 0.0765 ms with the explicit operator and 0.0739 ms with the
- * two products: S has about 4 times the entries of the block pattern, which
- * cancels its single product per iteration.  FP64 solves are unaffected. */
+/* Form of the inner CG's operator (no counterpart in the reference).  CGRAD
+ * multiplies by S = L - Gt G.  FP64 solves form S once per NSSOLVER call on
+ * the node graph's 2-ring where the pattern allows (every |col - row| of the
+ * 2-ring fits 16 bits, no row of it has more than 256 entries), which makes
+ * an iteration one sparse product and two grid barriers; on other patterns
+ * they multiply by L and Gt G as two products, as memLS does.  The
+ * mixed-precision solve multiplies by two FP32 products (explicit_schur = 0,
+ * the default) or, with explicit_schur = 1 and where the pattern allows, by S
+ * formed in FP64 and rounded once to FP32. */
 int crimson_memls_ls_set_schur(crimson_ls* ls, int explicit_schur);
 /* Per-solve log in the format of memLS's memLS_NS.log (LOGFILE,
  * flowsolver/src/memLS.f90:1720-1757), appended to path after every solve
@@ -527,13 +524,15 @@ int crimson_pvsq_noalloc(int nsurf, const int* surf_offsets, const int* d_nodes,
  * which: 0 = 3x3 block SpMV (SPARMULVV, K) on the sliced-ELL copy GMRES
  * uses, 2 = SPARMULSV (G), 3 = fused MGS step, 5 = the sliced 3x3 block SpMV
  * with FP32 K (after a mixed solve), 6 = the 3x3 block SpMV on CSR K.
- * which 1 / 4: time of one CGRAD iteration of the persistent CG kernel with
+ * which 1 / 4: time of one CGRAD iteration of its persistent kernel with
  * FP64 / FP32 matrices, averaged over every launch on this lhs so far (CUDA
  * events recorded around each cooperative launch; reps is ignored).
  * Valid after a solve on the lhs. */
 int crimson_memls_kernel_time(crimson_lhs* lhs, int which, int reps, double* ms);
 
-/* Diagnostics: column layout of the persistent CG kernel on this lhs.
+/* Diagnostics: column layout of the two-product CG kernel on this lhs (the
+ * form CGRAD takes where the explicit operator does not apply), for the
+ * precisions it has been solved in.
  * resident64 / resident32 = 1 when the kernel with FP64 / FP32 matrices keeps
  * every block's column indices in shared memory for the whole launch (16-bit
  * offsets col - row; chosen when the offsets fit and two blocks per SM fit
@@ -542,11 +541,12 @@ int crimson_memls_kernel_time(crimson_lhs* lhs, int which, int reps, double* ms)
  * exceed 16 bits).  Valid after a solve on the lhs. */
 int crimson_memls_cg_layout(const crimson_lhs* lhs, int* resident64, int* resident32, long long* smem_bytes);
 
-/* Diagnostics of the explicit FP32 Schur operator (crimson_memls_ls_set_schur)
- * on this lhs: state 1 = built and used by mixed solves, 0 = not built yet,
- * -1 = the pattern does not allow it; nnz / npad = its entries and sliced
- * positions (padding included); form_ms = average time of one formation
- * (CUDA events).  Valid after a mixed solve on the lhs. */
+/* Diagnostics of the explicit Schur operator on this lhs: state 1 = built and
+ * used by the solves whose ls asked for it (crimson_memls_ls_set_schur), -1 =
+ * the pattern does not allow it, 0 = no such solve has run; nnz / npad = its
+ * entries and sliced positions (padding included; 0: not in use, also by FP64
+ * solves); form_ms = average time of one formation (CUDA events).  Valid
+ * after a solve. */
 int crimson_memls_schur_info(const crimson_lhs* lhs, int* state, long long* nnz, long long* npad, double* form_ms);
 
 /* Number of CUDA kernels this library has launched since it was loaded. */
