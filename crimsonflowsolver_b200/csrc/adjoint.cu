@@ -12,14 +12,25 @@
 // The element tangent ElmGMR assembles (e3LHS) is the reference's
 // approximate Jacobian: it omits the derivatives of tauM, tauC, tauBar and
 // of uBar and the viscous-flux projection.  The adjoint needs the exact
-// transposed Jacobian, so each element's residual is re-evaluated in
-// forward-mode dual arithmetic: one thread per element, K derivative
-// directions per pass, and the contraction with the element's lambda is
-// scattered to the nodes.  Per tet the residual depends on 32 local inputs:
-// y_alpha (4 nodes x p,u,v,w), ac_alpha (4 x 3), div q (3: on a linear tet
-// div q = sum_n dN_n . q_n is an element constant) and mu.  The cotangent of
-// div q goes to the nodal qres through dN, and from qres through the
-// transposed lumped projection back to u and mu.
+// transposed Jacobian, so each tet's contraction J = sum_a lambda_a . rl_a is
+// differentiated by hand in reverse: per quadrature point the forward
+// quantities once, then their cotangents, about twice the residual's
+// arithmetic for all 32 local inputs together -- y_alpha (4 nodes x p,u,v,w),
+// ac_alpha (4 x 3), div q (3: on a linear tet div q = sum_n dN_n . q_n is an
+// element constant) and mu.  The cotangent of div q goes to the nodal qres
+// through dN, and from qres through the transposed lumped projection back to
+// u and mu.
+//
+// Scatter as in the assembly: the element kernels write records (the work
+// space of ElmGMR's records), node passes sum them per node in a fixed order;
+// mu's cotangent is summed per block and over the blocks in order.  Only the
+// boundary faces and outlet nodes, few, are added with atomics.
+//
+// Bound by the record traffic (416 B written per tet, 192 B read per tet and
+// node) and the latency of the element kernel's gathers.  On the 1M-tet
+// 3-outlet cylinder the whole product took 8.3 ms with forward-mode dual
+// numbers (four passes of eight directions, 2.2 KB of stack per thread, 64
+// FP64 atomics per tet).
 #include <vector>
 
 #include "common.cuh"
@@ -28,136 +39,6 @@ namespace crimson {
 
 int elmgmr_device(crimson_ctx* c, const double* d_y, const double* d_ac, const double* coef1, const double* coef2,
                   double* d_res, double* d_lhsK, double* d_lhsP, int lhs, float* d_lhs32 = nullptr);
-
-// ---------------------------------------------------------------------------
-// Forward-mode dual numbers
-// ---------------------------------------------------------------------------
-template <int K>
-struct Dual {
-    double v;
-    double d[K];
-};
-
-template <int K>
-__device__ __forceinline__ Dual<K> dconst(double x) {
-    Dual<K> r;
-    r.v = x;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = 0.0;
-    return r;
-}
-// input value x, seeded with unit derivative in slot `slot` (none if out of range)
-template <int K>
-__device__ __forceinline__ Dual<K> dseed(double x, int slot) {
-    Dual<K> r;
-    r.v = x;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = (k == slot) ? 1.0 : 0.0;
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator+(const Dual<K>& a, const Dual<K>& b) {
-    Dual<K> r;
-    r.v = a.v + b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] + b.d[k];
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator-(const Dual<K>& a, const Dual<K>& b) {
-    Dual<K> r;
-    r.v = a.v - b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] - b.d[k];
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator-(const Dual<K>& a) {
-    Dual<K> r;
-    r.v = -a.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = -a.d[k];
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator*(const Dual<K>& a, const Dual<K>& b) {
-    Dual<K> r;
-    r.v = a.v * b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator/(const Dual<K>& a, const Dual<K>& b) {
-    Dual<K> r;
-    r.v = a.v / b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) / b.v;
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator+(const Dual<K>& a, double b) {
-    Dual<K> r = a;
-    r.v += b;
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator+(double a, const Dual<K>& b) {
-    return b + a;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator-(const Dual<K>& a, double b) {
-    Dual<K> r = a;
-    r.v -= b;
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator-(double a, const Dual<K>& b) {
-    return -b + a;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator*(const Dual<K>& a, double b) {
-    Dual<K> r;
-    r.v = a.v * b;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * b;
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator*(double a, const Dual<K>& b) {
-    return b * a;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator/(const Dual<K>& a, double b) {
-    Dual<K> r;
-    r.v = a.v / b;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] / b;
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> operator/(double a, const Dual<K>& b) {
-    Dual<K> r;
-    r.v = a / b.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = -r.v * b.d[k] / b.v;
-    return r;
-}
-template <int K>
-__device__ __forceinline__ Dual<K> dsqrt(const Dual<K>& a) {
-    Dual<K> r;
-    r.v = sqrt(a.v);
-    const double h = 0.5 / r.v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * h;
-    return r;
-}
-__device__ __forceinline__ double dsqrt(double a) { return sqrt(a); }
-template <int K>
-__device__ __forceinline__ double val(const Dual<K>& a) {
-    return a.v;
-}
-__device__ __forceinline__ double val(double a) { return a; }
 
 // ---------------------------------------------------------------------------
 // Element tables and settings
@@ -256,155 +137,13 @@ __device__ __forceinline__ void adj_gijd(const double dx[3][3], double g[6]) {
 }
 
 // ---------------------------------------------------------------------------
-// Interior residual of one tet contracted with lambda:
-//   sum_a lambda_a . rl_a, rl as e3_elem forms it (itau = 0, iconvflow = 2,
-//   no body force, no ALE, flmpr = 0).  yl[n] = (p, u, v, w); acl[n] = (ax,
-//   ay, az); lam[n] = (momentum x, y, z, continuity) rows of node n.
-// ---------------------------------------------------------------------------
-template <typename T>
-__device__ T e3_res_dot(const AdjConst& C, const AdjParams& P, const double shg[4][3], double W, const double gijd[6],
-                        const T yl[4][4], const T acl[4][3], const T divqi[3], const T& mu, const double lam[4][4]) {
-    const double rho = P.rho;
-    const double rhoinv = 1.0 / rho;
-    T g[3][4];  // g[k][d] = d yl(:, d) / d x_k
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int d = 0; d < 4; ++d)
-            g[k][d] = shg[0][k] * yl[0][d] + shg[1][k] * yl[1][d] + shg[2][k] * yl[2][d] + shg[3][k] * yl[3][d];
-    const T rnu = mu * rhoinv;
-    const double dts = P.Dtgl * P.dtsfct;
-    const double gg = gijd[0] * gijd[0] + gijd[1] * gijd[1] + gijd[2] * gijd[2] +
-                      2.0 * (gijd[3] * gijd[3] + gijd[4] * gijd[4] + gijd[5] * gijd[5]);
-    const T visc = 36.0 * (rnu * rnu) * gg;
-    const double ff = P.taucfct / P.dtsfct;
-    const double trG = gijd[0] + gijd[1] + gijd[2];
-    const T divu = g[0][1] + g[1][2] + g[2][3];
-    T acc = 0.0 * rnu;
-    for (int q = 0; q < 4; ++q) {
-        const double* N = C.shp[q];
-        const T pres = N[0] * yl[0][0] + N[1] * yl[1][0] + N[2] * yl[2][0] + N[3] * yl[3][0];
-        T u[3], ac[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            u[i] = N[0] * yl[0][i + 1] + N[1] * yl[1][i + 1] + N[2] * yl[2][i + 1] + N[3] * yl[3][i + 1];
-            ac[i] = N[0] * acl[0][i] + N[1] * acl[1][i] + N[2] * acl[2][i] + N[3] * acl[3][i];
-        }
-        T rL[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            rL[i] = (ac[i] + u[0] * g[0][i + 1] + u[1] * g[1][i + 1] + u[2] * g[2][i + 1]) * rho + g[i][0] - divqi[i];
-        const T uGu = u[0] * (gijd[0] * u[0] + gijd[3] * u[1] + gijd[5] * u[2]) +
-                      u[1] * (gijd[3] * u[0] + gijd[1] * u[1] + gijd[4] * u[2]) +
-                      u[2] * (gijd[5] * u[0] + gijd[4] * u[1] + gijd[2] * u[2]);
-        const T fact = dsqrt((2.0 * dts) * (2.0 * dts) + uGu + visc);
-        const T tauC = rho * 0.125 * fact / trG * ff;
-        const T tauM = 1.0 / fact;
-        T tauBar = rL[0] * (gijd[0] * rL[0] + gijd[3] * rL[1] + gijd[5] * rL[2]) +
-                   rL[1] * (gijd[3] * rL[0] + gijd[1] * rL[1] + gijd[4] * rL[2]) +
-                   rL[2] * (gijd[5] * rL[0] + gijd[4] * rL[1] + gijd[2] * rL[2]);
-        if (val(tauBar) != 0.0) tauBar = tauM / dsqrt(tauBar);
-        T uB[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) uB[i] = u[i] - tauM * rL[i] * rhoinv;
-        const T tmp = tauC * divu - pres;
-        T rNa[3], rG[3][3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            rNa[i] = (ac[i] + uB[0] * g[0][i + 1] + uB[1] * g[1][i + 1] + uB[2] * g[2][i + 1]) * rho;
-            const T tb = tauBar * (rL[0] * g[0][i + 1] + rL[1] * g[1][i + 1] + rL[2] * g[2][i + 1]);
-            const T tm = tauM * rL[i];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                rG[i][j] = mu * (g[j][i + 1] + g[i][j + 1]) + tm * u[j] + tb * rL[j];
-                if (i == j) rG[i][j] = rG[i][j] + tmp;
-            }
-        }
-        // rl(a, 4) += W dN_a . uBar ; rl(a, i) -= W (N_a rNa_i + dN_a . rGNa_i)
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            T c = (shg[a][0] * uB[0] + shg[a][1] * uB[1] + shg[a][2] * uB[2]) * (W * lam[a][3]);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const T ri = N[a] * rNa[i] + shg[a][0] * rG[i][0] + shg[a][1] * rG[i][1] + shg[a][2] * rG[i][2];
-                c = c - ri * (W * lam[a][i]);
-            }
-            acc = acc + c;
-        }
-    }
-    return acc;
-}
-
-// Boundary residual of one face contracted with lambda (e3b/e3bvar rigid
-// wall, as k_asbmfg forms it).  Nodes 0..2 on the face, node 3 interior.
-template <typename T>
-__device__ T e3b_res_dot(const AdjConst& C, const AdjParams& P, const double shg[4][3], const double bn[3],
-                         double WdetJb, int bits, const double* bcb, const T yl[4][4], const T& mu,
-                         const double lam[3][4]) {
-    T g[3][4];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int d = 0; d < 4; ++d)
-            g[k][d] = shg[0][k] * yl[0][d] + shg[1][k] * yl[1][d] + shg[2][k] * yl[2][d] + shg[3][k] * yl[3][d];
-    T tau[3];
-    tau[0] = bn[0] * 2.0 * mu * g[0][1] + bn[1] * (mu * (g[1][1] + g[0][2])) + bn[2] * (mu * (g[2][1] + g[0][3]));
-    tau[1] = bn[0] * (mu * (g[1][1] + g[0][2])) + bn[1] * 2.0 * mu * g[1][2] + bn[2] * (mu * (g[2][2] + g[1][3]));
-    tau[2] = bn[0] * (mu * (g[2][1] + g[0][3])) + bn[1] * (mu * (g[2][2] + g[1][3])) + bn[2] * 2.0 * mu * g[2][3];
-    const T tn = bn[0] * tau[0] + bn[1] * tau[1] + bn[2] * tau[2];
-    T acc = 0.0 * mu;
-    for (int q = 0; q < 3; ++q) {
-        const double* Nb = C.shpb[q];
-        T pres = Nb[0] * yl[0][0] + Nb[1] * yl[1][0] + Nb[2] * yl[2][0];
-        T u[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) u[i] = Nb[0] * yl[0][i + 1] + Nb[1] * yl[1][i + 1] + Nb[2] * yl[2][i + 1];
-        T unm = bn[0] * u[0] + bn[1] * u[1] + bn[2] * u[2];
-        pres = pres - tn;
-        T tt[3] = {tau[0] - bn[0] * tn, tau[1] - bn[1] * tn, tau[2] - bn[2] * tn};
-        T unm_copy = 0.0 * unm;
-        if ((bits >> 1) & 1)
-            if (val(unm) < 0.0) unm_copy = unm;
-        if (bits & 1) {
-            double s = 0.0;
-            for (int n = 0; n < 3; ++n) s += Nb[n] * bcb[6 * n + 0];
-            unm = 0.0 * unm + s;
-        }
-        if ((bits >> 1) & 1) {
-            double s = 0.0;
-            for (int n = 0; n < 3; ++n) s += Nb[n] * bcb[6 * n + 1];
-            pres = 0.0 * pres + s;
-        }
-        if ((bits >> 2) & 1) {
-            double s[3] = {0.0, 0.0, 0.0};
-            for (int n = 0; n < 3; ++n) {
-                s[0] += Nb[n] * bcb[6 * n + 2];
-                s[1] += Nb[n] * bcb[6 * n + 3];
-                s[2] += Nb[n] * bcb[6 * n + 4];
-            }
-            for (int i = 0; i < 3; ++i) tt[i] = 0.0 * tt[i] + s[i];
-        }
-        if ((bits >> 4) & 1) {
-            pres = 0.0 * pres;
-            for (int i = 0; i < 3; ++i) tt[i] = 0.0 * tt[i];
-        }
-        const T rou_copy = P.rho * unm_copy;
-        T rNa[4];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) rNa[i] = (bn[i] * pres - tt[i] - P.stabflux * rou_copy * u[i]) * WdetJb;
-        rNa[3] = unm * WdetJb;
-#pragma unroll
-        for (int n = 0; n < 3; ++n)
-#pragma unroll
-            for (int d = 0; d < 4; ++d) acc = acc - rNa[d] * (Nb[n] * lam[n][d]);
-    }
-    return acc;
-}
-
-// ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
-constexpr int kAdjK = 8;  // derivative directions per pass
+// Element record (the first doubles of ElmGMR's): at 8 a the cotangents of
+// node a's (u, v, w, p) and (ax, ay, az, 0); grad N_a at 32 + 4 a; that of
+// div q at 48.
+constexpr int kAdjRS = 52;
+constexpr int kAdjBlocksPerSM = 8;   // cap of the element kernels' grids (partial sums of mu's cotangent)
 
 // lambda with the rows bc3Res zeroes set to zero (node-major (4, n))
 __global__ void k_adj_mask(const int* __restrict__ iBC, const double* __restrict__ lam, double* __restrict__ out,
@@ -421,103 +160,241 @@ __global__ void k_adj_mask(const int* __restrict__ iBC, const double* __restrict
     }
 }
 
-__device__ __forceinline__ void warp_atomic_add(double v, double* dst) {
-    v = warp_sum(v);
-    if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(dst, v);
+// Metric tensor product G v, G from gijd = (11, 22, 33, 12, 23, 13).
+__device__ __forceinline__ void adj_gv(const double G[6], const double v[3], double o[3]) {
+    o[0] = G[0] * v[0] + G[3] * v[1] + G[5] * v[2];
+    o[1] = G[3] * v[0] + G[1] * v[1] + G[4] * v[2];
+    o[2] = G[5] * v[0] + G[4] * v[1] + G[2] * v[2];
 }
 
-// Interior VJP: one thread per tet, all 32 local directions in 32/K passes.
-// Directions: 0..15 y (node n = k/4, dof (p,u,v,w) = k%4), 16..27 ac
-// (node (k-16)/3, comp (k-16)%3), 28..30 div q, 31 mu.
-__global__ void __launch_bounds__(64) k_adj_interior(const int4* __restrict__ ien, const double4* __restrict__ x,
-                                                     const double4* __restrict__ y, const double4* __restrict__ ac,
-                                                     const double* __restrict__ qres, const double4* __restrict__ lam,
-                                                     int nelem, AdjConst C, AdjParams P, double mu,
-                                                     double* __restrict__ ybar, double* __restrict__ abar,
-                                                     double* __restrict__ qbar, double* __restrict__ mubar) {
-    using D = Dual<kAdjK>;
+// Sum over an element's four lanes (fixed butterfly).
+__device__ __forceinline__ double adj_quad_sum(double v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return v;
+}
+
+// Interior cotangents, four lanes per tet: lane q evaluates quadrature point
+// q, lane a writes node a (one lane per tet holds the sums of all points and
+// nodes in 255 registers and spills).  Forward per point: u, ac, p,
+//   L_i = rho (ac_i + u . grad u_i) + p,i - divq_i,   F = sqrt(. + u.Gu + .)
+//   tauM = 1/F, tauC = kC F, B = L.GL, tauB = tauM / sqrt(B)
+//   uB = u - tauM L / rho, h_i = L . grad u_i, rN_i = rho (ac_i + uB . grad u_i)
+//   rG_ij = mu (u_i,j + u_j,i) + tauM L_i u_j + tauB h_i L_j + d_ij (tauC div u - p)
+//   J = W sum_q [ Lc . uB - l . rN - Lm_ij rG_ij ]
+// with Lc_j = sum_a lambda_a4 N_a,j, Lm_ij = sum_a lambda_ai N_a,j (element
+// constants) and l_i = sum_a lambda_ai N_a.
+__global__ void __launch_bounds__(128) k_adj_interior(const int4* __restrict__ ien, const double4* __restrict__ x,
+                                                      const double4* __restrict__ y, const double4* __restrict__ ac,
+                                                      const double* __restrict__ qres, const double4* __restrict__ lam,
+                                                      int nelem, AdjConst C, AdjParams P, double mu,
+                                                      double* __restrict__ erec, double* __restrict__ mupart) {
+    __shared__ double sm[32];
+    const int q = threadIdx.x & 3;
     double mub = 0.0;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += gridDim.x * blockDim.x) {
+    const double rho = P.rho, rinv = 1.0 / rho, dts = P.Dtgl * P.dtsfct;
+    double N[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) N[a] = C.shp[q][a];
+    // block-uniform loop: the shuffles always see all lanes; lanes past the
+    // last tet work on the last one and write nothing
+    for (int e0 = blockIdx.x * (blockDim.x >> 2); e0 < nelem; e0 += gridDim.x * (blockDim.x >> 2)) {
+        const bool live = e0 + (int)(threadIdx.x >> 2) < nelem;
+        const int e = live ? e0 + (int)(threadIdx.x >> 2) : nelem - 1;
         const int4 nn = ien[e];
         const int nd[4] = {nn.x, nn.y, nn.z, nn.w};
-        double xl[4][3], yv[4][4], av[4][3], lm[4][4];
+        double shg[4][3], W, G[6];
+        {
+            double xl[4][3], dxidx[3][3];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const double4 xx = x[nd[a]];
+                xl[a][0] = xx.x;
+                xl[a][1] = xx.y;
+                xl[a][2] = xx.z;
+            }
+            adj_metric(xl, C.Qwt, dxidx, shg, &W);
+            adj_gijd(dxidx, G);
+        }
+        double Lm[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, Lc[3] = {0, 0, 0};
+        double g[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};   // g[k][i] = u_i,k
+        double u[3] = {0, 0, 0}, L[3] = {0, 0, 0}, l[3] = {0, 0, 0}, res[3] = {0, 0, 0};
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            const double4 xx = x[nd[a]];
-            const double4 yy = y[nd[a]];
-            const double4 aa = ac[nd[a]];
-            const double4 ll = lam[nd[a]];
-            xl[a][0] = xx.x;
-            xl[a][1] = xx.y;
-            xl[a][2] = xx.z;
-            yv[a][0] = yy.w;
-            yv[a][1] = yy.x;
-            yv[a][2] = yy.y;
-            yv[a][3] = yy.z;
-            av[a][0] = aa.x;
-            av[a][1] = aa.y;
-            av[a][2] = aa.z;
-            lm[a][0] = ll.x;
-            lm[a][1] = ll.y;
-            lm[a][2] = ll.z;
-            lm[a][3] = ll.w;
-        }
-        double dxidx[3][3], shg[4][3], W, gijd[6];
-        adj_metric(xl, C.Qwt, dxidx, shg, &W);
-        adj_gijd(dxidx, gijd);
-        double dq[3] = {0.0, 0.0, 0.0};
-        if (P.idiff >= 1) {
-            for (int a = 0; a < 4; ++a) {
-                const double* q = qres + 9 * (size_t)nd[a];
-                for (int i = 0; i < 3; ++i) dq[i] += shg[a][0] * q[i] + shg[a][1] * q[i + 3] + shg[a][2] * q[i + 6];
-            }
-        }
-        for (int pass = 0; pass < 32 / kAdjK; ++pass) {
-            const int base = pass * kAdjK;
-            D yl[4][4], acl[4][3], dqi[3];
+            const double4 ll = lam[nd[a]], yy = y[nd[a]], aa = ac[nd[a]];
+            const double l3[3] = {ll.x, ll.y, ll.z}, u3[3] = {yy.x, yy.y, yy.z}, a3[3] = {aa.x, aa.y, aa.z};
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
+            for (int j = 0; j < 3; ++j) {
+                u[j] += N[a] * u3[j];
+                L[j] += N[a] * a3[j];   // ac at the point, for now
+                l[j] += N[a] * l3[j];
+                Lc[j] += ll.w * shg[a][j];
+                res[j] += shg[a][j] * yy.w;   // grad p - div q
 #pragma unroll
-                for (int d = 0; d < 4; ++d) yl[a][d] = dseed<kAdjK>(yv[a][d], 4 * a + d - base);
-#pragma unroll
-                for (int i = 0; i < 3; ++i) acl[a][i] = dseed<kAdjK>(av[a][i], 16 + 3 * a + i - base);
-            }
-#pragma unroll
-            for (int i = 0; i < 3; ++i) dqi[i] = dseed<kAdjK>(dq[i], 28 + i - base);
-            const D m = dseed<kAdjK>(mu, 31 - base);
-            const D r = e3_res_dot(C, P, shg, W, gijd, yl, acl, dqi, m, lm);
-#pragma unroll
-            for (int k = 0; k < kAdjK; ++k) {
-                const int dir = base + k;
-                const double v = r.d[k];
-                if (v == 0.0) continue;
-                if (dir < 16) {
-                    const int a = dir / 4, d = dir % 4;
-                    atomicAdd(ybar + 4 * (size_t)nd[a] + (d == 0 ? 3 : d - 1), v);
-                } else if (dir < 28) {
-                    const int a = (dir - 16) / 3, i = (dir - 16) % 3;
-                    atomicAdd(abar + 4 * (size_t)nd[a] + i, v);
-                } else if (dir < 31) {
-                    // div q_i = sum_a sum_j dN_a,j q_a(i + 3j)
-                    const int i = dir - 28;
-                    for (int a = 0; a < 4; ++a)
-                        for (int j = 0; j < 3; ++j) atomicAdd(qbar + 9 * (size_t)nd[a] + i + 3 * j, shg[a][j] * v);
-                } else {
-                    mub += v;
+                for (int i = 0; i < 3; ++i) {
+                    Lm[i][j] += l3[i] * shg[a][j];
+                    g[j][i] += shg[a][j] * u3[i];
                 }
             }
         }
+        if (P.idiff >= 1) {
+            // lane a gathers node a's projected flux
+            const double* f = qres + 9 * (size_t)(q == 0 ? nd[0] : (q == 1 ? nd[1] : (q == 2 ? nd[2] : nd[3])));
+            const double s0 = q == 0 ? shg[0][0] : (q == 1 ? shg[1][0] : (q == 2 ? shg[2][0] : shg[3][0]));
+            const double s1 = q == 0 ? shg[0][1] : (q == 1 ? shg[1][1] : (q == 2 ? shg[2][1] : shg[3][1]));
+            const double s2 = q == 0 ? shg[0][2] : (q == 1 ? shg[1][2] : (q == 2 ? shg[2][2] : shg[3][2]));
+#pragma unroll
+            for (int i = 0; i < 3; ++i) res[i] -= adj_quad_sum(s0 * f[i] + s1 * f[i + 3] + s2 * f[i + 6]);
+        }
+        const double gg = G[0] * G[0] + G[1] * G[1] + G[2] * G[2] + 2.0 * (G[3] * G[3] + G[4] * G[4] + G[5] * G[5]);
+        const double kC = rho * 0.125 / (G[0] + G[1] + G[2]) * (P.taucfct / P.dtsfct);
+        const double f0 = (2.0 * dts) * (2.0 * dts) + 36.0 * (mu * rinv) * (mu * rinv) * gg;
+        const double divu = g[0][0] + g[1][1] + g[2][2], trL = Lm[0][0] + Lm[1][1] + Lm[2][2];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) L[i] = (L[i] + u[0] * g[0][i] + u[1] * g[1][i] + u[2] * g[2][i]) * rho + res[i];
+        double Gu[3], GL[3];
+        adj_gv(G, u, Gu);
+        adj_gv(G, L, GL);
+        const double F = sqrt(f0 + u[0] * Gu[0] + u[1] * Gu[1] + u[2] * Gu[2]);
+        const double tauM = 1.0 / F, tauC = kC * F;
+        const double B = L[0] * GL[0] + L[1] * GL[1] + L[2] * GL[2];
+        const double rB = B != 0.0 ? 1.0 / sqrt(B) : 0.0;
+        const double tauB = tauM * rB;
+        double h[3], ml[3];   // ml_i: minus the cotangent of tauB h_i
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            h[i] = L[0] * g[0][i] + L[1] * g[1][i] + L[2] * g[2][i];
+            ml[i] = Lm[i][0] * L[0] + Lm[i][1] * L[1] + Lm[i][2] * L[2];
+        }
+        // cotangents (without W) of u, L, ac, the gradients gb[k][i], tau and mu at this point
+        double ub[3], Lb[3], acb[3], gb[3][3], tauMb = 0.0, tauBb = 0.0, mb = 0.0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double mu_i = Lm[i][0] * u[0] + Lm[i][1] * u[1] + Lm[i][2] * u[2];
+            const double lt = Lm[0][i] * L[0] + Lm[1][i] * L[1] + Lm[2][i] * L[2];
+            const double ht = Lm[0][i] * h[0] + Lm[1][i] * h[1] + Lm[2][i] * h[2];
+            const double uBb = Lc[i] - rho * (l[0] * g[i][0] + l[1] * g[i][1] + l[2] * g[i][2]);
+            ub[i] = uBb - tauM * lt;
+            Lb[i] = -tauM * mu_i - tauB * (ht + g[i][0] * ml[0] + g[i][1] * ml[1] + g[i][2] * ml[2]) - tauM * rinv * uBb;
+            tauMb -= L[i] * mu_i + uBb * L[i] * rinv;
+            tauBb -= ml[i] * h[i];
+            acb[i] = -rho * l[i];
+        }
+        tauMb += tauBb * rB;
+        const double Bb = -0.5 * tauBb * tauB * rB * rB;
+        // F: tauM = 1/F, tauC = kC F (cotangent -trL div u); F = sqrt(s)
+        const double sb = 0.5 * tauM * (-tauMb * tauM * tauM - kC * trL * divu);
+        mb = sb * 72.0 * mu * rinv * rinv * gg;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            Lb[i] += 2.0 * Bb * GL[i];
+            ub[i] += 2.0 * sb * Gu[i];
+            acb[i] += rho * Lb[i];
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double uBk = u[k] - tauM * L[k] * rinv;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                mb -= Lm[i][k] * (g[k][i] + g[i][k]);
+                gb[k][i] = -mu * (Lm[i][k] + Lm[k][i]) - L[k] * tauB * ml[i] - rho * l[i] * uBk + rho * u[k] * Lb[i];
+                ub[k] += rho * Lb[i] * g[k][i];
+            }
+            gb[k][k] -= trL * tauC;
+        }
+        // over the points: gradients' cotangents, div q's (-Lb), mu's
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) gb[k][i] = adj_quad_sum(gb[k][i]);
+        double gpb[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) gpb[i] = adj_quad_sum(Lb[i]);
+        // node a = q: sum over the points p of N_a(p) times the points' cotangents
+        double yb[3] = {0, 0, 0}, ab[3] = {0, 0, 0};
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const double Na = C.shp[p][q];
+            const int src = (threadIdx.x & 28) | p;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                yb[i] += Na * __shfl_sync(0xffffffffu, ub[i], src);
+                ab[i] += Na * __shfl_sync(0xffffffffu, acb[i], src);
+            }
+        }
+        if (!live) continue;
+        const double s[3] = {q == 0 ? shg[0][0] : (q == 1 ? shg[1][0] : (q == 2 ? shg[2][0] : shg[3][0])),
+                             q == 0 ? shg[0][1] : (q == 1 ? shg[1][1] : (q == 2 ? shg[2][1] : shg[3][1])),
+                             q == 0 ? shg[0][2] : (q == 1 ? shg[1][2] : (q == 2 ? shg[2][2] : shg[3][2]))};
+        double4* r4 = reinterpret_cast<double4*>(erec + (size_t)kAdjRS * e);
+        double o[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) o[i] = W * (yb[i] + s[0] * gb[0][i] + s[1] * gb[1][i] + s[2] * gb[2][i]);
+        r4[2 * q] = make_double4(o[0], o[1], o[2], W * (C.SN[q] * trL + s[0] * gpb[0] + s[1] * gpb[1] + s[2] * gpb[2]));
+        r4[2 * q + 1] = make_double4(W * ab[0], W * ab[1], W * ab[2], 0.0);
+        r4[8 + q] = make_double4(s[0], s[1], s[2], 0.0);
+        if (q == 0) r4[12] = make_double4(-W * gpb[0], -W * gpb[1], -W * gpb[2], 0.0);
+        mub += W * mb;
     }
-    warp_atomic_add(mub, mubar);
+    mub = block_sum(mub, sm);
+    if (threadIdx.x == 0) mupart[blockIdx.x] = mub;
+}
+
+// Lanes per node in the node passes, combined in a fixed butterfly.
+constexpr int kAdjLanes = 4;
+__device__ __forceinline__ double adj_lanes_sum(double v) {
+#pragma unroll
+    for (int o = kAdjLanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Cotangent of qres over the elements at each node, times 1 / rmass (qpbc):
+// div q_i = sum_a sum_j N_a,j q_a(i + 3 j).
+__global__ void __launch_bounds__(256) k_adj_qnode(const int* __restrict__ diag, const int* __restrict__ soff,
+                                                   const int* __restrict__ slist, const double* __restrict__ erec,
+                                                   const double* __restrict__ rmass, int nshg,
+                                                   double* __restrict__ qbar) {
+    constexpr int NPW = 32 / kAdjLanes;
+    const int lane = threadIdx.x & 31, sub = lane % kAdjLanes;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long i0 = warp * NPW; i0 < nshg; i0 += nwarp * NPW) {
+        const long long ig = i0 + lane / kAdjLanes;
+        const bool valid = ig < nshg;
+        const int i = valid ? (int)ig : nshg - 1;
+        const int d = diag[i], p1 = soff[d + 1];
+        double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        for (int p = soff[d] + sub; p < p1; p += kAdjLanes) {
+            const int t = slist[p];
+            const double4* r4 = reinterpret_cast<const double4*>(erec + (size_t)kAdjRS * (t >> 4));
+            const double4 s = r4[8 + ((t >> 2) & 3)], v = r4[12];
+            q[0] += s.x * v.x;
+            q[1] += s.x * v.y;
+            q[2] += s.x * v.z;
+            q[3] += s.y * v.x;
+            q[4] += s.y * v.y;
+            q[5] += s.y * v.z;
+            q[6] += s.z * v.x;
+            q[7] += s.z * v.y;
+            q[8] += s.z * v.z;
+        }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) q[k] = adj_lanes_sum(q[k]);
+        if (!valid || sub != 0) continue;
+        const double r = rmass[i];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) qbar[9 * (size_t)i + k] = r * q[k];
+    }
 }
 
 // Transposed lumped projection (AsIq + qpbc): qres_a = (sum_e W SN_a qdi_e) /
-// rmass_a with qdi = mu (grad u + grad u^T); given qbar, add its cotangent to
-// u and mu.  rinv = 1 / rmass (as qpbc leaves it).
+// rmass_a with qdi = mu (grad u + grad u^T).  Per tet the cotangent of grad u
+// (symmetric: 11, 22, 33, 12, 13, 23 of an 8-double record) and of mu.
 __global__ void __launch_bounds__(128) k_adj_asiq(const int4* __restrict__ ien, const double4* __restrict__ x,
                                                   const double4* __restrict__ y, const double* __restrict__ qbar,
-                                                  const double* __restrict__ rinv, int nelem, AdjConst C, double mu,
-                                                  double* __restrict__ ybar, double* __restrict__ mubar) {
+                                                  int nelem, AdjConst C, double mu, double* __restrict__ grec,
+                                                  double* __restrict__ mupart) {
+    __shared__ double sm[32];
     double mub = 0.0;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += gridDim.x * blockDim.x) {
         const int4 nn = ien[e];
@@ -539,7 +416,7 @@ __global__ void __launch_bounds__(128) k_adj_asiq(const int4* __restrict__ ien, 
         double qb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            const double w = W * C.SN[a] * rinv[nd[a]];
+            const double w = W * C.SN[a];
             const double* q = qbar + 9 * (size_t)nd[a];
 #pragma unroll
             for (int k = 0; k < 9; ++k) qb[k] += w * q[k];
@@ -550,42 +427,73 @@ __global__ void __launch_bounds__(128) k_adj_asiq(const int4* __restrict__ ien, 
 #pragma unroll
             for (int i = 0; i < 3; ++i)
                 g[k][i] = shg[0][k] * ul[0][i] + shg[1][k] * ul[1][i] + shg[2][k] * ul[2][i] + shg[3][k] * ul[3][i];
-        // qdi / mu for the mu cotangent
-        const double s[9] = {2.0 * g[0][0], g[0][1] + g[1][0], g[0][2] + g[2][0], g[0][1] + g[1][0], 2.0 * g[1][1],
-                             g[1][2] + g[2][1], g[0][2] + g[2][0], g[1][2] + g[2][1], 2.0 * g[2][2]};
-#pragma unroll
-        for (int k = 0; k < 9; ++k) mub += qb[k] * s[k];
-        // cotangent of g[k][i]
-        double gb[3][3];
-        gb[0][0] = 2.0 * mu * qb[0];
-        gb[1][1] = 2.0 * mu * qb[4];
-        gb[2][2] = 2.0 * mu * qb[8];
-        gb[0][1] = gb[1][0] = mu * (qb[1] + qb[3]);
-        gb[0][2] = gb[2][0] = mu * (qb[2] + qb[6]);
-        gb[1][2] = gb[2][1] = mu * (qb[5] + qb[7]);
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const double v = shg[b][0] * gb[0][i] + shg[b][1] * gb[1][i] + shg[b][2] * gb[2][i];
-                atomicAdd(ybar + 4 * (size_t)nd[b] + i, v);
-            }
+        const double s12 = qb[1] + qb[3], s13 = qb[2] + qb[6], s23 = qb[5] + qb[7];
+        mub += 2.0 * (qb[0] * g[0][0] + qb[4] * g[1][1] + qb[8] * g[2][2]) + s12 * (g[0][1] + g[1][0]) +
+               s13 * (g[0][2] + g[2][0]) + s23 * (g[1][2] + g[2][1]);
+        double4* r = reinterpret_cast<double4*>(grec + 8 * (size_t)e);
+        r[0] = make_double4(2.0 * mu * qb[0], 2.0 * mu * qb[4], 2.0 * mu * qb[8], mu * s12);
+        r[1] = make_double4(mu * s13, mu * s23, 0.0, 0.0);
     }
-    warp_atomic_add(mub, mubar);
+    mub = block_sum(mub, sm);
+    if (threadIdx.x == 0) mupart[blockIdx.x] = mub;
 }
 
-// Boundary-face VJP: 17 local directions (16 y + mu) in 3 passes.
-__global__ void __launch_bounds__(64) k_adj_faces(const int4* __restrict__ ienb, const int* __restrict__ iBCB,
-                                                  const double* __restrict__ BCB, const double4* __restrict__ x,
-                                                  const double4* __restrict__ y, const double4* __restrict__ lam,
-                                                  int nface, AdjConst C, AdjParams P, double mu,
-                                                  double* __restrict__ ybar, double* __restrict__ mubar) {
-    using D = Dual<kAdjK>;
+// ybar and abar of every node from its elements' records (and the projection
+// records grec, when there are).
+__global__ void __launch_bounds__(256) k_adj_node(const int* __restrict__ diag, const int* __restrict__ soff,
+                                                  const int* __restrict__ slist, const double* __restrict__ erec,
+                                                  const double* __restrict__ grec, int nshg, double4* __restrict__ ybar,
+                                                  double4* __restrict__ abar) {
+    constexpr int NPW = 32 / kAdjLanes;
+    const int lane = threadIdx.x & 31, sub = lane % kAdjLanes;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nwarp = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long i0 = warp * NPW; i0 < nshg; i0 += nwarp * NPW) {
+        const long long ig = i0 + lane / kAdjLanes;
+        const bool valid = ig < nshg;
+        const int i = valid ? (int)ig : nshg - 1;
+        const int d = diag[i], p1 = soff[d + 1];
+        double v[7] = {0, 0, 0, 0, 0, 0, 0};
+        for (int p = soff[d] + sub; p < p1; p += kAdjLanes) {
+            const int t = slist[p], a = (t >> 2) & 3;
+            const double4* r4 = reinterpret_cast<const double4*>(erec + (size_t)kAdjRS * (t >> 4));
+            const double4 yy = r4[2 * a], aa = r4[2 * a + 1];
+            v[0] += yy.x;
+            v[1] += yy.y;
+            v[2] += yy.z;
+            v[3] += yy.w;
+            v[4] += aa.x;
+            v[5] += aa.y;
+            v[6] += aa.z;
+            if (grec) {
+                const double4* q4 = reinterpret_cast<const double4*>(grec + 8 * (size_t)(t >> 4));
+                const double4 s = r4[8 + a], A = q4[0], B = q4[1];
+                v[0] += s.x * A.x + s.y * A.w + s.z * B.x;
+                v[1] += s.x * A.w + s.y * A.y + s.z * B.y;
+                v[2] += s.x * B.x + s.y * B.y + s.z * A.z;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 7; ++k) v[k] = adj_lanes_sum(v[k]);
+        if (!valid || sub != 0) continue;
+        ybar[i] = make_double4(v[0], v[1], v[2], v[3]);
+        abar[i] = make_double4(v[4], v[5], v[6], 0.0);
+    }
+}
+
+// Boundary-face cotangents (e3b/e3bvar rigid wall as k_asbmfg forms it),
+// nodes 0..2 on the face, node 3 interior; added to ybar after the node pass.
+__global__ void __launch_bounds__(128) k_adj_faces(const int4* __restrict__ ienb, const int* __restrict__ iBCB,
+                                                   const double4* __restrict__ x, const double4* __restrict__ y,
+                                                   const double4* __restrict__ lam, int nface, AdjConst C, AdjParams P,
+                                                   double mu, double* __restrict__ ybar,
+                                                   double* __restrict__ mupart) {
+    __shared__ double sm[32];
     double mub = 0.0;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nface; f += gridDim.x * blockDim.x) {
         const int4 nn = ienb[f];
         const int nd[4] = {nn.x, nn.y, nn.z, nn.w};
-        double xl[4][3], yv[4][4], lm[3][4];
+        double xl[4][3], yl[4][4], lm[3][4];
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const double4 xx = x[nd[a]];
@@ -593,10 +501,10 @@ __global__ void __launch_bounds__(64) k_adj_faces(const int4* __restrict__ ienb,
             xl[a][0] = xx.x;
             xl[a][1] = xx.y;
             xl[a][2] = xx.z;
-            yv[a][0] = yy.w;
-            yv[a][1] = yy.x;
-            yv[a][2] = yy.y;
-            yv[a][3] = yy.z;
+            yl[a][0] = yy.x;
+            yl[a][1] = yy.y;
+            yl[a][2] = yy.z;
+            yl[a][3] = yy.w;
         }
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
@@ -607,7 +515,6 @@ __global__ void __launch_bounds__(64) k_adj_faces(const int4* __restrict__ ienb,
             lm[a][3] = ll.w;
         }
         const int bits = iBCB[f];
-        const double* bcb = BCB + 18 * (size_t)f;
         double dxidx[3][3], shg[4][3], Wtmp;
         adj_metric(xl, C.Qwt, dxidx, shg, &Wtmp);
         double v1[3], v2[3];
@@ -621,31 +528,79 @@ __global__ void __launch_bounds__(64) k_adj_faces(const int4* __restrict__ ienb,
         const double t3 = v1[0] * v2[1] - v2[0] * v1[1];
         const double temp = 1.0 / sqrt(t1 * t1 + t2 * t2 + t3 * t3);
         const double bn[3] = {t1 * temp, t2 * temp, t3 * temp};
-        const double WdetJb = C.Qwtb / (4.0 * temp);
-        for (int pass = 0; pass < 3; ++pass) {
-            const int base = pass * kAdjK;
-            D yl[4][4];
+        const double Wb = C.Qwtb / (4.0 * temp);
+        // natural pressure (bit 1) replaces the pressure, bit 2 the traction,
+        // bit 4 both, bit 0 the normal velocity of the continuity row
+        const bool pres_live = !(bits & 2) && !(bits & 16), tt_live = !(bits & 4) && !(bits & 16);
+        double taub[3] = {0, 0, 0}, ybn[3][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}, {0, 0, 0, 0}};
+        for (int q = 0; q < 3; ++q) {
+            const double* Nb = C.shpb[q];
+            double u[3], l[4], pres = 0.0;
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int i = 0; i < 3; ++i) u[i] = Nb[0] * yl[0][i] + Nb[1] * yl[1][i] + Nb[2] * yl[2][i];
 #pragma unroll
-                for (int d = 0; d < 4; ++d) yl[a][d] = dseed<kAdjK>(yv[a][d], 4 * a + d - base);
-            const D m = dseed<kAdjK>(mu, 16 - base);
-            const D r = e3b_res_dot(C, P, shg, bn, WdetJb, bits, bcb, yl, m, lm);
+            for (int d = 0; d < 4; ++d) l[d] = Nb[0] * lm[0][d] + Nb[1] * lm[1][d] + Nb[2] * lm[2][d];
+            const double unm = bn[0] * u[0] + bn[1] * u[1] + bn[2] * u[2];
+            const bool back = (bits & 2) && unm < 0.0;
+            const double sf = P.stabflux * P.rho * (back ? unm : 0.0);
+            // rNa_i = (bn_i pres - tt_i - stabflux rho unm_copy u_i) Wb, rNa_4 = unm Wb; J = -l . rNa
+            double rb[3], presb = 0.0, tnb = 0.0, unb = bits & 1 ? 0.0 : -l[3] * Wb;
 #pragma unroll
-            for (int k = 0; k < kAdjK; ++k) {
-                const int dir = base + k;
-                const double v = r.d[k];
-                if (v == 0.0 || dir > 16) continue;
-                if (dir < 16) {
-                    const int a = dir / 4, d = dir % 4;
-                    atomicAdd(ybar + 4 * (size_t)nd[a] + (d == 0 ? 3 : d - 1), v);
-                } else {
-                    mub += v;
-                }
+            for (int i = 0; i < 3; ++i) {
+                rb[i] = -l[i] * Wb;
+                presb += bn[i] * rb[i];
+                if (back) unb -= P.stabflux * P.rho * u[i] * rb[i];
             }
+            if (!pres_live) presb = 0.0;
+            tnb -= presb;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const double ttb = tt_live ? -rb[i] : 0.0;
+                taub[i] += ttb;
+                tnb -= bn[i] * ttb;
+            }
+            pres = presb;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                taub[i] += bn[i] * tnb;
+                const double ub = bn[i] * unb - sf * rb[i];
+#pragma unroll
+                for (int n = 0; n < 3; ++n) ybn[n][i] += Nb[n] * ub;
+            }
+#pragma unroll
+            for (int n = 0; n < 3; ++n) ybn[n][3] += Nb[n] * pres;
+        }
+        // tau_i = mu sum_k bn_k (u_i,k + u_k,i)
+        double gb[3][3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                gb[k][i] = mu * (bn[k] * taub[i] + bn[i] * taub[k]);
+                const double g = shg[0][k] * yl[0][i] + shg[1][k] * yl[1][i] + shg[2][k] * yl[2][i] + shg[3][k] * yl[3][i];
+                mub += (bn[k] * taub[i] + bn[i] * taub[k]) * g;
+            }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            double* o = ybar + 4 * (size_t)nd[a];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                atomicAdd(o + i, (a < 3 ? ybn[a < 3 ? a : 0][i] : 0.0) + shg[a][0] * gb[0][i] + shg[a][1] * gb[1][i] +
+                                     shg[a][2] * gb[2][i]);
+            if (a < 3) atomicAdd(o + 3, ybn[a < 3 ? a : 0][3]);
         }
     }
-    warp_atomic_add(mub, mubar);
+    mub = block_sum(mub, sm);
+    if (threadIdx.x == 0) mupart[blockIdx.x] = mub;
+}
+
+// out = sum of the n partial sums, in order
+__global__ void k_adj_sum(const double* __restrict__ part, int n, double* __restrict__ out) {
+    __shared__ double sm[32];
+    double s = 0.0;
+    for (int t = threadIdx.x; t < n; t += blockDim.x) s += part[t];
+    s = block_sum(s, sm);
+    if (threadIdx.x == 0) *out = s;
 }
 
 // s_k = sum over outlet k's nodes of NABI . v (v = y or lambda), fixed order
@@ -687,13 +642,15 @@ int elmgmr_vjp(crimson_ctx* c, const double* d_y, const double* d_ac, const doub
     // primal residual at (y, ac): also leaves qres and 1/rmass in the context
     CR_CHECK(c->adj_res.alloc(4 * (size_t)n));
     CR_CHECK(elmgmr_device(c, d_y, d_ac, coef1, coef2, d_res ? d_res : c->adj_res.p, nullptr, nullptr, 0));
+    const int nc = c->ncoupled;
     CR_CHECK(c->adj_lam.alloc(4 * (size_t)n));
     CR_CHECK(c->adj_qbar.alloc(9 * (size_t)n));
-    CR_CHECK(c->adj_scal.alloc(4 + 2 * (size_t)std::max(c->ncoupled, 1)));
-    CR_CUDA(cudaMemsetAsync(d_ybar, 0, sizeof(double) * 4 * (size_t)n, s));
-    CR_CUDA(cudaMemsetAsync(d_abar, 0, sizeof(double) * 4 * (size_t)n, s));
-    CR_CUDA(cudaMemsetAsync(c->adj_qbar.p, 0, sizeof(double) * 9 * (size_t)n, s));
-    CR_CUDA(cudaMemsetAsync(c->adj_scal.p, 0, sizeof(double) * c->adj_scal.n, s));
+    // mu's cotangent, lambda . NABI and Q per outlet; then the blocks' partial sums of the former
+    const int gi = grid_for(4LL * c->nelem, 128, kAdjBlocksPerSM), ge = grid_for(c->nelem, 128, kAdjBlocksPerSM);
+    const int gf = c->nface > 0 ? grid_for(c->nface, 128, 4) : 0;
+    const int nscal = 1 + 2 * nc, npart = gi + ge + gf;
+    CR_CHECK(c->adj_scal.alloc((size_t)nscal + npart));
+    double* mupart = c->adj_scal.p + nscal;
     launch(k_adj_mask, grid_for(n, 256), 256, 0, s, (const int*)c->iBC.p, d_lam, c->adj_lam.p, n);
     const AdjConst C = make_adj_consts();
     AdjParams P;
@@ -707,43 +664,45 @@ int elmgmr_vjp(crimson_ctx* c, const double* d_y, const double* d_ac, const doub
     const double4* y4 = reinterpret_cast<const double4*>(d_y);
     const double4* a4 = reinterpret_cast<const double4*>(d_ac);
     const double4* l4 = reinterpret_cast<const double4*>(c->adj_lam.p);
-    double* mub = c->adj_scal.p;
-    launch(k_adj_interior, grid_for(c->nelem, 64, 16), 64, 0, s, (const int4*)c->ien.p, x4, y4, a4,
-           (const double*)c->qres.p, l4, c->nelem, C, P, p.mu, d_ybar, d_abar, c->adj_qbar.p, mub);
-    if (p.idiff == 1)
-        launch(k_adj_asiq, grid_for(c->nelem, 128, 16), 128, 0, s, (const int4*)c->ien.p, x4, y4,
-               (const double*)c->adj_qbar.p, (const double*)c->rmass.p, c->nelem, C, p.mu, d_ybar, mub);
-    if (c->nface > 0)
-        launch(k_adj_faces, grid_for(c->nface, 64, 16), 64, 0, s, (const int4*)c->ienb.p, (const int*)c->iBCB.p,
-               (const double*)c->BCB.p, x4, y4, l4, c->nface, C, P, p.mu, d_ybar, mub);
-    const int nc = c->ncoupled;
-    std::vector<double> hs(2 * (size_t)std::max(nc, 1), 0.0);
+    const int gn = grid_for((long long)kAdjLanes * n, 256);
+    launch(k_adj_interior, gi, 128, 0, s, (const int4*)c->ien.p, x4, y4, a4, (const double*)c->qres.p, l4, c->nelem, C, P,
+           p.mu, c->erec.p, mupart);
+    int np = gi;
+    if (p.idiff == 1) {
+        launch(k_adj_qnode, gn, 256, 0, s, (const int*)c->diag.p, (const int*)c->soff.p, (const int*)c->slist.p,
+               (const double*)c->erec.p, (const double*)c->rmass.p, n, c->adj_qbar.p);
+        launch(k_adj_asiq, ge, 128, 0, s, (const int4*)c->ien.p, x4, y4, (const double*)c->adj_qbar.p, c->nelem, C, p.mu,
+               c->qrec.p, mupart + np);
+        np += ge;
+    }
+    launch(k_adj_node, gn, 256, 0, s, (const int*)c->diag.p, (const int*)c->soff.p, (const int*)c->slist.p,
+           (const double*)c->erec.p, p.idiff == 1 ? (const double*)c->qrec.p : nullptr, n,
+           reinterpret_cast<double4*>(d_ybar), reinterpret_cast<double4*>(d_abar));
+    if (c->nface > 0) {
+        launch(k_adj_faces, gf, 128, 0, s, (const int4*)c->ienb.p, (const int*)c->iBCB.p, x4, y4, l4,
+                c->nface, C, P, p.mu, d_ybar, mupart + np);
+        np += gf;
+    }
+    launch(k_adj_sum, 1, 256, 0, s, (const double*)mupart, np, c->adj_scal.p);
     if (nc > 0) {
         const int* doff = c->d_onode_off.p;
-        DBuf<double> dc1;
-        std::vector<double> h1(nc);
-        for (int k = 0; k < nc; ++k) h1[k] = coef1 ? coef1[k] : 0.0;
-        CR_CHECK(dc1.upload(h1.data(), nc, s));
-        double* sl = c->adj_scal.p + 4;        // s_k = lambda . NABI
-        double* qf = c->adj_scal.p + 4 + nc;   // Q_k = y . NABI
-        launch(k_adj_flow, nc, 256, 0, s, (const int*)c->onodes.p, doff, (const double4*)c->onabi.p, l4,
-               sl);
-        launch(k_adj_flow, nc, 256, 0, s, (const int*)c->onodes.p, doff, (const double4*)c->onabi.p, y4,
-               qf);
-        launch(k_adj_pvsq, dim3(8, nc), 256, 0, s, (const int*)c->onodes.p, doff,
-               (const double4*)c->onabi.p, (const double*)sl, (const double*)dc1.p, nc, d_ybar);
-        CR_CUDA(cudaMemcpyAsync(hs.data(), sl, sizeof(double) * 2 * nc, cudaMemcpyDeviceToHost, s));
-        CR_CUDA(cudaStreamSynchronize(s));  // dc1 is released at scope exit
+        double* sl = c->adj_scal.p + 1;        // s_k = lambda . NABI
+        double* qf = c->adj_scal.p + 1 + nc;   // Q_k = y . NABI
+        launch(k_adj_flow, nc, 256, 0, s, (const int*)c->onodes.p, doff, (const double4*)c->onabi.p, l4, sl);
+        launch(k_adj_flow, nc, 256, 0, s, (const int*)c->onodes.p, doff, (const double4*)c->onabi.p, y4, qf);
+        // coef1 as the primal residual put it on the device
+        launch(k_adj_pvsq, dim3(8, nc), 256, 0, s, (const int*)c->onodes.p, doff, (const double4*)c->onabi.p,
+               (const double*)sl, (const double*)c->coefs.p, nc, d_ybar);
     }
-    double hm = 0.0;
-    CR_CUDA(cudaMemcpyAsync(&hm, mub, sizeof(double), cudaMemcpyDeviceToHost, s));
+    std::vector<double> hs((size_t)nscal, 0.0);
+    CR_CUDA(cudaMemcpyAsync(hs.data(), c->adj_scal.p, sizeof(double) * nscal, cudaMemcpyDeviceToHost, s));
     CR_CUDA(cudaStreamSynchronize(s));
     CR_CUDA(cudaGetLastError());
-    if (mubar) *mubar = hm;
+    if (mubar) *mubar = hs[0];
     for (int k = 0; k < nc; ++k) {
         // p_k = -(Q_k coef1_k) - coef2_k; res(vel) += p_k NABI
-        if (c1bar) c1bar[k] = -hs[nc + k] * hs[k];
-        if (c2bar) c2bar[k] = -hs[k];
+        if (c1bar) c1bar[k] = -hs[1 + nc + k] * hs[1 + k];
+        if (c2bar) c2bar[k] = -hs[1 + k];
     }
     return CRIMSON_OK;
 }
