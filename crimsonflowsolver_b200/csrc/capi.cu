@@ -793,6 +793,8 @@ int crimson_memls_lhs_free(crimson_lhs* L) {
     if (L->hscal) cudaFreeHost(L->hscal);
     if (L->ev0) cudaEventDestroy(L->ev0);
     if (L->ev1) cudaEventDestroy(L->ev1);
+    for (cudaEvent_t e : L->ev_gm)
+        if (e) cudaEventDestroy(e);
     if (L->s2_ev0) cudaEventDestroy(L->s2_ev0);
     if (L->s2_ev1) cudaEventDestroy(L->s2_ev1);
     cudaStream_t s = L->own_stream ? L->stream : nullptr;

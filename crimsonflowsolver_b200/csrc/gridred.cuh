@@ -95,4 +95,38 @@ __device__ __forceinline__ void gr_release() { asm volatile("fence.acq_rel.gpu;"
 // and, past a __syncthreads, to its block.
 __device__ __forceinline__ void gr_acquire() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
+// The reductions of one barrier.  red[32 k + w]: warp w's partial of value k
+// (shared memory); tot[k] (shared) receives the sums, valid on return for
+// every thread.  Value 0 comes from every block and is the barrier itself;
+// values 1 + 2 f and 2 + 2 f (f < nface) come only from the blocks whose
+// own_faces has bit f -- the others' are zero -- and fpend[32 f + lane] says
+// which these are (as gr_all_blocks).  Measured on 148 blocks: three values
+// from every block take 3.0 us where one takes 1.3.  pk: two regions of kvals
+// packets per block.  data: the block's global writes before the call are
+// visible to all blocks after it.  Returns whether a thread of the block gave
+// up a wait, in this call or before it (failed).
+static __device__ __noinline__ bool grid_reduce(ulonglong2* pk, int kvals, const double* red, int nface,
+                                                unsigned own_faces, const unsigned char* fpend, unsigned long long ep,
+                                                bool data, double* tot, bool failed) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, nv = 1 + 2 * nface;
+    pk += (size_t)(ep & 1) * kvals * gridDim.x;
+    bool fail = failed;
+    __syncthreads();
+    for (int k = wid; k < nv; k += nw)
+        if (k == 0 || ((own_faces >> ((k - 1) / 2)) & 1)) {
+            const double v = warp_sum(lane < nw ? red[32 * k + lane] : 0.0);
+            if (lane == 0) {
+                if (data) gr_release();
+                gr_publish(pk + (size_t)k * gridDim.x + blockIdx.x, v, ep);
+            }
+        }
+    for (int k = wid; k < nv; k += nw) {
+        const unsigned pend = k == 0 ? gr_all_blocks() : fpend[32 * ((k - 1) / 2) + lane];
+        const double v = gr_collect(pk + (size_t)k * gridDim.x, pend, ep, &fail);
+        if (data) gr_acquire();
+        if (lane == 0) tot[k] = v;
+    }
+    return __syncthreads_or(fail) != 0;
+}
+
 }  // namespace crimson

@@ -33,6 +33,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "gridred.cuh"
 #include "memls.cuh"
 
 namespace crimson {
@@ -262,11 +263,11 @@ __global__ void __launch_bounds__(256) k_spmv_vv3(const int* __restrict__ rowptr
     }
 }
 
-// KU(i) = sum K(:,j).U(:,col)  (3 -> 1)
+// KU(i) = sum K(:,j).U(:,col)  (3 -> 1), or minuend(i) less it
 template <typename M, typename IN, typename OUT>
 __global__ void __launch_bounds__(256) k_spmv_vs3(const int* __restrict__ rowptr, const int* __restrict__ col,
                                                   const M* __restrict__ K, const IN* __restrict__ U,
-                                                  OUT* __restrict__ KU, int n) {
+                                                  OUT* __restrict__ KU, const double* __restrict__ minuend, int n) {
     CR_ROW_LOOP(n)
     double a = 0.0;
     CR_ROW_BLOCKS(rowptr, col, {
@@ -277,15 +278,16 @@ __global__ void __launch_bounds__(256) k_spmv_vs3(const int* __restrict__ rowptr
         if (ok) a += t;
     })
     a = group_sum(a);
-    if (rv && lane == 0) KU[r] = (OUT)a;
+    if (rv && lane == 0) KU[r] = (OUT)(minuend ? minuend[r] - a : a);
     }
 }
 
-// KU(:,i) = sum K(:,j) U(col)  (1 -> 3)
+// KU(:,i) = sum K(:,j) U(col)  (1 -> 3); with rest, rest = minuend - KU
 template <typename M, typename IN, typename OUT>
 __global__ void __launch_bounds__(256) k_spmv_sv3(const int* __restrict__ rowptr, const int* __restrict__ col,
                                                   const M* __restrict__ K, const IN* __restrict__ U,
-                                                  OUT* __restrict__ KU, int n) {
+                                                  OUT* __restrict__ KU, const double* __restrict__ minuend,
+                                                  double* __restrict__ rest, int n) {
     CR_ROW_LOOP(n)
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
     CR_ROW_BLOCKS(rowptr, col, {
@@ -305,6 +307,11 @@ __global__ void __launch_bounds__(256) k_spmv_sv3(const int* __restrict__ rowptr
         KU[3 * r + 0] = (OUT)a0;
         KU[3 * r + 1] = (OUT)a1;
         KU[3 * r + 2] = (OUT)a2;
+        if (rest) {
+            rest[3 * r + 0] = minuend[3 * r + 0] - a0;
+            rest[3 * r + 1] = minuend[3 * r + 1] - a1;
+            rest[3 * r + 2] = minuend[3 * r + 2] - a2;
+        }
     }
     }
 }
@@ -529,11 +536,11 @@ struct CgArgs {
     const double* w;  // (nface, n)
     const double* z;  // (nface, n)
     double coef[kMaxCoupled];
-    double eps;   // squared tolerance
-    double err0;  // squared initial norm
+    const double* rr;       // squared initial norm
+    double relTol, absTol;
     int mItr;
     double* part;  // 3 regions of kCgPartStride * gridDim
-    double* out;   // err, errO, i, suc
+    double* out;   // err, errO, i, suc, initial norm
 };
 constexpr int kCgPartStride = kMaxCoupled + 2;
 
@@ -606,10 +613,13 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
     const int wbase = kRes ? cg_fill_cols(a.sp, a.scol, n, cg_res) : 0;
     constexpr int U = CgStage<M>::value;
     constexpr int UA = CgStageA<M>::value;
-    double err = a.err0, errO = a.err0;
+    const double norm0 = sqrt(*a.rr);
+    double err = norm0 * norm0, errO = err;
+    double eps = fmax(a.absTol, a.relTol * norm0);
+    eps = eps * eps;
     int suc = 0, i;
     for (i = 1; i <= a.mItr; ++i) {
-        if (err < a.eps) {
+        if (err < eps) {
             suc = 1;
             break;
         }
@@ -764,6 +774,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
         a.out[1] = errO;
         a.out[2] = (double)i;
         a.out[3] = (double)suc;
+        a.out[4] = norm0;
     }
 }
 
@@ -1001,11 +1012,12 @@ enum {
     kSlotErrO = 3,
     kSlotDen = 4,
     kSlotFace = 8,      // up to 16 faces
-    kSlotCg = 24,       // persistent CG outputs (4)
+    kSlotCg = 24,       // persistent CG outputs (5)
+    kSlotGm = 32,       // persistent GMRES outputs (6), two calls
     kSlotH = 64,        // Hessenberg column (sD + 1)
     kSlotY = 64 + 512,  // back-substitution coefficients
     kSlotGram = 64 + 1024,
-    kScalTotal = 64 + 1024 + 4096
+    kScalTotal = 64 + 1024 + 4096 + 1024
 };
 
 struct Ctx {
@@ -1027,12 +1039,12 @@ struct Ctx {
         launch(k_spmv_vv3<M, IN, OUT>, spmv_grid(), 256, 0, s, L->rowptr, L->col, K, U, KU, L->nNo);
     }
     template <typename M, typename IN, typename OUT>
-    void vs3(const M* K, const IN* U, OUT* KU) {
-        launch(k_spmv_vs3<M, IN, OUT>, spmv_grid(), 256, 0, s, L->rowptr, L->col, K, U, KU, L->nNo);
+    void vs3(const M* K, const IN* U, OUT* KU, const double* minuend = nullptr) {
+        launch(k_spmv_vs3<M, IN, OUT>, spmv_grid(), 256, 0, s, L->rowptr, L->col, K, U, KU, minuend, L->nNo);
     }
     template <typename M, typename IN, typename OUT>
-    void sv3(const M* K, const IN* U, OUT* KU) {
-        launch(k_spmv_sv3<M, IN, OUT>, spmv_grid(), 256, 0, s, L->rowptr, L->col, K, U, KU, L->nNo);
+    void sv3(const M* K, const IN* U, OUT* KU, const double* minuend = nullptr, double* rest = nullptr) {
+        launch(k_spmv_sv3<M, IN, OUT>, spmv_grid(), 256, 0, s, L->rowptr, L->col, K, U, KU, minuend, rest, L->nNo);
     }
     template <typename M, typename IN, typename OUT>
     void ss(const M* K, const IN* U, OUT* KU) {
@@ -1077,27 +1089,485 @@ struct Ctx {
 };
 
 // ---------------------------------------------------------------------------
-// One GMRES restart cycle (memLS.f90:715-770) as one persistent cooperative
-// kernel: Arnoldi iterations i = 1..sD with the fused modified Gram-Schmidt
-// order of the launch-per-step path, until |err_i| < eps.  Per iteration:
-// (P1) U(i) = K U(i-1) on the sliced K, with the coupled-face dots
-// S0_f = valM_f . U(i-1) and T_f = valM_f . K U(i-1) of ADDBCMUL; (MGS j)
-// the face terms of ADDBCMUL (op 0, then op 1 with S1_f = T_f + sum_g
-// coef0_g S0_g (valM_f . valM_g)) folded into the first pass, then
-// U(i) -= h_{j-1} U(j-2) and h_j = <U(i), U(j-1)>; (norm) U(i) -= h_i U(i-1)
-// and |U(i)|^2; every block then applies the Givens rotations to the new
-// Hessenberg column (identical arithmetic in every block, so the exit test
-// agrees) and block 0 stores the column and err; (normalize) U(i) /= h_{i+1}.
-// Every reduction is written per block and summed in block order after the
-// grid barrier (two alternating partial regions).  No host round trip per
-// iteration; the host does the back substitution and X update per cycle.
+// GMRES (memLS.f90:681-788) as one persistent cooperative kernel per call:
+// restarts, Arnoldi iterations, Givens rotations, exit tests, back
+// substitution and the update of X, without a host round trip.
+//
+// Per iteration: (P1) w = K u_{i-1} on the sliced K, with the coupled-face
+// dots S0_f = valM_f . u_{i-1} and T_f = valM_f . w of ADDBCMUL; (MGS j) the
+// face terms of ADDBCMUL (op 0, then op 1 with S1_f = T_f + sum_g coef0_g S0_g
+// (valM_f . valM_g)) folded into the first pass, then w -= h_{j-1} u_{j-2} and
+// h_j = <w, u_{j-1}>; (norm) w -= h_i u_{i-1} and |w|^2; every block applies
+// the Givens rotations to the new Hessenberg column (identical arithmetic on
+// identical sums, so the exit test agrees); u_i = w / h_{i+1}.
+//
+// Small and middle meshes are bound by the i + 3 grid barriers of an
+// iteration.  Each of them carries its reduction (gridred.cuh), and only the
+// last one, which publishes u_i to the neighbours' gathers, orders data.  Four
+// lanes share a block row (a row's entries are four dependent load stages for
+// one lane), lane c < 3 then owns component c: its w and the basis vector of
+// the running pass stay in registers (kSlots values each), and the next
+// pass's vector is loaded before the barrier that the pass waits for.  Meshes
+// of more than 150,000 nodes (8 values per thread) are bound by the
+// streams of K and the basis: one lane per row, w in memory (kSlots = 0).
 // ---------------------------------------------------------------------------
-constexpr int kGmThreads = 512;
+// Threads of a block: 128 registers each for the register form, 64 for the
+// streaming one.
+constexpr int gm_threads(int slots) { return slots > 0 ? 512 : 1024; }
 constexpr int kGmMaxSD = 64;
-constexpr int kGmPartStride = 2 * kMaxCoupled + 1;
+constexpr int kGmVals = 1 + 2 * kMaxCoupled;
 
 template <typename M, typename B>
 struct GmArgs {
+    const int* sp;
+    const int* scol;
+    long long npad;
+    int n;
+    const M* Ks;          // sliced K: {K0..K3} (npad), {K4..K7} (npad), K8 (npad)
+    B* u;                 // basis, vector k at u + k n3 (k = 0..sD)
+    long long n3;
+    int sD, mItr;
+    double relTol, absTol;
+    const double* R;      // right side (n3)
+    double* X;            // solution (n3)
+    int nface;            // coupled faces
+    const int* fptr;      // (n + 1) entries of node r: fent[fptr[r] .. fptr[r + 1])
+    const int* fent;      // entry ids grouped by node
+    const int* fface;     // (entries) face of the entry
+    const double* fval;   // (entries, 3) valM of the entry
+    const double* gram;   // (nface, nface) valM_f . valM_g (diagonal: nS)
+    double coef0[kMaxCoupled], coef1[kMaxCoupled];
+    ulonglong2* pk;       // 2 regions of kGmVals packets per block
+    unsigned long long epoch;
+    double* out;          // iterations, suc (-1: a wait ran out), iNorm, fNorm, norm before the last cycle, nothing to do
+};
+
+__device__ __forceinline__ double quad_sum(double v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return v;
+}
+
+// Entries k0, k0 + step, ... of row r of K times U.
+template <int UN, typename M, typename IN>
+__device__ __forceinline__ void gm_row(const int* __restrict__ sp, const int* __restrict__ scol,
+                                       const M* __restrict__ Ks, long long npad, int r, int k0, int step, const IN* U,
+                                       double a[3]) {
+    const int p0 = __ldg(sp + (r >> 5));
+    const int w = (__ldg(sp + (r >> 5) + 1) - p0) >> 5;
+    const int base = p0 + (r & (kSlice - 1));
+    for (int k = k0; k < w; k += step * UN) {
+        int c[UN];
+#pragma unroll
+        for (int q = 0; q < UN; ++q) c[q] = k + step * q < w ? __ldg(scol + base + kSlice * (k + step * q)) : r;
+#pragma unroll
+        for (int q = 0; q < UN; ++q)
+            if (k + step * q < w) {
+                const size_t pos = (size_t)base + (size_t)kSlice * (k + step * q);
+                const IN* u = U + 3 * (size_t)c[q];
+                const double u0 = (double)u[0], u1 = (double)u[1], u2 = (double)u[2];
+                const auto ka = ldcs4(reinterpret_cast<const typename V4<M>::type*>(Ks) + pos);
+                const auto kb = ldcs4(reinterpret_cast<const typename V4<M>::type*>(Ks + 4 * npad) + pos);
+                const double k8 = (double)__ldcs(Ks + 8 * npad + pos);
+                a[0] = a[0] + (double)ka.x * u0 + (double)ka.y * u1 + (double)ka.z * u2;
+                a[1] = a[1] + (double)ka.w * u0 + (double)kb.x * u1 + (double)kb.y * u2;
+                a[2] = a[2] + (double)kb.z * u0 + (double)kb.w * u1 + k8 * u2;
+            }
+    }
+}
+
+template <typename M, typename B, int kSlots>
+__global__ void __launch_bounds__(gm_threads(kSlots), 1) k_gmres(const __grid_constant__ GmArgs<M, B> a) {
+    constexpr bool kReg = kSlots > 0;
+    constexpr int NS = kReg ? kSlots : 1;
+    extern __shared__ double gm_dyn[];
+    __shared__ double red[32 * kGmVals], tot[kGmVals], cf[kMaxCoupled];
+    __shared__ unsigned char fpend[32 * kMaxCoupled];
+    __shared__ int sdone;
+    __shared__ unsigned sown;
+    const int sD = a.sD, ldh = sD + 1;
+    double* const H = gm_dyn;                 // (sD + 1, sD) column-major, rotated
+    double* const sc = H + (size_t)ldh * sD;  // rotations
+    double* const sn = sc + sD;
+    double* const err = sn + sD;              // (sD + 1)
+    double* const yv = err + ldh;             // (sD)
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n = a.n;
+    const int tid0 = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+    // kReg: slot s of this thread is component q of row r0 + s rs; the
+    // warp-uniform bound lets every lane reach the shuffles
+    const int q = kReg ? (int)(threadIdx.x & 3) : 0, r0 = kReg ? tid0 >> 2 : tid0, rs = kReg ? nth >> 2 : nth;
+    unsigned long long ep = a.epoch;
+    bool fail = false;
+    unsigned own = 0;
+    auto reduce = [&](double v, bool data) {   // one value; returns the sum
+        v = warp_sum(v);
+        if (lane == 0) red[wid] = v;
+        fail = grid_reduce(a.pk, kGmVals, red, 0, 0u, fpend, ++ep, data, tot, fail);
+        return tot[0];
+    };
+    // which blocks hold nodes of which face
+    if (a.nface > 0) {
+        if (threadIdx.x == 0) sown = 0u;
+        __syncthreads();
+        unsigned m = 0;
+        for (int r = r0; r < n; r += rs)
+            for (int k = a.fptr[r]; k < a.fptr[r + 1]; ++k) m |= 1u << a.fface[a.fent[k]];
+        m = __reduce_or_sync(0xffffffffu, m);
+        if (lane == 0 && m) atomicOr(&sown, m);
+        __syncthreads();
+        own = sown;
+        if (lane == 0) red[wid] = wid == 0 ? (double)own : 0.0;
+        fail = grid_reduce(a.pk, kGmVals, red, 0, 0u, fpend, ++ep, false, tot, fail);
+        const ulonglong2* pk = a.pk + (size_t)(ep & 1) * kGmVals * gridDim.x;
+        for (int f = wid; f < a.nface; f += blockDim.x >> 5) {
+            unsigned b = 0;
+#pragma unroll
+            for (int j = 0; j < kGrPolls; ++j)
+                if (lane + 32 * j < (int)gridDim.x &&
+                    (((unsigned)__longlong_as_double((long long)gr_load(pk + lane + 32 * j).x) >> f) & 1))
+                    b |= 1u << j;
+            fpend[32 * f + lane] = (unsigned char)b;
+        }
+        __syncthreads();
+    }
+    // face sums of value pairs (v0, v1): per-thread accumulation over the
+    // entries of its rows, then one barrier.  body(fe, f, c, row, &x0, &x1)
+    // adds an entry's component c.
+    auto face_reduce = [&](auto&& body) {
+        for (int f = 0; f < a.nface; ++f) {
+            double x0 = 0.0, x1 = 0.0;
+            if ((own >> f) & 1) {
+                int s = 0;
+                for (int r = r0; r < n; r += rs, ++s)
+                    for (int k = a.fptr[r]; k < a.fptr[r + 1]; ++k) {
+                        const int fe = a.fent[k];
+                        if (a.fface[fe] == f) body(fe, r, s, x0, x1);
+                    }
+            }
+            x0 = warp_sum(x0);
+            x1 = warp_sum(x1);
+            if (lane == 0) {
+                red[32 * (1 + 2 * f) + wid] = x0;
+                red[32 * (2 + 2 * f) + wid] = x1;
+            }
+        }
+        if (lane == 0) red[wid] = 0.0;
+        fail = grid_reduce(a.pk, kGmVals, red, a.nface, own, fpend, ++ep, false, tot, fail);
+    };
+    double w[NS];    // kReg: this thread's values of the running vector (rounded to B)
+#pragma unroll
+    for (int s = 0; s < NS; ++s) w[s] = 0.0;
+    auto at = [&](int s) { return 3 * (size_t)(r0 + s * rs) + q; };                  // kReg: index of slot s
+    auto has = [&](int s) { return q < 3 && r0 + s * rs < n; };
+    B* wm = a.u;     // memory of the running vector (kSlots = 0)
+    // component c of row r of the running vector (kReg: slot s)
+    auto wval = [&](int r, int s, int c) {
+        if (!kReg) return (double)wm[3 * (size_t)r + c];
+        double v = 0.0;
+#pragma unroll
+        for (int z = 0; z < NS; ++z)
+            if (z == s) v = w[z];
+        return v;
+    };
+    // w += sum_f cf_f valM_f at the faces' nodes: each face's term rounded to B
+    // (ADDBCMUL), or their sum (the closed form of its two passes)
+    auto face_add = [&](bool each) {
+        if (!own) return;
+        int s = 0;
+        for (int r = r0; r < n; r += rs, ++s) {
+            const int k0 = a.fptr[r], k1 = a.fptr[r + 1];
+            if (k1 == k0) continue;
+            for (int c = kReg ? q : 0; c < (kReg ? min(q + 1, 3) : 3); ++c) {
+                double v = wval(r, s, c), add = 0.0;
+                for (int k = k0; k < k1; ++k) {
+                    const int fe = a.fent[k];
+                    const double x = a.fval[3 * (size_t)fe + c] * cf[a.fface[fe]];
+                    if (each)
+                        v = (double)(B)(v + x);
+                    else
+                        add += x;
+                }
+                if (!each) v = (double)(B)(v + add);
+                if (kReg) {
+#pragma unroll
+                    for (int z = 0; z < NS; ++z)
+                        if (z == s) w[z] = v;
+                } else {
+                    wm[3 * (size_t)r + c] = (B)v;
+                }
+            }
+        }
+    };
+    // one component per lane (kReg) or all three: adds val . f over them
+    auto dot3 = [&](int fe, auto&& f) {
+        const double* v = a.fval + 3 * (size_t)fe;
+        if (kReg) return q < 3 ? v[q] * f(q) : 0.0;
+        return v[0] * f(0) + v[1] * f(1) + v[2] * f(2);
+    };
+
+    double eps = 0.0, iNorm = 0.0, fNorm = 0.0, dBase = 0.0;
+    int itr = 0, suc = 0, idle = 0;
+    for (int l = 1; l <= a.mItr && !fail; ++l) {
+        // ---- u_0: the preconditioned residual, normalized ----
+        wm = a.u;
+        if (l == 1) {
+            if (kReg) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) w[s] = has(s) ? (double)(B)a.R[at(s)] : 0.0;
+            } else {
+                for (int r = r0; r < n; r += rs)
+                    for (int c = 0; c < 3; ++c) wm[3 * (size_t)r + c] = (B)a.R[3 * (size_t)r + c];
+            }
+        } else {
+            ++itr;
+            if (kReg) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    const int r = r0 + s * rs;
+                    double x[3] = {0.0, 0.0, 0.0};
+                    if (r < n) gm_row<4>(a.sp, a.scol, a.Ks, a.npad, r, q, 4, (const double*)a.X, x);
+                    const double x0 = quad_sum(x[0]), x1 = quad_sum(x[1]), x2 = quad_sum(x[2]);
+                    w[s] = has(s) ? (double)(B)(q == 0 ? x0 : (q == 1 ? x1 : x2)) : 0.0;
+                }
+            } else {
+                for (int r = r0; r < n; r += rs) {
+                    double x[3] = {0.0, 0.0, 0.0};
+                    gm_row<4>(a.sp, a.scol, a.Ks, a.npad, r, 0, 1, (const double*)a.X, x);
+                    for (int c = 0; c < 3; ++c) wm[3 * (size_t)r + c] = (B)x[c];
+                }
+            }
+            if (a.nface > 0) {
+                face_reduce([&](int fe, int r, int, double& x0, double&) {
+                    x0 += dot3(fe, [&](int c) { return a.X[3 * (size_t)r + c]; });
+                });
+                if (threadIdx.x < (unsigned)a.nface) cf[threadIdx.x] = a.coef0[threadIdx.x] * tot[1 + 2 * threadIdx.x];
+                __syncthreads();
+                face_add(true);
+            }
+            if (kReg) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s)
+                    if (has(s)) w[s] = (double)(B)(a.R[at(s)] - w[s]);
+            } else {
+                for (int r = r0; r < n; r += rs)
+                    for (int c = 0; c < 3; ++c) {
+                        const size_t t = 3 * (size_t)r + c;
+                        wm[t] = (B)(a.R[t] - (double)wm[t]);
+                    }
+            }
+        }
+        if (a.nface > 0) {
+            face_reduce([&](int fe, int r, int s, double& x0, double&) {
+                x0 += dot3(fe, [&](int c) { return wval(r, s, c); });
+            });
+            if (threadIdx.x < (unsigned)a.nface) cf[threadIdx.x] = a.coef1[threadIdx.x] * tot[1 + 2 * threadIdx.x];
+            __syncthreads();
+            face_add(true);
+        }
+        double d = 0.0;
+        if (kReg) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s) d += w[s] * w[s];
+        } else {
+            for (int r = r0; r < n; r += rs)
+                for (int c = 0; c < 3; ++c) {
+                    const double v = (double)wm[3 * (size_t)r + c];
+                    d += v * v;
+                }
+        }
+        const double e0 = sqrt(reduce(d, false));
+        if (l == 1) {
+            if (e0 <= a.absTol) {
+                idle = 1;
+                for (int r = r0; r < n; r += rs)
+                    for (int c = kReg ? q : 0; c < (kReg ? min(q + 1, 3) : 3); ++c) a.X[3 * (size_t)r + c] = 0.0;
+                break;
+            }
+            iNorm = fNorm = e0;
+            eps = fmax(a.absTol, a.relTol * e0);
+        }
+        dBase = fNorm;
+        if (threadIdx.x == 0) err[0] = e0;
+        if (kReg) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                if (has(s)) a.u[at(s)] = (B)(w[s] / e0);
+        } else {
+            for (int r = r0; r < n; r += rs)
+                for (int c = 0; c < 3; ++c) {
+                    const size_t t = 3 * (size_t)r + c;
+                    wm[t] = (B)((double)wm[t] / e0);
+                }
+        }
+        reduce(0.0, true);
+        int i;
+        for (i = 1; i <= sD && !fail; ++i) {
+            ++itr;
+            // ---- P1: w = K u_{i-1} ----
+            const B* uin = a.u + (size_t)(i - 1) * a.n3;
+            wm = a.u + (size_t)i * a.n3;
+            if (kReg) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    const int r = r0 + s * rs;
+                    double x[3] = {0.0, 0.0, 0.0};
+                    if (r < n) gm_row<4>(a.sp, a.scol, a.Ks, a.npad, r, q, 4, uin, x);
+                    const double x0 = quad_sum(x[0]), x1 = quad_sum(x[1]), x2 = quad_sum(x[2]);
+                    w[s] = has(s) ? (double)(B)(q == 0 ? x0 : (q == 1 ? x1 : x2)) : 0.0;
+                }
+            } else {
+                for (int r = r0; r < n; r += rs) {
+                    double x[3] = {0.0, 0.0, 0.0};
+                    gm_row<4>(a.sp, a.scol, a.Ks, a.npad, r, 0, 1, uin, x);
+                    for (int c = 0; c < 3; ++c) wm[3 * (size_t)r + c] = (B)x[c];
+                }
+            }
+            B un[NS], up[NS];   // kReg: u_{j-1} of the pass, u_{j-2}
+            if (kReg) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    un[s] = has(s) ? a.u[at(s)] : B(0);
+                    up[s] = B(0);
+                }
+            }
+            if (a.nface > 0) {
+                face_reduce([&](int fe, int r, int s, double& x0, double& x1) {
+                    x0 += dot3(fe, [&](int c) { return (double)uin[3 * (size_t)r + c]; });
+                    x1 += dot3(fe, [&](int c) { return wval(r, s, c); });
+                });
+                if (threadIdx.x < (unsigned)a.nface) {
+                    const int f = threadIdx.x;
+                    double S1 = tot[2 + 2 * f];
+                    for (int g = 0; g < a.nface; ++g) S1 += a.coef0[g] * tot[1 + 2 * g] * a.gram[f * a.nface + g];
+                    cf[f] = a.coef0[f] * tot[1 + 2 * f] + a.coef1[f] * S1;
+                }
+                __syncthreads();
+                face_add(false);
+            }
+            // ---- MGS passes j = 1..i, then the norm (j = i + 1) ----
+            double* const hc = H + (size_t)(i - 1) * ldh;
+            double hp = 0.0;
+            for (int j = 1; j <= i + 1; ++j) {
+                const bool last = j == i + 1;
+                d = 0.0;
+                if (kReg) {
+#pragma unroll
+                    for (int s = 0; s < NS; ++s) {
+                        if (j > 1) w[s] = (double)(B)(w[s] - hp * (double)up[s]);
+                        d += w[s] * (last ? w[s] : (double)un[s]);
+                        up[s] = un[s];
+                    }
+                    if (j < i) {
+                        const B* uj = a.u + (size_t)j * a.n3;
+#pragma unroll
+                        for (int s = 0; s < NS; ++s)
+                            if (has(s)) un[s] = uj[at(s)];
+                    }
+                } else {
+                    const B* uj = last ? wm : a.u + (size_t)(j - 1) * a.n3;
+                    const B* uo = j > 1 ? a.u + (size_t)(j - 2) * a.n3 : wm;
+                    for (int r = r0; r < n; r += rs)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            const size_t t = 3 * (size_t)r + c;
+                            double wv = (double)wm[t];
+                            if (j > 1) {
+                                wv = (double)(B)(wv - hp * (double)uo[t]);
+                                wm[t] = (B)wv;
+                            }
+                            d += wv * (last ? wv : (double)__ldcs(uj + t));
+                        }
+                }
+                hp = reduce(d, false);
+                if (last) hp = sqrt(hp);
+                if (threadIdx.x == 0) hc[j - 1] = hp;
+            }
+            // ---- Givens (memLS.f90:750-760), identical in every block ----
+            if (threadIdx.x == 0) {
+                double h0 = hc[0];
+                for (int j = 1; j <= i - 1; ++j) {
+                    const double h1 = hc[j];
+                    hc[j - 1] = sc[j - 1] * h0 + sn[j - 1] * h1;
+                    h0 = -sn[j - 1] * h0 + sc[j - 1] * h1;
+                }
+                const double t = sqrt(h0 * h0 + hc[i] * hc[i]);
+                sc[i - 1] = h0 / t;
+                sn[i - 1] = hc[i] / t;
+                hc[i - 1] = t;
+                hc[i] = 0.0;
+                err[i] = -sn[i - 1] * err[i - 1];
+                err[i - 1] = sc[i - 1] * err[i - 1];
+                sdone = fabs(err[i]) < eps ? 1 : 0;
+            }
+            __syncthreads();
+            if (sdone) suc = 1;
+            if (sdone || i == sD) break;
+            // ---- normalize ----
+            if (kReg) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s)
+                    if (has(s)) a.u[(size_t)i * a.n3 + at(s)] = (B)(w[s] / hp);
+            } else {
+                for (int r = r0; r < n; r += rs)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const size_t t = 3 * (size_t)r + c;
+                        wm[t] = (B)((double)wm[t] / hp);
+                    }
+            }
+            reduce(0.0, true);
+        }
+        if (fail) break;
+        // ---- back substitution (one warp, columns from the last), X update ----
+        fNorm = fabs(err[i]);
+        if (wid == 0) {
+            for (int k = lane; k < i; k += 32) yv[k] = err[k];
+            __syncwarp();
+            for (int j = i - 1; j >= 0; --j) {
+                const double yj = yv[j] / H[(size_t)j * ldh + j];
+                __syncwarp();
+                if (lane == 0) yv[j] = yj;
+                for (int k = lane; k < j; k += 32) yv[k] = yv[k] - H[(size_t)j * ldh + k] * yj;
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        for (int r = r0; r < n; r += rs)
+            for (int c = kReg ? q : 0; c < (kReg ? min(q + 1, 3) : 3); ++c) {
+                const size_t t = 3 * (size_t)r + c;
+                double xv = l == 1 ? 0.0 : a.X[t];
+#pragma unroll 4
+                for (int j = 0; j < i; ++j) xv = xv + (double)a.u[(size_t)j * a.n3 + t] * yv[j];
+                a.X[t] = xv;
+            }
+        if (suc) break;
+        if (l < a.mItr) reduce(0.0, true);   // the next cycle gathers X
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.out[0] = (double)itr;
+        a.out[1] = fail ? -1.0 : (double)suc;
+        a.out[2] = iNorm;
+        a.out[3] = fNorm;
+        a.out[4] = dBase;
+        a.out[5] = (double)idle;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// One restart cycle as a persistent kernel with cooperative_groups barriers,
+// for the FP32-tangent mode (CRIMSON_MIXED_F32_TANGENT).  There the next
+// nonlinear iteration rounds its tangent to FP32, which turns the 1e-11 by
+// which any other order of summation moves a mixed solve (its basis is
+// rounded to FP32 at every step) into 1e-8 of the time step's result; the
+// mode keeps this kernel's order and with it its results.  Same iteration as
+// k_gmres; restart residual, back substitution and X update on the host.
+// ---------------------------------------------------------------------------
+constexpr int kGmcThreads = 512;
+constexpr int kGmPartStride = 2 * kMaxCoupled + 1;
+
+template <typename M, typename B>
+struct GmcArgs {
     const int* sp;
     const int* scol;
     long long npad;
@@ -1127,7 +1597,7 @@ __device__ __forceinline__ double gm_sum(const double* part, int k, double* sm) 
 }
 
 template <typename M, typename B, int NF>
-__global__ void __launch_bounds__(kGmThreads, 2) k_gmres_cycle(GmArgs<M, B> a) {
+__global__ void __launch_bounds__(kGmcThreads, 2) k_gmres_cycle(GmcArgs<M, B> a) {
     namespace cgrp = cooperative_groups;
     cgrp::grid_group grid = cgrp::this_grid();
     __shared__ double sm[32];
@@ -1410,12 +1880,124 @@ __global__ void k_gm_gram(const int* __restrict__ pairs, int npairs, const int* 
     }
 }
 
+// Coupled-face data of k_gmres for the NSSOLVER call: valM by entry and the
+// faces' valM_f . valM_g.  *ok = 0 when the kernel does not apply (more than
+// kMaxCoupled coupled faces).
+static int gm_faces_prepare(crimson_lhs* L, int* ok) {
+    CR_CHECK(gm_face_map(L, ok));
+    if (!*ok) return CRIMSON_OK;
+    cudaStream_t s = L->stream;
+    FaceNorms nsv{};
+    int off = 0;
+    const int nface = (int)L->gm_faces.size();
+    for (int q = 0; q < nface; ++q) {
+        const MemlsFace& f = L->face[L->gm_faces[q]];
+        launch(k_gm_fval, grid_for(f.nNo, 256), 256, 0, s, (const double*)f.valM.p, f.dof, std::min(f.dof, 3), f.nNo,
+               L->gmFval.p + 3 * (size_t)off);
+        nsv.v[q] = f.nS;
+        off += f.nNo;
+    }
+    if (nface > 0)
+        launch(k_gm_gram, 1, 32, 0, s, (const int*)L->gmPairs.p, L->gm_npairs, (const int*)L->gmFface.p,
+               (const double*)L->gmFval.p, nsv, nface, L->gmGram.p);
+    return CRIMSON_OK;
+}
+
+// Launches k_gmres for K X = R; the outcome goes to the scalar slots at slot
+// (gmres_finish reads them after the stream has been waited for).
+template <typename M, typename B>
+static int gmres_launch(Ctx& C, const crimson_subls& ls, const M* Ks, const double* R, double* X, int slot) {
+    crimson_lhs* L = C.L;
+    cudaStream_t s = C.s;
+    const int n = L->nNo;
+    const int sms = std::min(sm_count(), kGrMaxBlocks);
+    // Four lanes per row and at most 8 values per thread in registers; blocks
+    // of 256 threads until every SM has one, then larger ones.  Larger meshes:
+    // one lane per row.
+    const long long quads = 4LL * n;
+    const bool reg = quads <= 8LL * gm_threads(1) * sms;
+    const int grid = (int)std::max(1LL, std::min<long long>(sms, (quads + 255) / 256));
+    int threads = reg ? 256 : gm_threads(0);
+    while (reg && threads < gm_threads(1) && (long long)grid * threads < quads) threads *= 2;
+    const long long slots = reg ? (quads + (long long)grid * threads - 1) / ((long long)grid * threads) : 0;
+    const void* fns[5] = {(const void*)k_gmres<M, B, 0>, (const void*)k_gmres<M, B, 1>, (const void*)k_gmres<M, B, 2>,
+                          (const void*)k_gmres<M, B, 4>, (const void*)k_gmres<M, B, 8>};
+    const void* kfn = fns[slots > 4 ? 4 : (slots > 2 ? 3 : (int)slots)];
+    const size_t smem = sizeof(double) * ((size_t)(ls.sD + 1) * ls.sD + 4 * (size_t)ls.sD + 1);
+    if (L->gmPk.n != 2 * (size_t)kGmVals * sms) {
+        CR_CHECK(L->gmPk.alloc(2 * (size_t)kGmVals * sms));
+        CR_CUDA(cudaMemsetAsync(L->gmPk.p, 0, sizeof(ulonglong2) * L->gmPk.n, s));
+        L->gm_epoch = 0;
+    }
+    GmArgs<M, B> a;
+    a.sp = L->sell_ptr.p;
+    a.scol = L->sell_col.p;
+    a.npad = L->npad;
+    a.n = n;
+    a.Ks = Ks;
+    a.u = reinterpret_cast<B*>(L->basis.p);
+    a.n3 = 3LL * n;
+    a.sD = ls.sD;
+    a.mItr = ls.mItr;
+    a.relTol = ls.relTol;
+    a.absTol = ls.absTol;
+    a.R = R;
+    a.X = X;
+    a.nface = (int)L->gm_faces.size();
+    a.fptr = L->gmFptr.p;
+    a.fent = L->gmFent.p;
+    a.fface = L->gmFface.p;
+    a.fval = L->gmFval.p;
+    a.gram = L->gmGram.p;
+    for (int q = 0; q < kMaxCoupled; ++q) {
+        a.coef0[q] = a.coef1[q] = 0.0;
+        if (q < a.nface) {
+            const MemlsFace& f = L->face[L->gm_faces[q]];
+            a.coef0[q] = f.res;
+            a.coef1[q] = -f.res / (1.0 + f.res * f.nS);
+        }
+    }
+    a.pk = L->gmPk.p;
+    a.epoch = L->gm_epoch;
+    a.out = C.sc(slot);
+    // barriers of a call: per cycle at most 6, per iteration at most sD + 3
+    L->gm_epoch += 2 + (unsigned long long)std::max(ls.mItr, 0) * (6 + (unsigned long long)ls.sD * (ls.sD + 3));
+    CR_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * ((kGmMaxSD + 1) * kGmMaxSD + 4 * kGmMaxSD + 1))));
+    void* kargs[] = {&a};
+    note_launch();
+    CR_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(grid), dim3(threads), kargs, smem, s));
+    return CRIMSON_OK;
+}
+
+// memLS's statistics of a k_gmres call from the slots it left (on the host).
+static int gmres_finish(Ctx& C, crimson_subls& ls, int slot, double seconds) {
+    const double* o = C.L->hscal + slot;
+    ls.suc = 0;
+    if (o[1] < 0.0) {
+        set_last_error("GMRES: a wait of the persistent kernel ran out");
+        return CRIMSON_ERR_CUDA;
+    }
+    if (o[5] != 0.0) {   // right side below the absolute tolerance
+        ls.callD = 0.0;
+        ls.dB = 0.0;
+        return CRIMSON_OK;
+    }
+    ls.suc = (int)o[1];
+    ls.itr += (int)o[0];
+    ls.iNorm = o[2];
+    ls.fNorm = o[3];
+    ls.callD += seconds;
+    ls.dB = 10.0 * std::log(o[3] / o[4]);
+    return CRIMSON_OK;
+}
+
 // Runs one restart cycle on the device (k_gmres_cycle): U(0) normalized in
 // the basis, err0 = its norm before normalizing.  Returns the iterations
 // done, whether |err_i| < eps was reached, and the rotated Hessenberg
-// columns / err values in the host arrays of gmres().  *used = 0 when the
-// persistent cycle does not apply (sD too large, more than 8 coupled faces, or no
-// cooperative fit); the caller then runs the launch-per-step loop.
+// columns / err values in the host arrays of gmres().  The caller has prepared
+// the faces (gm_faces_prepare) and checked sD; *used = 0 when there is no
+// cooperative fit.
 template <typename M, typename B>
 static int gmres_cycle(Ctx& C, crimson_subls& ls, const M* Ks, double err0, double eps, std::vector<double>& h,
                        std::vector<double>& err, int* iters, int* suc, int* used) {
@@ -1424,18 +2006,15 @@ static int gmres_cycle(Ctx& C, crimson_subls& ls, const M* Ks, double err0, doub
     const int sD = ls.sD;
     *used = 0;
     if (sD < 1 || sD > kGmMaxSD) return CRIMSON_OK;
-    int ok = 0;
-    CR_CHECK(gm_face_map(L, &ok));
-    if (!ok) return CRIMSON_OK;
     const int nface = (int)L->gm_faces.size();
     const void* fns[3] = {(const void*)k_gmres_cycle<M, B, 0>, (const void*)k_gmres_cycle<M, B, 1>,
                           (const void*)k_gmres_cycle<M, B, kMaxCoupled>};
-    int& grid = std::is_same<M, float>::value ? L->gm_grid32 : L->gm_grid;
+    int& grid = L->gm_grid32;
     if (grid == 0) {
         int nb = 1 << 30;
         for (const void* f : fns) {
             int b = 0;
-            CR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kGmThreads, 0));
+            CR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kGmcThreads, 0));
             nb = std::min(nb, b);
         }
         grid = nb >= 1 ? sm_count() * std::min(nb, 2) : -1;
@@ -1444,8 +2023,8 @@ static int gmres_cycle(Ctx& C, crimson_subls& ls, const M* Ks, double err0, doub
     CR_CHECK(L->gmH.alloc((size_t)(kGmMaxSD + 1) * kGmMaxSD));
     CR_CHECK(L->gmErr.alloc(kGmMaxSD + 1));
     CR_CHECK(L->gmOut.alloc(2));
-    CR_CHECK(L->gmPart.alloc(2 * (size_t)kGmPartStride * std::max(L->gm_grid, L->gm_grid32)));
-    GmArgs<M, B> a;
+    CR_CHECK(L->gmPart.alloc(2 * (size_t)kGmPartStride * L->gm_grid32));
+    GmcArgs<M, B> a;
     a.sp = L->sell_ptr.p;
     a.scol = L->sell_col.p;
     a.npad = L->npad;
@@ -1460,21 +2039,14 @@ static int gmres_cycle(Ctx& C, crimson_subls& ls, const M* Ks, double err0, doub
     a.fface = L->gmFface.p;
     a.fval = L->gmFval.p;
     a.gram = L->gmGram.p;
-    FaceNorms nsv{};
-    int off = 0;
-    for (int q = 0; q < nface; ++q) {
-        const MemlsFace& f = L->face[L->gm_faces[q]];
-        launch(k_gm_fval, grid_for(f.nNo, 256), 256, 0, s, (const double*)f.valM.p, f.dof, std::min(f.dof, 3), f.nNo,
-               L->gmFval.p + 3 * (size_t)off);
-        a.coef0[q] = f.res;
-        a.coef1[q] = -f.res / (1.0 + f.res * f.nS);
-        nsv.v[q] = f.nS;
-        off += f.nNo;
+    for (int q = 0; q < kMaxCoupled; ++q) {
+        a.coef0[q] = a.coef1[q] = 0.0;
+        if (q < nface) {
+            const MemlsFace& f = L->face[L->gm_faces[q]];
+            a.coef0[q] = f.res;
+            a.coef1[q] = -f.res / (1.0 + f.res * f.nS);
+        }
     }
-    for (int q = nface; q < kMaxCoupled; ++q) a.coef0[q] = a.coef1[q] = 0.0;
-    if (nface > 0)
-        launch(k_gm_gram, 1, 32, 0, s, (const int*)L->gmPairs.p, L->gm_npairs, (const int*)L->gmFface.p,
-               (const double*)L->gmFval.p, nsv, nface, L->gmGram.p);
     a.err0 = err0;
     a.eps = eps;
     a.part = L->gmPart.p;
@@ -1484,7 +2056,7 @@ static int gmres_cycle(Ctx& C, crimson_subls& ls, const M* Ks, double err0, doub
     void* kargs[] = {&a};
     note_launch();
     const void* kfn = fns[nface == 0 ? 0 : (nface == 1 ? 1 : 2)];
-    CR_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(grid), dim3(kGmThreads), kargs, 0, s));
+    CR_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(grid), dim3(kGmcThreads), kargs, 0, s));
     double out[2];
     CR_CUDA(cudaMemcpyAsync(out, L->gmOut.p, sizeof(out), cudaMemcpyDeviceToHost, s));
     CR_CUDA(cudaStreamSynchronize(s));
@@ -1500,9 +2072,12 @@ static int gmres_cycle(Ctx& C, crimson_subls& ls, const M* Ks, double err0, doub
     return CRIMSON_OK;
 }
 
-// GMRES (memLS.f90:681-788) on dof = 3; K sliced in M, basis in B, R and X FP64; X may not alias R.
+// GMRES (memLS.f90:681-788) on dof = 3 with the restarts on the host: each
+// cycle as one kernel (cycles: the FP32-tangent mode), or with one launch per
+// step where no persistent kernel applies (more than kGmMaxSD Krylov vectors or
+// kMaxCoupled coupled faces); K sliced in M, basis in B, R and X FP64; X may not alias R.
 template <typename M, typename B>
-static int gmres(Ctx& C, crimson_subls& ls, const M* Ks, const double* R, double* X) {
+static int gmres(Ctx& C, crimson_subls& ls, const M* Ks, const double* R, double* X, bool cycles) {
     crimson_lhs* L = C.L;
     cudaStream_t s = C.s;
     const int dof = 3;
@@ -1544,11 +2119,10 @@ static int gmres(Ctx& C, crimson_subls& ls, const M* Ks, const double* R, double
         }
         ls.dB = ls.fNorm;
         launch(k_divide<B>, grid_for(n, 256), 256, 0, s, (const B*)U(0), (const double*)C.sc(kSlotNrm), U(0), n, 1);
-        // the cycle as one persistent kernel where it applies, else one launch per step
         int used = 0;
-        {
+        if (cycles && std::is_same<M, float>::value) {
             int it = 0, ok = 0;
-            CR_CHECK((gmres_cycle<M, B>(C, ls, Ks, err[0], eps, h, err, &it, &ok, &used)));
+            CR_CHECK((gmres_cycle<float, float>(C, ls, (const float*)Ks, err[0], eps, h, err, &it, &ok, &used)));
             if (used) {
                 ls.itr = ls.itr + it;
                 i = it;
@@ -1728,56 +2302,22 @@ int memls_cg_layout(crimson_lhs* L, int* resident64, int* resident32, long long*
 
 // CGRAD (memLS.f90:367-430) on the Schur-like operator L P - Gt G P; R in/out (n).
 // use_s2: on the explicit operator (schur.cu), else with two products on
-// Gs / GLs, the sliced G and {Gt, L} of this NSSOLVER call.
+// Gs / GLs, the sliced G and {Gt, L} of this NSSOLVER call.  Launches only;
+// the outcome goes to the slots kSlotCg (cgrad_finish).
 template <typename M>
-static int cgrad(Ctx& C, crimson_subls& ls, const M* Gs, const typename V4<M>::type* GLs, double* R, int nface,
-                 const double* coef, bool use_s2) {
+static int cgrad_launch(Ctx& C, const crimson_subls& ls, const M* Gs, const typename V4<M>::type* GLs, double* R,
+                        int nface, const double* coef, bool use_s2) {
     crimson_lhs* L = C.L;
     cudaStream_t s = C.s;
     const int n = L->nNo;
-    const double time = now_s();
-    ls.suc = 0;
     (std::is_same<M, float>::value ? L->cg_used32 : L->cg_used64) = true;
-    auto& acc = std::is_same<M, float>::value ? L->cg_acc32 : L->cg_acc64;
     if (use_s2) {
         CR_CUDA(cudaEventRecord(L->ev0, s));
         CR_CHECK(cg_schur_launch<M>(L, R, nface, coef, ls.relTol, ls.absTol, ls.mItr, C.sc(kSlotCg)));
         CR_CUDA(cudaEventRecord(L->ev1, s));
-        CR_CHECK(C.sync_scal(kSlotCg, 5));
-        const double err = L->hscal[kSlotCg + 0], errO = L->hscal[kSlotCg + 1];
-        const int i = (int)L->hscal[kSlotCg + 2];
-        if (L->hscal[kSlotCg + 3] < 0.0) {
-            set_last_error("CGRAD: a wait of the persistent kernel ran out");
-            return CRIMSON_ERR_CUDA;
-        }
-        ls.suc = (int)L->hscal[kSlotCg + 3];
-        ls.iNorm = L->hscal[kSlotCg + 4];
-        float ms = 0.f;
-        CR_CUDA(cudaEventElapsedTime(&ms, L->ev0, L->ev1));
-        acc.ms += ms;
-        acc.iters += i - 1;
-        acc.launches += 1;
-        if (L->s2_form_pending) {
-            float fm = 0.f;
-            CR_CUDA(cudaEventElapsedTime(&fm, L->s2_ev0, L->s2_ev1));
-            L->s2_form_ms += fm;
-            L->s2_forms += 1;
-            L->s2_form_pending = false;
-        }
-        ls.fNorm = std::sqrt(err);
-        ls.callD = now_s() - time + ls.callD;
-        ls.dB = 5.0 * std::log(err / errO);
-        ls.itr = ls.itr + i - 1;
         return CRIMSON_OK;
     }
     C.dot((const double*)R, (const double*)R, n, kSlotErr);
-    CR_CHECK(C.sync_scal(kSlotErr, 1));
-    double errO = std::sqrt(L->hscal[kSlotErr]);
-    ls.iNorm = errO;
-    double eps = std::max(ls.absTol, ls.relTol * errO);
-    eps = eps * eps;
-    double err = errO;
-    err = err * err;
     size_t rbytes = 0;
     CR_CHECK(cg_layout<M>(L, &rbytes));
     const int grid = std::is_same<M, float>::value ? L->cg_grid32 : L->cg_grid;
@@ -1813,8 +2353,9 @@ static int cgrad(Ctx& C, crimson_subls& ls, const M* Gs, const typename V4<M>::t
     a.w = L->cgW.p;
     a.z = L->cgZ.p;
     for (int f = 0; f < kMaxCoupled; ++f) a.coef[f] = f < nface ? coef[f] : 0.0;
-    a.eps = eps;
-    a.err0 = err;
+    a.rr = C.sc(kSlotErr);
+    a.relTol = ls.relTol;
+    a.absTol = ls.absTol;
     a.mItr = ls.mItr;
     a.part = L->cgPart.p;
     a.out = C.sc(kSlotCg);
@@ -1823,20 +2364,38 @@ static int cgrad(Ctx& C, crimson_subls& ls, const M* Gs, const typename V4<M>::t
     CR_CUDA(cudaEventRecord(L->ev0, s));
     CR_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(grid), dim3(kCgThreads), kargs, dyn, s));
     CR_CUDA(cudaEventRecord(L->ev1, s));
-    CR_CHECK(C.sync_scal(kSlotCg, 4));
-    err = L->hscal[kSlotCg + 0];
-    errO = L->hscal[kSlotCg + 1];
+    CR_CUDA(cudaMemcpyAsync(R, L->cgX.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+    return CRIMSON_OK;
+}
+
+// memLS's statistics of the CGRAD call from the slots it left (on the host),
+// after the stream has been waited for.
+template <typename M>
+static int cgrad_finish(Ctx& C, crimson_subls& ls) {
+    crimson_lhs* L = C.L;
+    const double err = L->hscal[kSlotCg + 0], errO = L->hscal[kSlotCg + 1];
     const int i = (int)L->hscal[kSlotCg + 2];
+    if (L->hscal[kSlotCg + 3] < 0.0) {
+        set_last_error("CGRAD: a wait of the persistent kernel ran out");
+        return CRIMSON_ERR_CUDA;
+    }
     ls.suc = (int)L->hscal[kSlotCg + 3];
+    ls.iNorm = L->hscal[kSlotCg + 4];
     float ms = 0.f;
     CR_CUDA(cudaEventElapsedTime(&ms, L->ev0, L->ev1));
+    auto& acc = std::is_same<M, float>::value ? L->cg_acc32 : L->cg_acc64;
     acc.ms += ms;
     acc.iters += i - 1;
     acc.launches += 1;
-    CR_CUDA(cudaMemcpyAsync(R, L->cgX.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-    CR_CUDA(cudaStreamSynchronize(s));
+    if (L->s2_form_pending) {
+        float fm = 0.f;
+        CR_CUDA(cudaEventElapsedTime(&fm, L->s2_ev0, L->s2_ev1));
+        L->s2_form_ms += fm;
+        L->s2_forms += 1;
+        L->s2_form_pending = false;
+    }
     ls.fNorm = std::sqrt(err);
-    ls.callD = now_s() - time + ls.callD;
+    ls.callD = 1e-3 * ms + ls.callD;
     ls.dB = 5.0 * std::log(err / errO);
     ls.itr = ls.itr + i - 1;
     return CRIMSON_OK;
@@ -1880,6 +2439,97 @@ static int ge_solve(int N, const double* A, double* B) {
     }
     for (int i = 0; i < N; ++i) B[i] = c(i, N);
     return CRIMSON_OK;
+}
+
+// ---------------------------------------------------------------------------
+// NSSOLVER's least-squares system (memLS.f90:1540-1570): the products of the
+// two newest columns A d (u part n3 values, p part n) with every column and
+// with the right side.  Column c is MU + c n3 / MP + c n; pair (k, j) for
+// k = c0, c0 + 1 and j <= k, and (k, right side).  One pass reads the two new
+// columns, the right side and kGramCols older columns; per-block sums, then
+// one warp per product sums the blocks in order.  (One reduction launch per
+// product and part took 28 launches per outer iteration and re-read the new
+// columns each time: 10 of 143 ms of a 452k-tet mixed time step.)
+// ---------------------------------------------------------------------------
+constexpr int kGramCols = 4;
+constexpr int kGramSums = 5 + 2 * kGramCols;   // n.n, n.m, m.m, n.r, m.r, then n.o, m.o of every older column
+constexpr int kGramThreads = 256;
+
+__global__ void __launch_bounds__(kGramThreads) k_gram_part(const double* __restrict__ MU, const double* __restrict__ MP,
+                                                            const double* __restrict__ Ru, const double* __restrict__ Rp,
+                                                            long long n3, long long n, int c0, int o0, int no,
+                                                            double* __restrict__ part) {
+    __shared__ double red[kGramSums][kGramThreads / 32];
+    double acc[kGramSums];
+#pragma unroll
+    for (int k = 0; k < kGramSums; ++k) acc[k] = 0.0;
+    const long long tot = n3 + n;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (long long)gridDim.x * blockDim.x) {
+        const bool u = t < n3;
+        const double* base = u ? MU + t : MP + (t - n3);
+        const size_t ld = (size_t)(u ? n3 : n);
+        const double a = base[(size_t)c0 * ld], b = base[(size_t)(c0 + 1) * ld];
+        double o[kGramCols];
+#pragma unroll
+        for (int k = 0; k < kGramCols; ++k) o[k] = k < no ? base[(size_t)(o0 + k) * ld] : 0.0;
+        if (o0 == 0) {
+            const double r = u ? Ru[t] : Rp[t - n3];
+            acc[0] += a * a;
+            acc[1] += a * b;
+            acc[2] += b * b;
+            acc[3] += a * r;
+            acc[4] += b * r;
+        }
+#pragma unroll
+        for (int k = 0; k < kGramCols; ++k) {
+            acc[5 + 2 * k] += a * o[k];
+            acc[6 + 2 * k] += b * o[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kGramSums; ++k) {
+        const double v = warp_sum(acc[k]);
+        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < kGramSums) {
+        double v = 0.0;
+        for (int w = 0; w < kGramThreads / 32; ++w) v += red[threadIdx.x][w];
+        part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = v;
+    }
+}
+
+// out[k] = sum of the nblk block sums of product k, in order; one block per product
+__global__ void __launch_bounds__(32) k_gram_sum(const double* __restrict__ part, int nblk, double* __restrict__ out) {
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nblk; b += 32) s += part[(size_t)blockIdx.x * nblk + b];
+    s = warp_sum(s);
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
+// y = y0 + sum_j c_j x_j, columns x_j at stride ld * step, terms added in
+// order (y0 may be null: 0); u and p parts in one launch
+constexpr int kMaxCols = 44;
+struct ColCoefs {
+    double c[kMaxCols];
+};
+__global__ void __launch_bounds__(256) k_combine(const __grid_constant__ ColCoefs cf, int m, int step,
+                                                 const double* __restrict__ Xu, const double* __restrict__ Xp,
+                                                 const double* __restrict__ y0u, const double* __restrict__ y0p,
+                                                 double* __restrict__ yu, double* __restrict__ yp, long long n3,
+                                                 long long n) {
+    const long long tot = (yu ? n3 : 0) + n;
+    const long long nu = yu ? n3 : 0;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (long long)gridDim.x * blockDim.x) {
+        const bool u = t < nu;
+        const long long i = u ? t : t - nu;
+        const double* x = u ? Xu + i : Xp + i;
+        const size_t ld = (size_t)(u ? n3 : n) * step;
+        const double* y0 = u ? y0u : y0p;
+        double y = y0 ? y0[i] : 0.0;
+        for (int j = 0; j < m; ++j) y = y + cf.c[j] * x[(size_t)j * ld];
+        (u ? yu : yp)[i] = y;
+    }
 }
 
 // Sliced matrix buffers of one precision (zeroed at allocation, so the
@@ -1998,15 +2648,23 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
     eps = std::max(ls->RI.absTol, ls->RI.relTol * eps);
     // BCPRE (memLS.f90:1683-1716): nS = |valM|^2 per coupled face, summed on
     // the host in the reference's node order (faces are small).
-    for (auto& f : L->face) {
-        if (!f.coupledFlag) continue;
-        std::vector<double> vm((size_t)f.dof * f.nNo);
-        CR_CUDA(cudaMemcpyAsync(vm.data(), f.valM.p, sizeof(double) * vm.size(), cudaMemcpyDeviceToHost, s));
+    {
+        std::vector<std::vector<double>> vm(L->face.size());
+        for (size_t k = 0; k < L->face.size(); ++k) {
+            const MemlsFace& f = L->face[k];
+            if (!f.coupledFlag) continue;
+            vm[k].resize((size_t)f.dof * f.nNo);
+            CR_CUDA(cudaMemcpyAsync(vm[k].data(), f.valM.p, sizeof(double) * vm[k].size(), cudaMemcpyDeviceToHost, s));
+        }
         CR_CUDA(cudaStreamSynchronize(s));
-        f.nS = 0.0;
-        const int nsd = std::min(f.dof, 3);
-        for (int a = 0; a < f.nNo; ++a)
-            for (int i = 0; i < nsd; ++i) f.nS = f.nS + std::pow(vm[(size_t)f.dof * a + i], 2.0);
+        for (size_t k = 0; k < L->face.size(); ++k) {
+            MemlsFace& f = L->face[k];
+            if (!f.coupledFlag) continue;
+            f.nS = 0.0;
+            const int nsd = std::min(f.dof, 3);
+            for (int a = 0; a < f.nNo; ++a)
+                for (int i = 0; i < nsd; ++i) f.nS = f.nS + std::pow(vm[k][(size_t)f.dof * a + i], 2.0);
+        }
     }
     int cg_nface = 0;
     double cg_coef[kMaxCoupled];
@@ -2028,21 +2686,43 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
     CR_CHECK(sell_mats(L, &Ks, &Gs, &GLs, !use_s2));
     launch(k_to_sell<M>, grid_for(nNo, 256), 256, 0, s, L->rowptr, (const int*)L->sell_ptr.p, nNo, mK, mG, Gt, mL,
            L->npad, Ks, use_s2 ? nullptr : Gs, GLs);
+    // the FP32-tangent mode keeps the summation orders of its results (k_gmres_cycle)
+    const bool kept = ls->precision == CRIMSON_MIXED_F32_TANGENT;
+    int gm_ok = 0;
+    if (ls->GM.sD >= 1 && ls->GM.sD <= kGmMaxSD) CR_CHECK(gm_faces_prepare(L, &gm_ok));
+    // One GMRES solve K X = R: k_gmres, whose statistics wait in slot g, or
+    // the launch-per-step form
+    auto gmres_any = [&](const double* R_, double* X_, int g) -> int {
+        if (!gm_ok || kept) return gmres<M, B>(C, ls->GM, (const M*)Ks, R_, X_, gm_ok != 0);
+        CR_CUDA(cudaEventRecord(L->ev_gm[2 * g], s));
+        CR_CHECK((gmres_launch<M, B>(C, ls->GM, (const M*)Ks, R_, X_, kSlotGm + 8 * g)));
+        CR_CUDA(cudaEventRecord(L->ev_gm[2 * g + 1], s));
+        return CRIMSON_OK;
+    };
+    auto gmres_stats = [&](int g) -> int {
+        if (!gm_ok || kept) return CRIMSON_OK;
+        float ms = 0.f;
+        CR_CUDA(cudaEventElapsedTime(&ms, L->ev_gm[2 * g], L->ev_gm[2 * g + 1]));
+        return gmres_finish(C, ls->GM, kSlotGm + 8 * g, 1e-3 * ms);
+    };
+    const int gram_grid = grid_for(4LL * nNo, kGramThreads, 4);
+    CR_CHECK(L->gramPart.alloc((size_t)kGramSums * gram_grid));
+    auto combine = [&](const ColCoefs& cf, int m, int step, const double* Xu, const double* Xp, const double* y0u,
+                       const double* y0p, double* yu, double* yp) {
+        launch(k_combine, grid_for((yu ? 4LL : 1LL) * nNo, 256), 256, 0, s, cf, m, step, Xu, Xp, y0u, y0p, yu, yp, nv,
+               (long long)nNo);
+    };
     int i, iBB = 0;
     for (i = 1; i <= ls->RI.mItr; ++i) {
         iB = 2 * i - 1;
         iBB = 2 * i;
         ls->RI.dB = ls->RI.fNorm;
-        CR_CHECK((gmres<M, B>(C, ls->GM, (const M*)Ks, L->Rm.p, Ucol(i - 1))));
-        C.vs3(mD, (const double*)Ucol(i - 1), Pcol(i - 1));
-        launch(k_sub<double, double, double>, grid_for(nNo, 256), 256, 0, s, (const double*)L->Rc.p,
-               (const double*)Pcol(i - 1), Pcol(i - 1), (long long)nNo);
-        CR_CHECK(cgrad<M>(C, ls->CG, (const M*)Gs, (const typename V4<M>::type*)GLs, Pcol(i - 1), cg_nface, cg_coef,
-                          use_s2));
-        C.sv3(mG, (const double*)Pcol(i - 1), MUc(iB - 1));
-        launch(k_sub<double, double, double>, grid_for(nv, 256), 256, 0, s, (const double*)L->Rm.p,
-               (const double*)MUc(iB - 1), MUc(iBB - 1), nv);
-        CR_CHECK((gmres<M, B>(C, ls->GM, (const M*)Ks, MUc(iBB - 1), Ucol(i - 1))));
+        CR_CHECK(gmres_any(L->Rm.p, Ucol(i - 1), 0));
+        C.vs3(mD, (const double*)Ucol(i - 1), Pcol(i - 1), (const double*)L->Rc.p);   // Rc - D u
+        CR_CHECK(cgrad_launch<M>(C, ls->CG, (const M*)Gs, (const typename V4<M>::type*)GLs, Pcol(i - 1), cg_nface,
+                                 cg_coef, use_s2));
+        C.sv3(mG, (const double*)Pcol(i - 1), MUc(iB - 1), (const double*)L->Rm.p, MUc(iBB - 1));   // G p, Rm - G p
+        CR_CHECK(gmres_any(MUc(iBB - 1), Ucol(i - 1), 1));
         if (std::is_same<M, double>::value)
             C.vv3s((const M*)Ks, (const double*)Ucol(i - 1), MUc(iBB - 1));  // the sliced copy is FP64
         else
@@ -2051,29 +2731,48 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
         C.ss(mL, (const double*)Pcol(i - 1), MPc(iB - 1));
         C.vs3(mD, (const double*)Ucol(i - 1), MPc(iBB - 1));
         // Gram matrix entries for columns iB, iBB
-        int slot = kSlotGram;
-        for (int k = iB; k <= iBB; ++k) {
-            for (int j = 1; j <= k - 1; ++j) {
-                C.dot((const double*)MUc(j - 1), (const double*)MUc(k - 1), nv, slot++);
-                C.dot((const double*)MPc(j - 1), (const double*)MPc(k - 1), nNo, slot++);
+        int nsum = 0;
+        if (kept)
+            for (int k = iB; k <= iBB; ++k) {
+                auto both = [&](const double* u, const double* p) {
+                    C.dot((const double*)u, (const double*)MUc(k - 1), nv, kSlotGram + nsum++);
+                    C.dot((const double*)p, (const double*)MPc(k - 1), nNo, kSlotGram + nsum++);
+                };
+                for (int j = 1; j <= k; ++j) both(MUc(j - 1), MPc(j - 1));
+                both(L->Rmi.p, L->Rci.p);
             }
-            C.dot((const double*)MUc(k - 1), (const double*)MUc(k - 1), nv, slot++);
-            C.dot((const double*)MPc(k - 1), (const double*)MPc(k - 1), nNo, slot++);
-            C.dot((const double*)MUc(k - 1), (const double*)L->Rmi.p, nv, slot++);
-            C.dot((const double*)MPc(k - 1), (const double*)L->Rci.p, nNo, slot++);
+        for (int o0 = 0; !kept && (o0 == 0 || o0 < iB - 1); o0 += kGramCols) {
+            launch(k_gram_part, gram_grid, kGramThreads, 0, s, (const double*)L->MU.p, (const double*)L->MP.p,
+                   (const double*)L->Rmi.p, (const double*)L->Rci.p, nv, (long long)nNo, iB - 1, o0,
+                   std::min(kGramCols, iB - 1 - o0), L->gramPart.p);
+            launch(k_gram_sum, kGramSums, 32, 0, s, (const double*)L->gramPart.p, gram_grid, C.sc(kSlotGram + nsum));
+            nsum += kGramSums;
         }
-        CR_CHECK(C.sync_scal(kSlotGram, slot - kSlotGram));
-        slot = kSlotGram;
-        for (int k = iB; k <= iBB; ++k) {
-            for (int j = 1; j <= k - 1; ++j) {
-                Aa(j - 1, k - 1) = L->hscal[slot] + L->hscal[slot + 1];
-                slot += 2;
-                Aa(k - 1, j - 1) = Aa(j - 1, k - 1);
+        CR_CUDA(cudaMemcpyAsync(L->hscal + kSlotCg, L->scal.p + kSlotCg, sizeof(double) * (64 - kSlotCg),
+                                cudaMemcpyDeviceToHost, s));
+        CR_CHECK(C.sync_scal(kSlotGram, nsum));
+        CR_CHECK(gmres_stats(0));
+        CR_CHECK(cgrad_finish<M>(C, ls->CG));
+        CR_CHECK(gmres_stats(1));
+        const double* g = L->hscal + kSlotGram;
+        if (kept) {
+            for (int k = iB; k <= iBB; ++k) {
+                for (int j = 1; j < k; ++j, g += 2) Aa(j - 1, k - 1) = Aa(k - 1, j - 1) = g[0] + g[1];
+                Aa(k - 1, k - 1) = std::pow(std::sqrt(g[0]), 2.0) + std::pow(std::sqrt(g[1]), 2.0);
+                Bv[k - 1] = g[2] + g[3];
+                g += 4;
             }
-            Aa(k - 1, k - 1) = std::pow(std::sqrt(L->hscal[slot]), 2.0) + std::pow(std::sqrt(L->hscal[slot + 1]), 2.0);
-            slot += 2;
-            Bv[k - 1] = L->hscal[slot] + L->hscal[slot + 1];
-            slot += 2;
+        } else {
+            Aa(iB - 1, iB - 1) = g[0];
+            Aa(iB - 1, iBB - 1) = Aa(iBB - 1, iB - 1) = g[1];
+            Aa(iBB - 1, iBB - 1) = g[2];
+            Bv[iB - 1] = g[3];
+            Bv[iBB - 1] = g[4];
+            for (int j = 0; j < iB - 1; ++j) {
+                const double* o = g + (size_t)(j / kGramCols) * kGramSums + 5 + 2 * (j % kGramCols);
+                Aa(j, iB - 1) = Aa(iB - 1, j) = o[0];
+                Aa(j, iBB - 1) = Aa(iBB - 1, j) = o[1];
+            }
         }
         for (int t = 0; t < iBB; ++t) xB[t] = Bv[t];
         std::vector<double> Asub((size_t)iBB * iBB);
@@ -2093,39 +2792,32 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
             break;
         }
         // Rm = Rmi - sum xB_j MU_j ; Rc = Rci - sum xB_j MP_j
-        CR_CUDA(cudaMemcpyAsync(L->Rm.p, L->Rmi.p, sizeof(double) * nv, cudaMemcpyDeviceToDevice, s));
-        CR_CUDA(cudaMemcpyAsync(L->Rc.p, L->Rci.p, sizeof(double) * nNo, cudaMemcpyDeviceToDevice, s));
-        for (int j = 1; j <= iBB; ++j) {
-            launch(k_axpy<double, double>, grid_for(nv, 256), 256, 0, s, -xB[j - 1], (const double*)MUc(j - 1),
-                   L->Rm.p, nv);
-            launch(k_axpy<double, double>, grid_for(nNo, 256), 256, 0, s, -xB[j - 1], (const double*)MPc(j - 1),
-                   L->Rc.p, (long long)nNo);
-        }
+        ColCoefs cf;
+        for (int j = 0; j < iBB; ++j) cf.c[j] = -xB[j];
+        combine(cf, iBB, 1, L->MU.p, L->MP.p, L->Rmi.p, L->Rci.p, L->Rm.p, L->Rc.p);
     }
     if (i > ls->RI.mItr) {
         ls->RI.itr = ls->RI.mItr;
     } else {
         ls->RI.itr = i;
-        CR_CUDA(cudaMemcpyAsync(L->Rc.p, L->Rci.p, sizeof(double) * nNo, cudaMemcpyDeviceToDevice, s));
-        for (int j = 1; j <= iBB; ++j)
-            launch(k_axpy<double, double>, grid_for(nNo, 256), 256, 0, s, -xB[j - 1], (const double*)MPc(j - 1),
-                   L->Rc.p, (long long)nNo);
+        ColCoefs cf;
+        for (int j = 0; j < iBB; ++j) cf.c[j] = -xB[j];
+        combine(cf, iBB, 1, nullptr, L->MP.p, nullptr, L->Rci.p, nullptr, L->Rc.p);
     }
     C.dot((const double*)L->Rc.p, (const double*)L->Rc.p, nNo, 0);
     CR_CHECK(C.sync_scal(0, 1));
     ls->Resc = (int)std::lround(100.0 * std::pow(std::sqrt(L->hscal[0]) / ls->RI.fNorm, 2.0));
     ls->Resm = 100 - ls->Resc;
     // solution: Rmi = xB(2) U_1 + sum xB(2i) U_i ; Rci = xB(1) P_1 + sum xB(2i-1) P_i
-    CR_CUDA(cudaMemsetAsync(L->Rmi.p, 0, sizeof(double) * nv, s));
-    CR_CUDA(cudaMemsetAsync(L->Rci.p, 0, sizeof(double) * nNo, s));
-    launch(k_axpy<double, double>, grid_for(nv, 256), 256, 0, s, xB[1], (const double*)Ucol(0), L->Rmi.p, nv);
-    launch(k_axpy<double, double>, grid_for(nNo, 256), 256, 0, s, xB[0], (const double*)Pcol(0), L->Rci.p,
-           (long long)nNo);
-    for (i = 2; i <= ls->RI.itr; ++i) {
-        launch(k_axpy<double, double>, grid_for(nv, 256), 256, 0, s, xB[2 * i - 1], (const double*)Ucol(i - 1),
-               L->Rmi.p, nv);
-        launch(k_axpy<double, double>, grid_for(nNo, 256), 256, 0, s, xB[2 * i - 2], (const double*)Pcol(i - 1),
-               L->Rci.p, (long long)nNo);
+    {
+        ColCoefs cu, cp;
+        for (i = 1; i <= ls->RI.itr; ++i) {
+            cu.c[i - 1] = xB[2 * i - 1];
+            cp.c[i - 1] = xB[2 * i - 2];
+        }
+        combine(cp, ls->RI.itr, 1, nullptr, L->P.p, nullptr, nullptr, nullptr, L->Rci.p);
+        launch(k_combine, grid_for(nv, 256), 256, 0, s, cu, ls->RI.itr, 1, (const double*)nullptr, (const double*)L->U.p,
+               (const double*)nullptr, (const double*)nullptr, (double*)nullptr, L->Rmi.p, 0LL, nv);
     }
     launch(k_merge4, grid_for(nNo, 256), 256, 0, s, R, (const double*)L->Rmi.p, (const double*)L->Rci.p, nNo);
     CR_CUDA(cudaStreamSynchronize(s));
@@ -2140,7 +2832,7 @@ static int lhs_work_alloc(crimson_lhs* L, const crimson_ls* ls) {
     const long long nnz = L->nnz;
     const int iB = ls->RI.mItr;
     const int sD = ls->GM.sD;
-    if (sD + 1 > 512 || 8 * iB * iB + 64 > 4096) return CRIMSON_ERR_UNSUPPORTED;
+    if (sD + 1 > 512 || 8 * iB * iB + 64 > 4096 || iB > kMaxCols / 2) return CRIMSON_ERR_UNSUPPORTED;
     CR_CHECK(L->W.alloc(4 * (size_t)nNo));
     CR_CHECK(L->R.alloc(4 * (size_t)nNo));
     CR_CHECK(L->mK.alloc(9 * (size_t)nnz));
@@ -2164,6 +2856,7 @@ static int lhs_work_alloc(crimson_lhs* L, const crimson_ls* ls) {
         CR_CUDA(cudaMallocHost(&L->hscal, sizeof(double) * kScalTotal));
         CR_CUDA(cudaEventCreate(&L->ev0));
         CR_CUDA(cudaEventCreate(&L->ev1));
+        for (cudaEvent_t& e : L->ev_gm) CR_CUDA(cudaEventCreate(&e));
         CR_CUDA(cudaEventCreate(&L->s2_ev0));
         CR_CUDA(cudaEventCreate(&L->s2_ev1));
     }

@@ -76,14 +76,17 @@ struct crimson_lhs {
     int cg_res64 = 0, cg_res32 = 0;    // CG kernel with block-resident columns (per matrix type)
     long long cg_res_bytes = -1;       // its shared memory per block (0: offsets exceed 16 bits); -1 unknown
     DBuf<int> cg_tmp;
-    // persistent GMRES cycle: Hessenberg / err outputs, partial sums and the
-    // coupled-face node map (built for the coupled faces in gm_faces)
-    DBuf<double> gmH, gmErr, gmOut, gmPart, gmFval, gmGram;
+    // persistent GMRES: the barriers' packets and the coupled-face node map
+    // (built for the coupled faces in gm_faces)
+    DBuf<ulonglong2> gmPk;
+    unsigned long long gm_epoch = 0;
+    DBuf<double> gmFval, gmGram;
+    DBuf<double> gmH, gmErr, gmOut, gmPart;   // k_gmres_cycle: Hessenberg, err, outcome, partial sums
+    int gm_grid32 = 0;
     DBuf<int> gmFptr, gmFent, gmFface, gmPairs;
     std::vector<int> gm_faces;
     int gm_npairs = 0;
     int gm_map_ok = -1;   // 1: map built, 0: not usable (more than 8 coupled faces), -1: not built
-    int gm_grid = 0, gm_grid32 = 0;
     // mixed precision: FP64 right side and accumulated solution of the
     // iterative refinement
     DBuf<double> R0, X4;
@@ -95,6 +98,8 @@ struct crimson_lhs {
         long long iters = 0, launches = 0;
     } cg_acc64, cg_acc32;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_gm[4] = {nullptr, nullptr, nullptr, nullptr};   // around the two GMRES calls of an outer iteration
+    DBuf<double> gramPart;            // block sums of NSSOLVER's products
     // explicit Schur operator S = L - Gt G of CGRAD (schur.cu): slices of the
     // 2-ring pattern, chunk descriptors, the blocks' ranges, and the operator
     // (values and int16 column offsets by chunk) per storage precision

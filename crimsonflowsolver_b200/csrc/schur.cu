@@ -521,36 +521,6 @@ struct S2Lane<float> {
     }
 };
 
-// The reductions of one barrier.  red[32 k + w]: warp w's partial of value k;
-// tot[k] (shared) receives the sums.  Value 0 comes from every block (and is
-// the barrier); values 1 + 2 f, 2 + 2 f of face f only from the blocks whose
-// slices touch the face (fpend: per lane, as gr_all_blocks), the others'
-// being zero.  data: the block's global writes before the call are visible to
-// all blocks after it.
-__device__ __noinline__ bool s2_reduce(const CgS2Args& a, const double* red, int nface, unsigned own_faces,
-                                       const unsigned char* fpend, unsigned long long ep, bool data, double* tot,
-                                       bool failed) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, nv = 1 + 2 * nface;
-    ulonglong2* pk = a.pk + (size_t)(ep & 1) * kS2Vals * gridDim.x;
-    bool fail = failed;
-    __syncthreads();
-    for (int k = wid; k < nv; k += nw)
-        if (k == 0 || ((own_faces >> ((k - 1) / 2)) & 1)) {
-            const double v = warp_sum(lane < nw ? red[32 * k + lane] : 0.0);
-            if (lane == 0) {
-                if (data) gr_release();
-                gr_publish(pk + (size_t)k * gridDim.x + blockIdx.x, v, ep);
-            }
-        }
-    for (int k = wid; k < nv; k += nw) {
-        const unsigned pend = k == 0 ? gr_all_blocks() : fpend[32 * ((k - 1) / 2) + lane];
-        const double v = gr_collect(pk + (size_t)k * gridDim.x, pend, ep, &fail);
-        if (data) gr_acquire();
-        if (lane == 0) tot[k] = v;
-    }
-    return __syncthreads_or(fail) != 0;
-}
-
 // kRes: the block's chunks stay in shared memory (loaded once), else they
 // stream through the warps' rings.
 template <typename M, bool kRes>
@@ -664,7 +634,7 @@ __global__ void __launch_bounds__(32 * kS2CgWarps, 1) k_cg_schur(const __grid_co
         }
     part = warp_sum(part);
     if (lane == 0) red[wid] = part;
-    bool fail = s2_reduce(a, red, 0, 0u, fpend, ++ep, true, tot, false);
+    bool fail = grid_reduce(a.pk, kS2Vals, red, 0, 0u, fpend, ++ep, true, tot, false);
     if (threadIdx.x == 0) {
         const double e = sqrt(tot[0]), eps = fmax(a.absTol, a.relTol * e);
         scal[0] = e * e;
@@ -796,7 +766,7 @@ __global__ void __launch_bounds__(32 * kS2CgWarps, 1) k_cg_schur(const __grid_co
         }
         dps = warp_sum(dps);
         if (lane == 0) red[wid] = dps;
-        fail = s2_reduce(a, red, a.nface, own_faces, fpend, ++ep, false, tot, !ok || fail);
+        fail = grid_reduce(a.pk, kS2Vals, red, a.nface, own_faces, fpend, ++ep, false, tot, !ok || fail);
         double den = tot[0];
         for (int f = 0; f < a.nface; ++f) den = den - a.coef[f] * tot[1 + 2 * f] * tot[2 + 2 * f];
         const double alpha = scal[0] / den;
@@ -818,7 +788,7 @@ __global__ void __launch_bounds__(32 * kS2CgWarps, 1) k_cg_schur(const __grid_co
         }
         rs = warp_sum(rs);
         if (lane == 0) red[wid] = rs;
-        fail = s2_reduce(a, red, 0, 0u, fpend, ++ep, true, tot, fail);
+        fail = grid_reduce(a.pk, kS2Vals, red, 0, 0u, fpend, ++ep, true, tot, fail);
         if (threadIdx.x == 0) {
             const double e2 = sqrt(tot[0]), err = e2 * e2;
             scal[4] = err / scal[0];
