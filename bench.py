@@ -498,7 +498,7 @@ def run_ours(args):
                    "parallelism": "replicas" if ws > 1 else "single GPU",
                    "epstol_ns": P.epstol_ns, "epstol_gmres_cg": [P.epstol_mom, P.epstol_cont],
                    "mixed_refine_tol": Pm.refine_tol if Pm.refine_tol > 0 else P.epstol_ns,
-                   "l2": "inputs larger than L2 (sliced FP32 matrices 0.66 GB, FP64 K and Schur operator 1.2 GB per solve)"},
+                   "l2": "inputs larger than L2 (K and Schur operator 0.63 GB FP32, 1.2 GB FP64 per solve)"},
         "fp64": {"value": v64, "unit": "s/timestep", "ms_per_step": t64_ms / args.steps,
                  "e2e": {"value": e2e64, "unit": "s/timestep", "h2d_bytes_per_step": 2 * 4 * n * 8,
                          "d2h_bytes_per_step": 2 * 4 * n * 8},

@@ -17,8 +17,8 @@
 // blocks per lane issued together; dot products and norms use a single-pass
 // grid reduction whose last block sums the per-block partials in a fixed
 // order (deterministic).  CGRAD runs as one persistent cooperative kernel per
-// call: in FP64 on the explicitly formed Schur operator (schur.cu) where the
-// pattern allows, else on the two-product kernel below.  The Krylov control flow (Givens rotations, back substitution, the
+// call: on the explicitly formed Schur operator (schur.cu) where the pattern
+// allows, else on the two-product kernel below.  The Krylov control flow (Givens rotations, back substitution, the
 // 2i x 2i Gram system solved by GE) runs on the host in FP64 on scalars
 // copied back per step, as the reference's serial code does.
 //
@@ -486,8 +486,8 @@ __global__ void k_to_sell(const int* __restrict__ rowptr, const int* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// CGRAD as one persistent cooperative kernel (memLS.f90:367-430): the mixed
-// solve, and FP64 on patterns that the explicit operator (schur.cu) excludes.
+// CGRAD as one persistent cooperative kernel (memLS.f90:367-430): on patterns
+// that the explicit operator (schur.cu) excludes, and in the FP32-tangent mode.
 //
 // Per iteration three grid-wide barriers: (A) P = R + beta P formed on the
 // fly while computing GP = G P, plus the coupled-face dots w_f . P; (B)
@@ -2672,10 +2672,11 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
     M* Ks = nullptr;
     M* Gs = nullptr;
     typename V4<M>::type* GLs = nullptr;
-    // CGRAD's operator: in FP64 formed explicitly where the pattern allows
-    // (schur.cu); in the mixed solve only on request, since rounding S
-    // instead of G, Gt and L moves its result by up to 1e-9.
-    const bool want_s2 = std::is_same<M, double>::value || ls->schur;
+    // the FP32-tangent mode keeps the summation orders of its results (k_gmres_cycle)
+    const bool kept = ls->precision == CRIMSON_MIXED_F32_TANGENT;
+    // CGRAD's operator: formed explicitly where the pattern allows (schur.cu);
+    // in the FP32-tangent mode only on request
+    const bool want_s2 = !kept || ls->schur;
     if (want_s2) CR_CHECK(schur_pattern(L));
     const bool use_s2 = want_s2 && L->s2_state == 1;
     if (ls->schur) L->s2_asked = true;
@@ -2686,8 +2687,6 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
     CR_CHECK(sell_mats(L, &Ks, &Gs, &GLs, !use_s2));
     launch(k_to_sell<M>, grid_for(nNo, 256), 256, 0, s, L->rowptr, (const int*)L->sell_ptr.p, nNo, mK, mG, Gt, mL,
            L->npad, Ks, use_s2 ? nullptr : Gs, GLs);
-    // the FP32-tangent mode keeps the summation orders of its results (k_gmres_cycle)
-    const bool kept = ls->precision == CRIMSON_MIXED_F32_TANGENT;
     int gm_ok = 0;
     if (ls->GM.sD >= 1 && ls->GM.sD <= kGmMaxSD) CR_CHECK(gm_faces_prepare(L, &gm_ok));
     // One GMRES solve K X = R: k_gmres, whose statistics wait in slot g, or

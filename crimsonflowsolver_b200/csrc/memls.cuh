@@ -111,7 +111,7 @@ struct crimson_lhs {
     DBuf<int2> s2_blk;
     DBuf<unsigned> s2_mask;
     DBuf<unsigned char> s2_op64, s2_op32;
-    DBuf<double> s2_R;
+    DBuf<double> s2_R, s2_rowfix;
     DBuf<ulonglong2> s2_pk;
     unsigned long long s2_epoch = 0;
     long long s2_nnz = 0, s2_npad = 0;
@@ -132,7 +132,7 @@ struct crimson_ls {
     int precision = CRIMSON_FP64;  // CRIMSON_FP64, CRIMSON_MIXED or CRIMSON_MIXED_F32_TANGENT
     int max_refine = 4;            // FP64 refinement sweeps of the mixed solve
     double refine_tol = 0.0;       // target |R - A x| / |R|; <= 0: RI.relTol
-    int schur = 0;                 // 1: the mixed solve's CG runs on the explicit Schur operator too, where the pattern allows
+    int schur = 0;                 // 1: report the explicit Schur operator; FP32-tangent mode: run the CG on it
     std::string log_path;          // per-solve log (memLS_NS.log format); empty: off
 };
 

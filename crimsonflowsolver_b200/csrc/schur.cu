@@ -5,8 +5,12 @@
 // SP = L P - Gt (G P) - (coupled-face terms) as two sparse products.  Here
 // S = L - Gt G is formed once per NSSOLVER call, in FP64 and in a fixed
 // order, on the 2-ring pattern of the node graph, stored in FP64 or, for the
-// mixed-precision solve, rounded once to FP32; an iteration is then one
-// sparse product.  Against the two products the stream per row is smaller
+// mixed-precision solve, rounded once to FP32 with an FP64 correction of the
+// own row's term that restores the row sum; an iteration is then one sparse
+// product.  (The smooth modes are the ones the operator nearly annihilates
+// and the rounding disturbs most: without the correction a mixed solve is up
+// to 5e-10 from the FP64 one, with it 4e-11 in the median of 70 drawn
+// systems; two products with rounded G, Gt, L and gathered {GP, P} 1.7e-10.)  Against the two products the stream per row is smaller
 // (about 62 entries of 8 + 2 B against 14.7 blocks of 7 values: 620 / 823 B
 // in FP64, 372 / 412 B in FP32), and an iteration has two grid-wide barriers
 // instead of three.  (The two-product kernel stays for patterns that do not
@@ -34,7 +38,7 @@
 //     stop at slice ends, barriers or iteration ends; bound by HBM (the
 //     product phase reads 6.7 TB/s in FP64, 5.8 in FP32).
 // Per iteration, before (two-product kernel) and now, B200: 4M-tet cylinder
-// 118 / 80 us FP64, 74 / 56 FP32; 452k-tet bifurcation 24.6 / 16 FP32;
+// 118 / 80 us FP64, 74 / 57 FP32; 452k-tet bifurcation 24.6 / 16 FP32;
 // 108k-tet cylinder 20 / 9.2 FP64; 1152 tets 15 / 5.5 FP64.
 //
 // Iteration.  S P is kept by the recurrence S P = S R + beta S P_prev, so the
@@ -338,7 +342,8 @@ __global__ void __launch_bounds__(32 * kS2FormWarps) k_s2_form(const int* __rest
                                                               const double* __restrict__ Gt,
                                                               const double* __restrict__ mL,
                                                               const int* __restrict__ len2, const int* __restrict__ sc,
-                                                              int n, int nrows_pad, unsigned char* __restrict__ op) {
+                                                              int n, int nrows_pad, unsigned char* __restrict__ op,
+                                                              double* __restrict__ rowfix) {
     extern __shared__ double s2_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     // odd row stride: the write-back reads one column of 16 rows at a time
@@ -375,6 +380,12 @@ __global__ void __launch_bounds__(32 * kS2FormWarps) k_s2_form(const int* __rest
                 }
                 __syncwarp();
             }
+            if (sizeof(M) == 4) {
+                double d = 0.0;
+                for (int e = lane; e < len; e += 32) d += a[e] - (double)(M)a[e];
+                d = warp_sum(d);
+                if (lane == 0) rowfix[r] = d;
+            }
         }
         __syncthreads();
         for (int p = threadIdx.x; p < kS2FormWarps * w; p += blockDim.x) {
@@ -392,12 +403,13 @@ int schur_form(crimson_lhs* L, const double* mG, const double* Gt, const double*
     cudaStream_t s = L->stream;
     DBuf<unsigned char>& op = s2_op(L, (const M*)nullptr);
     CR_CHECK(s2_buffer<M>(L, op));
+    if (sizeof(M) == 4) CR_CHECK(L->s2_rowfix.alloc((size_t)L->nNo));
     const size_t smem = kS2FormWarps * ((kS2Cap + 1) * sizeof(double) + kS2Cap * sizeof(int));
     CR_CUDA(cudaFuncSetAttribute(k_s2_form<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CR_CUDA(cudaEventRecord(L->s2_ev0, s));
     const int rows = 32 * L->s2_nslice;
     launch(k_s2_form<M>, grid_for(rows, kS2FormWarps, 4), 32 * kS2FormWarps, smem, s, L->rowptr, L->col, mG, Gt, mL,
-           (const int*)L->s2_len.p, (const int*)L->s2_sc.p, L->nNo, rows, op.p);
+           (const int*)L->s2_len.p, (const int*)L->s2_sc.p, L->nNo, rows, op.p, L->s2_rowfix.p);
     CR_CUDA(cudaEventRecord(L->s2_ev1, s));
     CR_CUDA(cudaGetLastError());
     L->s2_form_pending = true;
@@ -455,6 +467,7 @@ struct CgS2Args {
     int n, stages, nvec;     // nvec: vectors over the block's rows in shared memory
     int max_rows, max_cols;  // of a block
     int evict_first;         // the operator exceeds the L2: its lines go first
+    const double* rowfix;    // (n) FP32 operator: what rounding took from the row sums
     double* rhs;             // in: right side; out: solution
     double* R;               // (2 n) the gathered residual, two alternating buffers
     double* Pg;              // (n) P, SP, X when they do not fit in shared memory
@@ -666,9 +679,10 @@ __global__ void __launch_bounds__(32 * kS2CgWarps, 1) k_cg_schur(const __grid_co
         auto finish = [&](double acc) {
             const int t = 32 * (slice - b0.x) + lane;
             if (row0 + t < n) {
-                const double beta = scal[4];
+                const double beta = scal[4], r = Rc[row0 + t];
+                if (sizeof(M) == 4) acc = acc + a.rowfix[row0 + t] * r;
                 const double sv = acc + beta * vp[1][t];
-                const double pr = Rc[row0 + t] + beta * vp[0][t];
+                const double pr = r + beta * vp[0][t];
                 vp[1][t] = sv;
                 vp[0][t] = pr;
                 dps += pr * sv;
@@ -869,6 +883,7 @@ int cg_schur_launch(crimson_lhs* L, double* R, int nface, const double* coef, do
     a.nvec = nvec;
     a.max_rows = L->s2_max_rows;
     a.evict_first = s2_op(L, (const M*)nullptr).n > (size_t)80 << 20;
+    a.rowfix = L->s2_rowfix.p;
     a.rhs = R;
     a.R = L->s2_R.p;
     a.Pg = L->cgPd.p;

@@ -141,9 +141,10 @@ class FlowParams:
     precision: str = "fp64"
     max_refine: int = 4
     refine_tol: float = 0.0
-    # Mixed precision only: 1 runs the inner CG on the explicit FP32 Schur
-    # operator S = L - Gt G formed once per NS solve, 0 (default) on the two
-    # FP32 products L P and Gt (G P) (crimson_memls_ls_set_schur).
+    # 1: crimson_memls_schur_info reports the explicit Schur operator S = L -
+    # Gt G of the inner CG, and the "mixed_f32_tangent" solve uses it too
+    # (crimson_memls_ls_set_schur); "fp64" and "mixed" use it where the pattern
+    # allows.
     explicit_schur: int = 0
 
     def outlets(self) -> list:

@@ -164,14 +164,15 @@ int crimson_memls_ls_free(crimson_ls* ls);
  * pressure relative to the FP64 tangent). */
 int crimson_memls_ls_set_precision(crimson_ls* ls, int precision, int max_refine, double refine_tol);
 /* Form of the inner CG's operator (no counterpart in the reference).  CGRAD
- * multiplies by S = L - Gt G.  FP64 solves form S once per NSSOLVER call on
- * the node graph's 2-ring where the pattern allows (every |col - row| of the
- * 2-ring fits 16 bits, no row of it has more than 256 entries), which makes
- * an iteration one sparse product and two grid barriers; on other patterns
- * they multiply by L and Gt G as two products, as memLS does.  The
- * mixed-precision solve multiplies by two FP32 products (explicit_schur = 0,
- * the default) or, with explicit_schur = 1 and where the pattern allows, by S
- * formed in FP64 and rounded once to FP32. */
+ * multiplies by S = L - Gt G.  Where the pattern allows (every |col - row| of
+ * the node graph's 2-ring fits 16 bits and no row of it has more than 256
+ * entries) each NSSOLVER call forms S in FP64 -- for CRIMSON_MIXED rounded to
+ * FP32 with an FP64 term per row that keeps the row sums -- which makes a CG
+ * iteration one sparse product and two grid barriers; on other patterns it
+ * multiplies by L and Gt G as two products, as memLS does.
+ * explicit_schur = 1 (default 0): crimson_memls_schur_info reports the
+ * operator's state for this ls, and CRIMSON_MIXED_F32_TANGENT solves, which
+ * otherwise multiply by two FP32 products, use it too. */
 int crimson_memls_ls_set_schur(crimson_ls* ls, int explicit_schur);
 /* Per-solve log in the format of memLS's memLS_NS.log (LOGFILE,
  * flowsolver/src/memLS.f90:1720-1757), appended to path after every solve
@@ -542,11 +543,10 @@ int crimson_memls_kernel_time(crimson_lhs* lhs, int which, int reps, double* ms)
 int crimson_memls_cg_layout(const crimson_lhs* lhs, int* resident64, int* resident32, long long* smem_bytes);
 
 /* Diagnostics of the explicit Schur operator on this lhs: state 1 = built and
- * used by the solves whose ls asked for it (crimson_memls_ls_set_schur), -1 =
- * the pattern does not allow it, 0 = no such solve has run; nnz / npad = its
- * entries and sliced positions (padding included; 0: not in use, also by FP64
- * solves); form_ms = average time of one formation (CUDA events).  Valid
- * after a solve. */
+ * used by CGRAD, -1 = the pattern does not allow it, 0 = no solve whose ls
+ * asked for the report (crimson_memls_ls_set_schur) has run; nnz / npad = its
+ * entries and sliced positions (padding included; 0: not in use); form_ms =
+ * average time of one formation (CUDA events).  Valid after a solve. */
 int crimson_memls_schur_info(const crimson_lhs* lhs, int* state, long long* nnz, long long* npad, double* form_ms);
 
 /* Number of CUDA kernels this library has launched since it was loaded. */
