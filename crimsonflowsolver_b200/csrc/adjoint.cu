@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(128) k_adj_interior(const int4* __restrict__ i
             double xl[4][3], dxidx[3][3];
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const double4 xx = x[nd[a]];
+                const double4 xx = ld32(x + nd[a]);
                 xl[a][0] = xx.x;
                 xl[a][1] = xx.y;
                 xl[a][2] = xx.z;
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(128) k_adj_interior(const int4* __restrict__ i
         double u[3] = {0, 0, 0}, L[3] = {0, 0, 0}, l[3] = {0, 0, 0}, res[3] = {0, 0, 0};
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            const double4 ll = lam[nd[a]], yy = y[nd[a]], aa = ac[nd[a]];
+            const double4 ll = ld32(lam + nd[a]), yy = y[nd[a]], aa = ac[nd[a]];
             const double l3[3] = {ll.x, ll.y, ll.z}, u3[3] = {yy.x, yy.y, yy.z}, a3[3] = {aa.x, aa.y, aa.z};
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
@@ -330,10 +330,11 @@ __global__ void __launch_bounds__(128) k_adj_interior(const int4* __restrict__ i
         double o[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) o[i] = W * (yb[i] + s[0] * gb[0][i] + s[1] * gb[1][i] + s[2] * gb[2][i]);
-        r4[2 * q] = make_double4(o[0], o[1], o[2], W * (C.SN[q] * trL + s[0] * gpb[0] + s[1] * gpb[1] + s[2] * gpb[2]));
-        r4[2 * q + 1] = make_double4(W * ab[0], W * ab[1], W * ab[2], 0.0);
-        r4[8 + q] = make_double4(s[0], s[1], s[2], 0.0);
-        if (q == 0) r4[12] = make_double4(-W * gpb[0], -W * gpb[1], -W * gpb[2], 0.0);
+        st32(r4 + 2 * q, make_double4(o[0], o[1], o[2],
+                                      W * (C.SN[q] * trL + s[0] * gpb[0] + s[1] * gpb[1] + s[2] * gpb[2])));
+        st32(r4 + 2 * q + 1, make_double4(W * ab[0], W * ab[1], W * ab[2], 0.0));
+        st32(r4 + 8 + q, make_double4(s[0], s[1], s[2], 0.0));
+        if (q == 0) st32(r4 + 12, make_double4(-W * gpb[0], -W * gpb[1], -W * gpb[2], 0.0));
         mub += W * mb;
     }
     mub = block_sum(mub, sm);
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(256) k_adj_qnode(const int* __restrict__ diag,
         for (int p = soff[d] + sub; p < p1; p += kAdjLanes) {
             const int t = slist[p];
             const double4* r4 = reinterpret_cast<const double4*>(erec + (size_t)kAdjRS * (t >> 4));
-            const double4 s = r4[8 + ((t >> 2) & 3)], v = r4[12];
+            const double4 s = ld32(r4 + 8 + ((t >> 2) & 3)), v = ld32(r4 + 12);
             q[0] += s.x * v.x;
             q[1] += s.x * v.y;
             q[2] += s.x * v.z;
@@ -402,7 +403,7 @@ __global__ void __launch_bounds__(128) k_adj_asiq(const int4* __restrict__ ien, 
         double xl[4][3], ul[4][3];
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            const double4 xx = x[nd[a]];
+            const double4 xx = ld32(x + nd[a]);
             const double4 yy = y[nd[a]];
             xl[a][0] = xx.x;
             xl[a][1] = xx.y;
@@ -431,8 +432,8 @@ __global__ void __launch_bounds__(128) k_adj_asiq(const int4* __restrict__ ien, 
         mub += 2.0 * (qb[0] * g[0][0] + qb[4] * g[1][1] + qb[8] * g[2][2]) + s12 * (g[0][1] + g[1][0]) +
                s13 * (g[0][2] + g[2][0]) + s23 * (g[1][2] + g[2][1]);
         double4* r = reinterpret_cast<double4*>(grec + 8 * (size_t)e);
-        r[0] = make_double4(2.0 * mu * qb[0], 2.0 * mu * qb[4], 2.0 * mu * qb[8], mu * s12);
-        r[1] = make_double4(mu * s13, mu * s23, 0.0, 0.0);
+        st32(r, make_double4(2.0 * mu * qb[0], 2.0 * mu * qb[4], 2.0 * mu * qb[8], mu * s12));
+        st32(r + 1, make_double4(mu * s13, mu * s23, 0.0, 0.0));
     }
     mub = block_sum(mub, sm);
     if (threadIdx.x == 0) mupart[blockIdx.x] = mub;
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(256) k_adj_node(const int* __restrict__ diag, 
         for (int p = soff[d] + sub; p < p1; p += kAdjLanes) {
             const int t = slist[p], a = (t >> 2) & 3;
             const double4* r4 = reinterpret_cast<const double4*>(erec + (size_t)kAdjRS * (t >> 4));
-            const double4 yy = r4[2 * a], aa = r4[2 * a + 1];
+            const double4 yy = ld32(r4 + 2 * a), aa = ld32(r4 + 2 * a + 1);
             v[0] += yy.x;
             v[1] += yy.y;
             v[2] += yy.z;
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(256) k_adj_node(const int* __restrict__ diag, 
             v[6] += aa.z;
             if (grec) {
                 const double4* q4 = reinterpret_cast<const double4*>(grec + 8 * (size_t)(t >> 4));
-                const double4 s = r4[8 + a], A = q4[0], B = q4[1];
+                const double4 s = ld32(r4 + 8 + a), A = ld32(q4), B = ld32(q4 + 1);
                 v[0] += s.x * A.x + s.y * A.w + s.z * B.x;
                 v[1] += s.x * A.w + s.y * A.y + s.z * B.y;
                 v[2] += s.x * B.x + s.y * B.y + s.z * A.z;

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(128) k_asiq_rec(const int4* __restrict__ ien, 
         double xl[4][3], ul[4][3];
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            double4 xv = x[nd[a]];
+            double4 xv = ld32(x + nd[a]);
             double4 yv = y[nd[a]];
             xl[a][0] = xv.x;
             xl[a][1] = xv.y;
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(128) k_asiq_rec(const int4* __restrict__ ien, 
                 g[k][i] = shg[0][k] * ul[0][i] + shg[1][k] * ul[1][i] + shg[2][k] * ul[2][i] + shg[3][k] * ul[3][i];
         const double mu = P.mu;
         double4* r = reinterpret_cast<double4*>(qrec + 8 * (size_t)e);
-        r[0] = make_double4(W, 2.0 * mu * g[0][0], mu * (g[0][1] + g[1][0]), mu * (g[0][2] + g[2][0]));
-        r[1] = make_double4(2.0 * mu * g[1][1], mu * (g[1][2] + g[2][1]), 2.0 * mu * g[2][2], 0.0);
+        st32(r, make_double4(W, 2.0 * mu * g[0][0], mu * (g[0][1] + g[1][0]), mu * (g[0][2] + g[2][0])));
+        st32(r + 1, make_double4(2.0 * mu * g[1][1], mu * (g[1][2] + g[2][1]), 2.0 * mu * g[2][2], 0.0));
     }
 }
 
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) k_q_node(const int* __restrict__ diag, co
             const int t = slist[p];
             const int e = t >> 4, a = (t >> 2) & 3;
             const double4* r = reinterpret_cast<const double4*>(qrec + 8 * (size_t)e);
-            const double4 A = r[0], B = r[1];
+            const double4 A = ld32(r), B = ld32(r + 1);
             const double wa = A.x * c_el.SN[a];
             // qdi(1:9) column-major 3x3, symmetric
             const double qd[9] = {A.y, A.z, A.w, A.z, B.x, B.y, A.w, B.y, B.z};
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(128, 4) k_asigmr(const int4* __restrict__ ien,
         }
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            double4 xv = live ? x[nd[a]] : make_double4(0, 0, 0, 0);
+            double4 xv = live ? ld32(x + nd[a]) : make_double4(0, 0, 0, 0);
             double4 yv = live ? y[nd[a]] : make_double4(0, 0, 0, 0);
             xl[a][0] = xv.x;
             xl[a][1] = xv.y;
@@ -489,8 +489,8 @@ __global__ void __launch_bounds__(128, 4) k_asigmr(const int4* __restrict__ ien,
             double v[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) v[i] = sN[i] + shg[a][0] * sG[i][0] + shg[a][1] * sG[i][1] + shg[a][2] * sG[i][2];
-            reinterpret_cast<double4*>(rec + RO)[a] = make_double4(-WdetJ * v[0], -WdetJ * v[1], -WdetJ * v[2],
-                                                                   WdetJ * div_ub);
+            st32(reinterpret_cast<double4*>(rec + RO) + a,
+                 make_double4(-WdetJ * v[0], -WdetJ * v[1], -WdetJ * v[2], WdetJ * div_ub));
         }
         if (kLhs == 1 && live) {
             const double lhsFct = P.alfi * P.gami * P.Delt;
@@ -521,9 +521,9 @@ __global__ void __launch_bounds__(128, 4) k_asigmr(const int4* __restrict__ ien,
                 Kd[b] = tsFct * c_el.M[a][b] + tlW * (rho * conv + 4.0 * mu * grad + sym);
             }
             double4* r4 = reinterpret_cast<double4*>(rec);
-            r4[5 + a] = make_double4(Kd[0], Kd[1], Kd[2], Kd[3]);
-            r4[1 + a] = make_double4(shg[a][0], shg[a][1], shg[a][2], 0.0);
-            if (a == 3) r4[0] = make_double4(tlW * TC, tlW * 4.0 * mu, tlW, tlW / rho * TM);
+            st32(r4 + 5 + a, make_double4(Kd[0], Kd[1], Kd[2], Kd[3]));
+            st32(r4 + 1 + a, make_double4(shg[a][0], shg[a][1], shg[a][2], 0.0));
+            if (a == 3) st32(r4, make_double4(tlW * TC, tlW * 4.0 * mu, tlW, tlW / rho * TM));
         }
         if (kLhs == 2 && live) {
             // FP32 element quadrature of the tangent
@@ -589,10 +589,10 @@ template <int kLhs>
 __device__ __forceinline__ void record_block(const double* __restrict__ rec, int a, int b, double o[13]) {
     if (kLhs == 1) {
         const double4* r4 = reinterpret_cast<const double4*>(rec);
-        const double4 sc = r4[0], ga = r4[1 + a], gb = r4[1 + b];
+        const double4 sc = ld32(r4), ga = ld32(r4 + 1 + a), gb = ld32(r4 + 1 + b);
         const double sa[3] = {ga.x, ga.y, ga.z};
         const double sb[3] = {gb.x, gb.y, gb.z};
-        const double Kd = rec[20 + 4 * a + b];
+        const double Kd = __ldg(rec + 20 + 4 * a + b);
         pair_block<double>(sa, sb, Kd, sc.x, sc.y, sc.z * c_el.SN[a], sc.w, o);
     } else {
         const float* rf = reinterpret_cast<const float*>(rec + 16);
@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(256) k_node_pass(const int* __restrict__ diag,
             const int t = slist[p];
             const int e = t >> 4, a = (t >> 2) & 3;
             const double* rec = erec + (size_t)RS * (size_t)e;
-            const double4 rl = reinterpret_cast<const double4*>(rec + RO)[a];
+            const double4 rl = ld32(reinterpret_cast<const double4*>(rec + RO) + a);
             r0 += rl.x;
             r1 += rl.y;
             r2 += rl.z;
@@ -806,6 +806,10 @@ __global__ void __launch_bounds__(256) k_node_pass(const int* __restrict__ diag,
 // Slot pass: every off-diagonal CSR block (i, j) from the elements that
 // contain the edge (ascending element order).  One thread per slot; the
 // diagonal slots (first contribution with a == b) belong to the node pass.
+// Bound by the lines its record reads touch (every lane another record): four
+// 32-byte loads per contribution.  The FP64 blocks of a warp's 32 slots are
+// written through shared memory: from the lanes, a block's 13 values lie 72 and
+// 32 bytes apart between lanes and every store touches 18 lines.
 template <int kLhs, bool kProj>
 __global__ void __launch_bounds__(256) k_slot_pass(const int* __restrict__ soff, const int* __restrict__ slist,
                                                    const double* __restrict__ erec, long long nnz,
@@ -814,14 +818,19 @@ __global__ void __launch_bounds__(256) k_slot_pass(const int* __restrict__ soff,
                                                    double* __restrict__ lhsK, double* __restrict__ lhsP,
                                                    float* __restrict__ lhs32) {
     constexpr int RS = RecLayout<kLhs>::RS;
-    for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < nnz;
-         s += (long long)gridDim.x * blockDim.x) {
-        const int p0 = soff[s], p1 = soff[s + 1];
-        const int t0 = slist[p0];
-        if (((t0 >> 2) & 3) == (t0 & 3)) continue;
+    __shared__ double stage[kLhs == 1 ? 8 : 1][32 * 13];
+    const int lane = threadIdx.x & 31;
+    double* const st = stage[kLhs == 1 ? threadIdx.x >> 5 : 0];
+    // warp-uniform loop over 32 slots at a time
+    for (long long s0 = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); s0 < nnz;
+         s0 += (long long)gridDim.x * blockDim.x) {
+        const long long s = s0 + lane;
+        const int p0 = s < nnz ? soff[s] : 0, p1 = s < nnz ? soff[s + 1] : 0;
+        const int t0 = s < nnz ? slist[p0] : 0;
+        const bool mine = ((t0 >> 2) & 3) != (t0 & 3);   // false past the end
         // bc3LHS: row operation of the row node, column operation of the column node
         NodeBC ni{0, 0.0, 0.0, 0.0}, nj{0, 0.0, 0.0, 0.0};
-        if (kProj) {
+        if (kProj && mine) {
             const int4 nn = ien[t0 >> 4];
             const int na[4] = {nn.x, nn.y, nn.z, nn.w};
             ni = node_bc(iBC, BC, ndofBC, na[(t0 >> 2) & 3]);
@@ -829,7 +838,7 @@ __global__ void __launch_bounds__(256) k_slot_pass(const int* __restrict__ soff,
         }
         const bool proj = kProj && (bc_partial(ni.m) || bc_partial(nj.m));
         double acc[13] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-        for (int p = p0; p < p1; ++p) {
+        for (int p = p0; p < (mine ? p1 : p0); ++p) {
             const int t = p == p0 ? t0 : slist[p];
             const int e = t >> 4, a = (t >> 2) & 3, b = t & 3;
             double o[13];
@@ -846,7 +855,25 @@ __global__ void __launch_bounds__(256) k_slot_pass(const int* __restrict__ soff,
 #pragma unroll
             for (int c = 0; c < 13; ++c) acc[c] += o[c];
         }
-        store_block<kLhs>(s, acc, lhsK, lhsP, lhs32);
+        if (kLhs != 1) {
+            if (mine) store_block<kLhs>(s, acc, lhsK, lhsP, lhs32);
+            continue;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, mine);
+#pragma unroll
+        for (int c = 0; c < 13; ++c) st[13 * lane + c] = acc[c];
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int v = lane + 32 * k, b = v / 9;
+            if ((m >> b) & 1) lhsK[9 * (size_t)s0 + v] = st[13 * b + (v - 9 * b)];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int v = lane + 32 * k, b = v >> 2;
+            if ((m >> b) & 1) lhsP[4 * (size_t)s0 + v] = st[13 * b + 9 + (v & 3)];
+        }
+        __syncwarp();
     }
 }
 

@@ -106,6 +106,21 @@ inline int grid_for(long long n, int block, int per_sm = 8) {
 }
 
 // ---------------------------------------------------------------------------
+// 32-byte accesses (one sector): a double4 as one 256-bit instruction instead
+// of two of 128 bits.  Lanes that read records at unrelated addresses are bound
+// by the lines an instruction touches, so this halves their cost.  The address
+// must be 32-byte aligned: the library's own arrays, not a caller's.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double4 ld32(const double4* p) {
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st32(double4* p, const double4& v) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // Warp / block reductions (FP64)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v) {

@@ -139,7 +139,7 @@ __device__ __forceinline__ void sclr_gather_x(const int4 nn, const double4* __re
     const int nd[4] = {nn.x, nn.y, nn.z, nn.w};
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        const double4 v = x[nd[a]];
+        const double4 v = ld32(x + nd[a]);
         xl[a][0] = v.x;
         xl[a][1] = v.y;
         xl[a][2] = v.z;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(128) k_sclr_q(const int4* __restrict__ ien, co
         for (int n = 0; n < 4; ++n)
 #pragma unroll
             for (int k = 0; k < 3; ++k) gT[k] = gT[k] + shg[n][k] * sl[n];
-        qrec[e] = make_double4(diffus * gT[0], diffus * gT[1], diffus * gT[2], W);
+        st32(qrec + e, make_double4(diffus * gT[0], diffus * gT[1], diffus * gT[2], W));
     }
 }
 
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256) k_sclr_qnode(const int* __restrict__ diag
         for (int p = soff[d] + sub; p < p1; p += kNodeLanes) {
             const int t = slist[p];
             const int a = (t >> 2) & 3;
-            const double4 r = qrec[t >> 4];
+            const double4 r = ld32(qrec + (t >> 4));
             double ql0 = 0.0, ql1 = 0.0, ql2 = 0.0, rm = 0.0;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -370,13 +370,13 @@ __global__ void __launch_bounds__(128, 3) k_sclr_elem(const int4* __restrict__ i
                 for (int b = 0; b < 4; ++b) xS[a][b] = 0.0;
         }
         double4* r = reinterpret_cast<double4*>(erec + 8 * (size_t)e);
-        r[0] = make_double4(rl[0], xS[0][0], rl[1], xS[1][1]);
-        r[1] = make_double4(rl[2], xS[2][2], rl[3], xS[3][3]);
+        st32(r, make_double4(rl[0], xS[0][0], rl[1], xS[1][1]));
+        st32(r + 1, make_double4(rl[2], xS[2][2], rl[3], xS[3][3]));
         if (P.lhs) {
             double4* o = reinterpret_cast<double4*>(xoff + 12 * (size_t)e);
-            o[0] = make_double4(xS[0][1], xS[0][2], xS[0][3], xS[1][0]);
-            o[1] = make_double4(xS[1][2], xS[1][3], xS[2][0], xS[2][1]);
-            o[2] = make_double4(xS[2][3], xS[3][0], xS[3][1], xS[3][2]);
+            st32(o, make_double4(xS[0][1], xS[0][2], xS[0][3], xS[1][0]));
+            st32(o + 1, make_double4(xS[1][2], xS[1][3], xS[2][0], xS[2][1]));
+            st32(o + 2, make_double4(xS[2][3], xS[3][0], xS[3][1], xS[3][2]));
         }
     }
 }

@@ -43,6 +43,8 @@ struct Vec4<double> {
         const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 1);
         return make_double4(a.x, a.y, b.x, b.y);
     }
+    // one row of a sliced block (the library's own, 32-byte aligned array)
+    static __device__ __forceinline__ double4 load_block(const double4* p) { return ld32(p); }
     static __device__ __forceinline__ double4 make(double a, double b, double c, double d) {
         return make_double4(a, b, c, d);
     }
@@ -51,6 +53,7 @@ template <>
 struct Vec4<float> {
     using type = float4;
     static __device__ __forceinline__ float4 load(const float4* p) { return __ldg(p); }
+    static __device__ __forceinline__ float4 load_block(const float4* p) { return __ldg(p); }
     static __device__ __forceinline__ float4 make(float a, float b, float c, float d) { return make_float4(a, b, c, d); }
 };
 
@@ -93,10 +96,10 @@ __global__ void __launch_bounds__(256) k_spmv4(const int* __restrict__ sp, const
             for (int u = 0; u < UN; ++u) {
                 const size_t pos = (size_t)base + (size_t)kS4Slice * ((k0 + u < w) ? (k0 + u) : 0);
                 x[u] = V::load(U + __ldg(scol + pos));
-                b0[u] = V::load(blk + 4 * pos + 0);
-                b1[u] = V::load(blk + 4 * pos + 1);
-                b2[u] = V::load(blk + 4 * pos + 2);
-                b3[u] = V::load(blk + 4 * pos + 3);
+                b0[u] = V::load_block(blk + 4 * pos + 0);
+                b1[u] = V::load_block(blk + 4 * pos + 1);
+                b2[u] = V::load_block(blk + 4 * pos + 2);
+                b3[u] = V::load_block(blk + 4 * pos + 3);
             }
 #pragma unroll
             for (int u = 0; u < UN; ++u) {
