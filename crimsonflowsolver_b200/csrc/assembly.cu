@@ -299,13 +299,226 @@ struct RecLayout {
     static constexpr int RO = kLhs == 1 ? 36 : 0;
 };
 
-// Four blocks of 128 threads per SM (128 registers).
+// Sum over an element's four lanes (fixed butterfly).
+__device__ __forceinline__ double quad_add(double v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return v;
+}
+// Sums over an element's four lanes of 16 values each, v[4 a .. 4 a + 3] going
+// to lane a (12 exchanges).
+__device__ __forceinline__ void quad_scatter(const double v[16], int lane4, double out[4]) {
+    double h[8];
+    const bool hi = lane4 & 2, od = lane4 & 1;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const double give = hi ? v[k] : v[8 + k];
+        h[k] = (hi ? v[8 + k] : v[k]) + __shfl_xor_sync(0xffffffffu, give, 2);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double give = od ? h[k] : h[4 + k];
+        out[k] = (od ? h[4 + k] : h[k]) + __shfl_xor_sync(0xffffffffu, give, 1);
+    }
+}
+
+// FP64 element kernel (kLhs 1 with the tangent, 0 residual only).  Lane q
+// evaluates quadrature point q and its terms of all four rows; the rows' sums
+// over the points are then scattered to the lanes, lane a finishing row a.
+// Exchanging the points' quantities through shared memory instead (28 values
+// written, about 120 read per lane) kept the shared-memory pipe at 79% and the
+// FP64 pipe at 42%.  Four blocks of 128 threads per SM (128 registers).
 template <int kLhs>
 __global__ void __launch_bounds__(128, 4) k_asigmr(const int4* __restrict__ ien, const double4* __restrict__ x,
                                                 const double4* __restrict__ y, const double4* __restrict__ ac,
                                                 const double* __restrict__ qres, int nelem, ElmParams P,
                                                 double* __restrict__ erec) {
     constexpr int RS = RecLayout<kLhs>::RS, RO = RecLayout<kLhs>::RO;
+    const int lane4 = threadIdx.x & 3;
+    double Nq[4], Ma[4];   // the point's shape values, row a of the mass table
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        Nq[n] = c_el.shp[lane4][n];
+        Ma[n] = kLhs ? c_el.M[lane4][n] : 0.0;
+    }
+    const int ngroups = gridDim.x * (blockDim.x >> 2);
+    // warp-uniform loop: the shuffles always see all lanes; lanes past the
+    // last element repeat it and write nothing
+    for (int e0 = blockIdx.x * (blockDim.x >> 2); e0 < nelem; e0 += ngroups) {
+        const bool live = e0 + (int)(threadIdx.x >> 2) < nelem;
+        const int e = live ? e0 + (int)(threadIdx.x >> 2) : nelem - 1;
+        const int4 nn = ien[e];
+        const int nd[4] = {nn.x, nn.y, nn.z, nn.w};
+        double dxidx[3][3], shg[4][3], WdetJ;
+        {
+            double xl[4][3];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const double4 xv = ld32(x + nd[a]);
+                xl[a][0] = xv.x;
+                xl[a][1] = xv.y;
+                xl[a][2] = xv.z;
+            }
+            elem_metric(xl, dxidx, shg, &WdetJ);
+        }
+        // gradients g[k][d] of (p, u, v, w) and the point's values
+        double g[3][4], pres = 0.0, u[3] = {0.0, 0.0, 0.0}, aci[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int d = 0; d < 4; ++d) g[k][d] = 0.0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const double4 yv = y[nd[a]], av = ac[nd[a]];
+            pres += Nq[a] * yv.w;
+            u[0] += Nq[a] * yv.x;
+            u[1] += Nq[a] * yv.y;
+            u[2] += Nq[a] * yv.z;
+            aci[0] += Nq[a] * av.x;
+            aci[1] += Nq[a] * av.y;
+            aci[2] += Nq[a] * av.z;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                g[k][0] += shg[a][k] * yv.w;
+                g[k][1] += shg[a][k] * yv.x;
+                g[k][2] += shg[a][k] * yv.y;
+                g[k][3] += shg[a][k] * yv.z;
+            }
+        }
+        // this lane's node and its gradient
+        const double sa[3] = {lane4 == 0 ? shg[0][0] : (lane4 == 1 ? shg[1][0] : (lane4 == 2 ? shg[2][0] : shg[3][0])),
+                              lane4 == 0 ? shg[0][1] : (lane4 == 1 ? shg[1][1] : (lane4 == 2 ? shg[2][1] : shg[3][1])),
+                              lane4 == 0 ? shg[0][2] : (lane4 == 1 ? shg[1][2] : (lane4 == 2 ? shg[2][2] : shg[3][2]))};
+        // div q (e3ivar.f90:354-368): lane a gathers node a's projected flux
+        double divq[3] = {0.0, 0.0, 0.0};
+        if (P.idiff >= 1) {
+            const double* f = qres + 9 * (size_t)(lane4 == 0 ? nd[0] : (lane4 == 1 ? nd[1] : (lane4 == 2 ? nd[2] : nd[3])));
+#pragma unroll
+            for (int i = 0; i < 3; ++i) divq[i] = quad_add(sa[0] * f[i] + sa[1] * f[3 + i] + sa[2] * f[6 + i]);
+        }
+        // metric tensor, tet branch (e3stab.f90:487-528)
+        double gij[6];
+        {
+            const double c1 = 1.259921049894873e+00, c2 = 6.299605249474365e-01;
+            double t1, t2, t3;
+            t1 = c1 * dxidx[0][0] + c2 * (dxidx[1][0] + dxidx[2][0]);
+            t2 = c1 * dxidx[1][0] + c2 * (dxidx[0][0] + dxidx[2][0]);
+            t3 = c1 * dxidx[2][0] + c2 * (dxidx[0][0] + dxidx[1][0]);
+            gij[0] = dxidx[0][0] * t1 + dxidx[1][0] * t2 + dxidx[2][0] * t3;
+            t1 = c1 * dxidx[0][1] + c2 * (dxidx[1][1] + dxidx[2][1]);
+            t2 = c1 * dxidx[1][1] + c2 * (dxidx[0][1] + dxidx[2][1]);
+            t3 = c1 * dxidx[2][1] + c2 * (dxidx[0][1] + dxidx[1][1]);
+            gij[1] = dxidx[0][1] * t1 + dxidx[1][1] * t2 + dxidx[2][1] * t3;
+            gij[3] = dxidx[0][0] * t1 + dxidx[1][0] * t2 + dxidx[2][0] * t3;
+            t1 = c1 * dxidx[0][2] + c2 * (dxidx[1][2] + dxidx[2][2]);
+            t2 = c1 * dxidx[1][2] + c2 * (dxidx[0][2] + dxidx[2][2]);
+            t3 = c1 * dxidx[2][2] + c2 * (dxidx[0][2] + dxidx[1][2]);
+            gij[2] = dxidx[0][2] * t1 + dxidx[1][2] * t2 + dxidx[2][2] * t3;
+            gij[4] = dxidx[0][1] * t1 + dxidx[1][1] * t2 + dxidx[2][1] * t3;
+            gij[5] = dxidx[0][0] * t1 + dxidx[1][0] * t2 + dxidx[2][0] * t3;
+        }
+        // ---- quadrature point q = lane4: e3ivar / e3stab / e3Res ----
+        const double rho = P.rho, mu = P.mu;
+        double rL[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            rL[i] = (aci[i] + u[0] * g[0][i + 1] + u[1] * g[1][i + 1] + u[2] * g[2][i + 1]) * rho + g[i][0] - divq[i];
+        const double rnu = mu / rho;
+        const double dts = P.Dtgl * P.dtsfct;
+        double uGu = u[0] * (gij[0] * u[0] + gij[3] * u[1] + gij[5] * u[2]) +
+                     u[1] * (gij[3] * u[0] + gij[1] * u[1] + gij[4] * u[2]) +
+                     u[2] * (gij[5] * u[0] + gij[4] * u[1] + gij[2] * u[2]);
+        double gg = gij[0] * gij[0] + gij[1] * gij[1] + gij[2] * gij[2] +
+                    2.0 * (gij[3] * gij[3] + gij[4] * gij[4] + gij[5] * gij[5]);
+        double tauM = (2.0 * dts) * (2.0 * dts) + uGu + 36.0 * (rnu * rnu) * gg;
+        double fact = sqrt(tauM);
+        double tauC = rho * 0.125 * fact / (gij[0] + gij[1] + gij[2]) * (P.taucfct / P.dtsfct);
+        tauM = 1.0 / fact;
+        double tauBar = rL[0] * (gij[0] * rL[0] + gij[3] * rL[1] + gij[5] * rL[2]) +
+                        rL[1] * (gij[3] * rL[0] + gij[1] * rL[1] + gij[4] * rL[2]) +
+                        rL[2] * (gij[5] * rL[0] + gij[4] * rL[1] + gij[2] * rL[2]);
+        if (tauBar != 0.0) tauBar = tauM / sqrt(tauBar);
+        double uBar[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) uBar[i] = u[i] - tauM * rL[i] / rho;
+        // e3Res, advective form (e3res.f90:104-284)
+        double rNa[3], rGNa[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            rNa[i] = (aci[i] + uBar[0] * g[0][i + 1] + uBar[1] * g[1][i + 1] + uBar[2] * g[2][i + 1]) * rho;
+        {
+            double divu = g[0][1] + g[1][2] + g[2][3];
+            double tmp = -pres + tauC * divu;
+            double lg[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) lg[i] = tauBar * (rL[0] * g[0][i + 1] + rL[1] * g[1][i + 1] + rL[2] * g[2][i + 1]);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    rGNa[i][j] = mu * (g[j][i + 1] + g[i][j + 1]) + (i == j ? tmp : 0.0) + tauM * rL[i] * u[j] +
+                                 lg[i] * rL[j];
+        }
+        // ---- residual rows (e3res.f90:263-284; momentum 1-3, continuity) ----
+        double v[16], row[4], gam[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            gam[a] = uBar[0] * shg[a][0] + uBar[1] * shg[a][1] + uBar[2] * shg[a][2];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                v[4 * a + i] = Nq[a] * rNa[i] + shg[a][0] * rGNa[i][0] + shg[a][1] * rGNa[i][1] + shg[a][2] * rGNa[i][2];
+            v[4 * a + 3] = gam[a];
+        }
+        quad_scatter(v, lane4, row);
+        double* rec = erec + (size_t)RS * (size_t)e;
+        if (live)
+            st32(reinterpret_cast<double4*>(rec + RO) + lane4,
+                 make_double4(-WdetJ * row[0], -WdetJ * row[1], -WdetJ * row[2], WdetJ * row[3]));
+        if (kLhs == 0) continue;
+        // ---- tangent: Kd rows and the element's scalars ----
+        const double lhsFct = P.alfi * P.gami * P.Delt;
+        const double tlW = lhsFct * WdetJ;
+        const double tsFct = P.almi * WdetJ * rho;
+        const double TC = quad_add(tauC), TM = quad_add(tauM);
+        double al[4], be[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            al[a] = u[0] * shg[a][0] + u[1] * shg[a][1] + u[2] * shg[a][2];
+            be[a] = rL[0] * shg[a][0] + rL[1] * shg[a][1] + rL[2] * shg[a][2];
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = a; b < 4; ++b) {
+                const double sym = tauM * rho * al[a] * al[b] + tauBar * be[a] * be[b];
+                v[4 * a + b] = rho * Nq[a] * gam[b] + sym;
+                v[4 * b + a] = b == a ? v[4 * a + b] : rho * Nq[b] * gam[a] + sym;
+            }
+        quad_scatter(v, lane4, row);
+        if (live) {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const double grad = sa[0] * shg[b][0] + sa[1] * shg[b][1] + sa[2] * shg[b][2];
+                row[b] = tsFct * Ma[b] + tlW * (4.0 * mu * grad + row[b]);
+            }
+            double4* r4 = reinterpret_cast<double4*>(rec);
+            st32(r4 + 5 + lane4, make_double4(row[0], row[1], row[2], row[3]));
+            st32(r4 + 1 + lane4, make_double4(sa[0], sa[1], sa[2], 0.0));
+            if (lane4 == 3) st32(r4, make_double4(tlW * TC, tlW * 4.0 * mu, tlW, tlW / rho * TM));
+        }
+    }
+}
+
+// Element kernel with the FP32 quadrature of the tangent: the points' data
+// exchanged through shared memory.  (Its residual keeps its order of summation:
+// the FP32 tangent of the next nonlinear iteration turns a difference in the
+// last bits into 1e-8 of a time step's result.)  Four blocks of 128 threads per
+// SM (128 registers).
+__global__ void __launch_bounds__(128, 4) k_asigmr_f32(const int4* __restrict__ ien, const double4* __restrict__ x,
+                                                const double4* __restrict__ y, const double4* __restrict__ ac,
+                                                const double* __restrict__ qres, int nelem, ElmParams P,
+                                                double* __restrict__ erec) {
+    constexpr int RS = RecLayout<2>::RS, RO = RecLayout<2>::RO;
     __shared__ double sq[32 * kQE];
     const int lane4 = threadIdx.x & 3;
     double* const sqe = sq + (threadIdx.x >> 2) * kQE;   // this element's per-point data
@@ -492,40 +705,7 @@ __global__ void __launch_bounds__(128, 4) k_asigmr(const int4* __restrict__ ien,
             st32(reinterpret_cast<double4*>(rec + RO) + a,
                  make_double4(-WdetJ * v[0], -WdetJ * v[1], -WdetJ * v[2], WdetJ * div_ub));
         }
-        if (kLhs == 1 && live) {
-            const double lhsFct = P.alfi * P.gami * P.Delt;
-            const double tlW = lhsFct * WdetJ;
-            const double tsFct = P.almi * WdetJ * rho;
-            double TC = 0.0, TM = 0.0, aqa[4], bqa[4], tMq[4], tBq[4];
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) {
-                const double* Sx = Sq[qq];
-                aqa[qq] = Sx[a];
-                bqa[qq] = Sx[4 + a];
-                tMq[qq] = Sx[12];
-                tBq[qq] = Sx[13];
-                TC += Sx[14];
-                TM += Sx[12];
-            }
-            double Kd[4];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                double conv = 0.0, sym = 0.0;
-#pragma unroll
-                for (int qq = 0; qq < 4; ++qq) {
-                    const double* Sx = Sq[qq];
-                    conv += Na[qq] * Sx[8 + b];
-                    sym += tMq[qq] * rho * aqa[qq] * Sx[b] + tBq[qq] * bqa[qq] * Sx[4 + b];
-                }
-                double grad = shg[a][0] * shg[b][0] + shg[a][1] * shg[b][1] + shg[a][2] * shg[b][2];
-                Kd[b] = tsFct * c_el.M[a][b] + tlW * (rho * conv + 4.0 * mu * grad + sym);
-            }
-            double4* r4 = reinterpret_cast<double4*>(rec);
-            st32(r4 + 5 + a, make_double4(Kd[0], Kd[1], Kd[2], Kd[3]));
-            st32(r4 + 1 + a, make_double4(shg[a][0], shg[a][1], shg[a][2], 0.0));
-            if (a == 3) st32(r4, make_double4(tlW * TC, tlW * 4.0 * mu, tlW, tlW / rho * TM));
-        }
-        if (kLhs == 2 && live) {
+        if (live) {
             // FP32 element quadrature of the tangent
             const float rhof = (float)rho, muf = (float)mu;
             const float lhsFct = (float)(P.alfi * P.gami * P.Delt);
@@ -1086,7 +1266,7 @@ int elmgmr_device(crimson_ctx* c, const double* d_y, const double* d_ac, const d
     const int blk = 128;
     const int grid = grid_for((long long)c->nelem * 4, blk, 16);
     if (lhs == 2)
-        launch(k_asigmr<2>, grid, blk, 0, s, c->ien.p, c->x.p, y4, a4, c->qres.p, c->nelem, P, c->erec.p);
+        launch(k_asigmr_f32, grid, blk, 0, s, c->ien.p, c->x.p, y4, a4, c->qres.p, c->nelem, P, c->erec.p);
     else if (lhs)
         launch(k_asigmr<1>, grid, blk, 0, s, c->ien.p, c->x.p, y4, a4, c->qres.p, c->nelem, P, c->erec.p);
     else
