@@ -5,9 +5,10 @@
 // Reference: flowsolver/src/elmgmr.f90:82-555 and the e3* routines it calls.
 //
 // Element kernels use four lanes per linear tet.  In the quadrature phase lane
-// q evaluates quadrature point q (e3ivar/e3stab/e3Res at that point); in the
-// output phase lane a owns row a of the element.  Per-point quantities are
-// exchanged through shared memory.  On a linear tet the metrics, gradients
+// q evaluates quadrature point q (e3ivar/e3stab/e3Res at that point) and its
+// terms of all rows; lane exchanges leave the sums over the points on the lane
+// that writes them (the FP32 tangent's kernel: lane a owns row a, the points'
+// quantities go through shared memory).  On a linear tet the metrics, gradients
 // and div q are element constants, so they are computed once per element
 // (the reference recomputes them per point with identical inputs), and the
 // sums over quadrature points of the tangent terms are formed algebraically:
@@ -25,15 +26,15 @@
 // record per element (its residual rows and the tangent's element constants
 // above: 52 doubles); it never writes a global sum.  A node pass then forms,
 // for every node, the residual row and the diagonal tangent block from the
-// records of the elements containing it, and a slot pass forms every
-// off-diagonal CSR block from the records of the elements containing that
-// edge.  Each sum runs over the pattern pass's contribution list of the
+// records of the elements containing it, and an edge pass (or slot pass)
+// forms every off-diagonal CSR block from the records of the elements
+// containing that edge.  Each sum runs over the pattern pass's contribution list of the
 // slot (ascending element order, the order of the reference's serial
-// scatter, local.f90:64-75, fillsparse.f90:47-60): the slot pass in that
+// scatter, local.f90:64-75, fillsparse.f90:47-60): the edge pass in that
 // order, the node pass over kOwnerLanes lanes per node that take the list
 // round-robin and combine in a fixed butterfly -- so every result is the
 // same bit for bit on every run.  Records are written once and re-read by
-// the 4 (node pass) and 12 (slot pass) owners of their element, mostly from
+// the 4 (node pass) and 6 (edge pass) owners of their element, mostly from
 // L2 on banded node numberings.
 #include <mutex>
 
@@ -280,13 +281,14 @@ __global__ void __launch_bounds__(256) k_q_node(const int* __restrict__ diag, co
 //     [0:4)   tc, tm, tlW, cc = tlW/rho sum_q tauM_q
 //     [4:20)  grad N_a = (shg[a][0..2], 0) at 4 + 4a: a block (a, b) reads
 //             {tc..cc}, grad N_a, grad N_b and Kd(a,b), four sectors
-//     [20:36) Kd(a,b) at 20 + 4a + b
+//     [20:36) Kd(a,a) at 20 + a; Kd(a,b) and Kd(b,a), a < b, side by side
+//     from 24 on (kd_at): the two blocks of an edge read one sector
 //     [36:52) rl(a, 0:4) at 36 + 4a  (momentum 1-3, continuity)
 //   kLhs == 2 (FP32 tangent quadrature), RS = 32: rl at [0:16), then 32
 //     floats at double offset 16 with the FP32 layout of [0:32) above.
 //   kLhs == 0 (residual only), RS = 16: rl at [0:16).
 // ---------------------------------------------------------------------------
-constexpr int kQ = 28;        // doubles of per-point data exchanged in shared memory
+constexpr int kQ = 28;        // doubles of per-point data exchanged in shared memory (FP32 tangent)
 // Shared-memory exchange: element k of a block at k * kQE + q * kQ.  The odd
 // element stride (4 kQ + 1 doubles) puts the 8 elements a warp reads at one
 // index on 8 different bank pairs (conflict-free broadcast reads), and the
@@ -298,6 +300,11 @@ struct RecLayout {
     static constexpr int RS = kLhs == 1 ? 52 : (kLhs == 2 ? 32 : 16);
     static constexpr int RO = kLhs == 1 ? 36 : 0;
 };
+
+// Place of Kd(a, b) among the 16.
+__host__ __device__ constexpr int kd_at(int a, int b) {
+    return a == b ? a : a < b ? 2 + 2 * b + a * (5 - a) : 3 + 2 * a + b * (5 - b);
+}
 
 // Sum over an element's four lanes (fixed butterfly).
 __device__ __forceinline__ double quad_add(double v) {
@@ -324,7 +331,8 @@ __device__ __forceinline__ void quad_scatter(const double v[16], int lane4, doub
 
 // FP64 element kernel (kLhs 1 with the tangent, 0 residual only).  Lane q
 // evaluates quadrature point q and its terms of all four rows; the rows' sums
-// over the points are then scattered to the lanes, lane a finishing row a.
+// over the points are then scattered to the lanes, lane a finishing row a of the
+// residual and the a-th four entries of Kd in the record's order.
 // Exchanging the points' quantities through shared memory instead (28 values
 // written, about 120 read per lane) kept the shared-memory pipe at 79% and the
 // FP64 pipe at 42%.  Four blocks of 128 threads per SM (128 registers).
@@ -335,12 +343,9 @@ __global__ void __launch_bounds__(128, 4) k_asigmr(const int4* __restrict__ ien,
                                                 double* __restrict__ erec) {
     constexpr int RS = RecLayout<kLhs>::RS, RO = RecLayout<kLhs>::RO;
     const int lane4 = threadIdx.x & 3;
-    double Nq[4], Ma[4];   // the point's shape values, row a of the mass table
+    double Nq[4];   // the point's shape values
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-        Nq[n] = c_el.shp[lane4][n];
-        Ma[n] = kLhs ? c_el.M[lane4][n] : 0.0;
-    }
+    for (int n = 0; n < 4; ++n) Nq[n] = c_el.shp[lane4][n];
     const int ngroups = gridDim.x * (blockDim.x >> 2);
     // warp-uniform loop: the shuffles always see all lanes; lanes past the
     // last element repeat it and write nothing
@@ -475,32 +480,32 @@ __global__ void __launch_bounds__(128, 4) k_asigmr(const int4* __restrict__ ien,
             st32(reinterpret_cast<double4*>(rec + RO) + lane4,
                  make_double4(-WdetJ * row[0], -WdetJ * row[1], -WdetJ * row[2], WdetJ * row[3]));
         if (kLhs == 0) continue;
-        // ---- tangent: Kd rows and the element's scalars ----
+        // ---- tangent: Kd and the element's scalars ----
         const double lhsFct = P.alfi * P.gami * P.Delt;
         const double tlW = lhsFct * WdetJ;
         const double tsFct = P.almi * WdetJ * rho;
         const double TC = quad_add(tauC), TM = quad_add(tauM);
-        double al[4], be[4];
+        double al[4], be[4], Nr[4];
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             al[a] = u[0] * shg[a][0] + u[1] * shg[a][1] + u[2] * shg[a][2];
             be[a] = rL[0] * shg[a][0] + rL[1] * shg[a][1] + rL[2] * shg[a][2];
+            Nr[a] = tlW * rho * Nq[a];
         }
+        // the mass and viscous terms ride along as the point's share, so that
+        // what a lane receives is final whichever entries of Kd it gets
+        const double cal = tlW * rho * tauM, cbe = tlW * tauBar, cmu = tlW * mu;
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
             for (int b = a; b < 4; ++b) {
-                const double sym = tauM * rho * al[a] * al[b] + tauBar * be[a] * be[b];
-                v[4 * a + b] = rho * Nq[a] * gam[b] + sym;
-                v[4 * b + a] = b == a ? v[4 * a + b] : rho * Nq[b] * gam[a] + sym;
+                const double grad = shg[a][0] * shg[b][0] + shg[a][1] * shg[b][1] + shg[a][2] * shg[b][2];
+                const double sym = cal * al[a] * al[b] + cbe * be[a] * be[b] + cmu * grad + tsFct * Nq[a] * Nq[b];
+                v[kd_at(a, b)] = Nr[a] * gam[b] + sym;
+                if (b > a) v[kd_at(b, a)] = Nr[b] * gam[a] + sym;
             }
         quad_scatter(v, lane4, row);
         if (live) {
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const double grad = sa[0] * shg[b][0] + sa[1] * shg[b][1] + sa[2] * shg[b][2];
-                row[b] = tsFct * Ma[b] + tlW * (4.0 * mu * grad + row[b]);
-            }
             double4* r4 = reinterpret_cast<double4*>(rec);
             st32(r4 + 5 + lane4, make_double4(row[0], row[1], row[2], row[3]));
             st32(r4 + 1 + lane4, make_double4(sa[0], sa[1], sa[2], 0.0));
@@ -772,7 +777,7 @@ __device__ __forceinline__ void record_block(const double* __restrict__ rec, int
         const double4 sc = ld32(r4), ga = ld32(r4 + 1 + a), gb = ld32(r4 + 1 + b);
         const double sa[3] = {ga.x, ga.y, ga.z};
         const double sb[3] = {gb.x, gb.y, gb.z};
-        const double Kd = __ldg(rec + 20 + 4 * a + b);
+        const double Kd = __ldg(rec + 20 + kd_at(a, b));
         pair_block<double>(sa, sb, Kd, sc.x, sc.y, sc.z * c_el.SN[a], sc.w, o);
     } else {
         const float* rf = reinterpret_cast<const float*>(rec + 16);
@@ -983,8 +988,9 @@ __global__ void __launch_bounds__(256) k_node_pass(const int* __restrict__ diag,
     }
 }
 
-// Slot pass: every off-diagonal CSR block (i, j) from the elements that
-// contain the edge (ascending element order).  One thread per slot; the
+// Slot pass (FP32 tangent, or FP64 with projected nodes): every off-diagonal
+// CSR block (i, j) from the elements that contain the edge (ascending element
+// order).  One thread per slot; the
 // diagonal slots (first contribution with a == b) belong to the node pass.
 // Bound by the lines its record reads touch (every lane another record): four
 // 32-byte loads per contribution.  The FP64 blocks of a warp's 32 slots are
@@ -1054,6 +1060,87 @@ __global__ void __launch_bounds__(256) k_slot_pass(const int* __restrict__ soff,
             if ((m >> b) & 1) lhsP[4 * (size_t)s0 + v] = st[13 * b + 9 + (v & 3)];
         }
         __syncwarp();
+    }
+}
+
+// Edge pass: the blocks (i, j) and (j, i) of every edge i < j from the elements
+// that contain it (ascending element order), FP64.  The two blocks read the
+// same sectors of a record: with M = sum (tc gb ga^T + tm ga gb^T),
+//   K_ij = M + sum Kd(a, b) I,    K_ji = M^T + sum Kd(b, a) I,
+// so one walk over the edge's elements makes both, where a thread per block
+// read every sector twice.  Bound by the lines the record reads touch (four
+// 32-byte sectors per element and edge, every lane another record; L1 pipe 65%)
+// and the DRAM traffic of records and blocks (3.6 TB/s).  The whole assembly of
+// 6M tets: 4.38 ms by blocks, 4.27 by edges (256 threads, two blocks per SM),
+// 4.17 with 128 threads and five blocks (six: 4.27), 4.02 with the two Kd side
+// by side.  A warp's blocks are written
+// through shared memory: from the lanes a block's 13 values lie 72 and 32
+// bytes apart between lanes.
+// Not with projected nodes (bc3LHS changes every element's block by the
+// order of its nodes) nor for the FP32 tangent, whose solves turn another
+// order of sums into 1e-8 of a step's result.
+// uslot: the slots above the diagonal, row by row.
+__global__ void __launch_bounds__(128, 5) k_edge_pass(const int* __restrict__ uslot, const int* __restrict__ trans,
+                                                   const int* __restrict__ soff, const int* __restrict__ slist,
+                                                   const double* __restrict__ erec, long long nedge,
+                                                   double* __restrict__ lhsK, double* __restrict__ lhsP) {
+    __shared__ double stage[4][32 * 13];
+    const int lane = threadIdx.x & 31;
+    double* const st = stage[threadIdx.x >> 5];
+    // warp-uniform loop over 32 edges at a time
+    for (long long u0 = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); u0 < nedge;
+         u0 += (long long)gridDim.x * blockDim.x) {
+        const bool in = u0 + lane < nedge;
+        const int s = in ? uslot[u0 + lane] : 0, l = in ? trans[s] : 0;
+        double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, gij[3] = {0, 0, 0}, gji[3] = {0, 0, 0}, kab = 0.0, kba = 0.0, c = 0.0;
+        const int p1 = in ? soff[s + 1] : 0;
+        for (int p = in ? soff[s] : 0; p < p1; ++p) {
+            const int t = slist[p], a = (t >> 2) & 3, b = t & 3;
+            const double* rec = erec + (size_t)RecLayout<1>::RS * (size_t)(t >> 4);
+            const double4* r4 = reinterpret_cast<const double4*>(rec);
+            const double4 sc = ld32(r4), ga = ld32(r4 + 1 + a), gb = ld32(r4 + 1 + b);
+            const double2 kd = __ldg(reinterpret_cast<const double2*>(rec + 20 + kd_at(min(a, b), max(a, b))));
+            kab += a < b ? kd.x : kd.y;
+            kba += a < b ? kd.y : kd.x;
+            const double sa[3] = {ga.x, ga.y, ga.z}, sb[3] = {gb.x, gb.y, gb.z};
+            const double na = sc.z * c_el.SN[a], nb = sc.z * c_el.SN[b];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) M[3 * i + j] += sc.x * sb[i] * sa[j] + sc.y * sb[j] * sa[i];
+                gij[i] += na * sb[i];
+                gji[i] += nb * sa[i];
+            }
+            c += sc.w * (sa[0] * sb[0] + sa[1] * sb[1] + sa[2] * sb[2]);
+        }
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const double kd = side == 0 ? kab : kba;
+            const int slot = side == 0 ? s : l;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    st[13 * lane + 3 * i + j] = (side == 0 ? M[3 * i + j] : M[3 * j + i]) + (i == j ? kd : 0.0);
+                st[13 * lane + 9 + i] = side == 0 ? gij[i] : gji[i];
+            }
+            st[13 * lane + 12] = c;
+            __syncwarp();
+            const int n = (int)min(32LL, nedge - u0);   // edges of this warp
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const int v = lane + 32 * k, b = v / 9;
+                const size_t at = 9 * (size_t)__shfl_sync(0xffffffffu, slot, b);
+                if (b < n) lhsK[at + (v - 9 * b)] = st[13 * b + (v - 9 * b)];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int v = lane + 32 * k, b = v >> 2;
+                const size_t at = 4 * (size_t)__shfl_sync(0xffffffffu, slot, b);
+                if (b < n) lhsP[at + (v & 3)] = st[13 * b + 9 + (v & 3)];
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -1229,8 +1316,8 @@ __global__ void k_bc3res(const int* __restrict__ iBC, const double* __restrict__
     }
 }
 
-// Grid caps (blocks of 256 per SM) of the owner passes: a grid-stride loop
-// over rows / slots in order, so the cap sets how many rows are in flight.
+// Grid caps (blocks of 256 per SM; the edge pass takes twice as many of 128)
+// of the owner passes: a grid-stride loop over rows / slots in order, so the cap sets how many rows are in flight.
 #ifndef CRIMSON_NODE_PASS_BLOCKS_PER_SM
 #define CRIMSON_NODE_PASS_BLOCKS_PER_SM 8
 #endif
@@ -1308,8 +1395,8 @@ int elmgmr_device(crimson_ctx* c, const double* d_y, const double* d_ac, const d
             launch(k_slot_pass<1, true>, gs, 256, 0, s, c->soff.p, c->slist.p, c->erec.p, c->nnz, c->ien.p, c->iBC.p,
                    c->BC.p, nb, np, d_lhsK, d_lhsP, nullptr);
         else
-            launch(k_slot_pass<1, false>, gs, 256, 0, s, c->soff.p, c->slist.p, c->erec.p, c->nnz, c->ien.p, c->iBC.p,
-                   c->BC.p, nb, np, d_lhsK, d_lhsP, nullptr);
+            launch(k_edge_pass, grid_for(c->nedge, 128, 2 * kSlotPassBlocksPerSM), 128, 0, s, c->uslot.p, c->trans.p,
+                   c->soff.p, c->slist.p, c->erec.p, c->nedge, d_lhsK, d_lhsP);
     } else {
         launch(k_node_pass<0, false>, ng, 256, 0, s, c->diag.p, c->soff.p, c->slist.p, c->erec.p, fno, c->flist.p,
                c->frec.p, c->nshg, c->iBC.p, c->BC.p, nb, np, bcnt, d_res, nullptr, nullptr, nullptr);

@@ -213,6 +213,8 @@ struct crimson_ctx {
     // node i lists exactly the elements containing i (b == a).
     crimson::DBuf<int> slist;       // (nelem*16)
     crimson::DBuf<int> soff;        // (nnz+1)
+    crimson::DBuf<int> uslot;       // (nedge) the slots above the diagonal, row by row
+    long long nedge = 0;
 
     // ElmGMR work space
     crimson::DBuf<double> qres;     // (nshg, 9) node-major: q[9*i + k]

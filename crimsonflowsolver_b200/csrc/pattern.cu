@@ -14,6 +14,7 @@
 //                fillsparse.f90:29-60; replaces sparseloc's searches,
 //                fillsparse.f90:210-246)
 //   diag  - diagonal slot per row                   (diagPtr, memLS.f90:1121-1131)
+//   uslot - the slots above the diagonal (the edges), row by row
 //   trans - slot of the transposed block (j,i)      (solfar.f90:225-232, memLS.f90:1664-1675)
 #include <cub/cub.cuh>
 
@@ -82,6 +83,20 @@ __global__ void k_diag_trans(const int* __restrict__ rowptr, const int* __restri
             trans[j] = t;
             if (t < 0) atomicAdd(bad, 1);
         }
+    }
+}
+
+// Slots above the diagonal: row i has rowptr[i + 1] - diag[i] - 1 of them.
+__global__ void k_upper_count(const int* __restrict__ rowptr, const int* __restrict__ diag, int nshg,
+                              int* __restrict__ cnt) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= nshg; i += gridDim.x * blockDim.x)
+        cnt[i] = i < nshg ? rowptr[i + 1] - diag[i] - 1 : 0;
+}
+__global__ void k_upper_fill(const int* __restrict__ rowptr, const int* __restrict__ diag, const int* __restrict__ off,
+                             int nshg, int* __restrict__ uslot) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nshg; i += gridDim.x * blockDim.x) {
+        const int d = diag[i];
+        for (int j = d + 1; j < rowptr[i + 1]; ++j) uslot[off[i] + j - d - 1] = j;
     }
 }
 
@@ -154,6 +169,18 @@ int build_pattern(crimson_ctx* c) {
         set_last_error("pattern: missing diagonal / transposed block");
         return CRIMSON_ERR_PATTERN;
     }
+    // the pattern is symmetric with its diagonal: half of the rest lies above
+    c->nedge = (c->nnz - c->nshg) / 2;
+    CR_CHECK(c->uslot.alloc((size_t)c->nedge));
+    if (c->nedge > 0) {
+        // counts is no longer needed and holds npair + 1 >= nshg + 1 entries
+        launch(k_upper_count, grid_for(c->nshg + 1, 256), 256, 0, s, c->rowptr.p, c->diag.p, c->nshg, vals.p);
+        CR_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb_scan, vals.p, counts.p, c->nshg + 1, s));
+        launch(k_upper_fill, grid_for(c->nshg, 256), 256, 0, s, c->rowptr.p, c->diag.p, (const int*)counts.p, c->nshg,
+               c->uslot.p);
+        CR_CUDA(cudaStreamSynchronize(s));
+    }
+    CR_CUDA(cudaGetLastError());
     return CRIMSON_OK;
 }
 
