@@ -390,23 +390,19 @@ constexpr int kSellUnroll = 8;
         }                                                                                \
     }
 #define CR_SELL_ROW(sp, scol, r, ...) CR_SELL_ROW_U(kSellUnroll, sp, scol, r, __VA_ARGS__)
-// Entries per stage of the CG's software-pipelined row loops: the matrix
-// records of the next stage are loaded while the current stage's gathers are
-// in flight (two stages live: 2 x 5 x 16 B FP32, 2 x 2 x 32 B FP64, within
-// the 64 registers of two 512-thread blocks per SM).
-template <typename M>
-struct CgStage {
-    static constexpr int value = 5;
-};
-template <>
-struct CgStage<double> {
-    static constexpr int value = 2;
-};
-// Phase A (G P) uses its own stage width (5 FP32 entries, 2 FP64: FP32
-// measured 4% faster per iteration than 4, 6 spills; FP64 3 spills).
+// Entries per stage of the CG's software-pipelined row loops, phases A (G P)
+// and B: the matrix records of the next stage are loaded while the current
+// stage's gathers are in flight.  Two stages are live, and across a barrier
+// the first one, within the 64 registers of two 512-thread blocks per SM: FP32
+// 4 and 3 (5 and 5 spill across the barriers; per iteration on 118k nodes
+// 21.2 us against 22.0, and 4 and 4 21.6), FP64 2 and 2.
 template <typename M>
 struct CgStageA {
-    static constexpr int value = sizeof(M) == 4 ? 5 : 2;
+    static constexpr int value = sizeof(M) == 4 ? 4 : 2;
+};
+template <typename M>
+struct CgStage {
+    static constexpr int value = sizeof(M) == 4 ? 3 : 2;
 };
 
 // KU = K U on the sliced copy: K as {K0..K3} and {K4..K7} 4-vectors (npad
@@ -613,6 +609,47 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
     const int wbase = kRes ? cg_fill_cols(a.sp, a.scol, n, cg_res) : 0;
     constexpr int U = CgStage<M>::value;
     constexpr int UA = CgStageA<M>::value;
+    const int r0 = blockIdx.x * blockDim.x + threadIdx.x, rstride = gridDim.x * blockDim.x;
+    // A row's slice and the first stage of its matrix entries.  They are loaded
+    // before the barrier that the row's gathers wait for: the matrix does not
+    // change, and the loads' latency passes under the wait (per iteration 22.3 ->
+    // 21.2 us on 118k nodes, 89.1 -> 86.1 on 695k).  19 us remain on the
+    // smallest meshes: three barriers with their sums, two passes over a row.
+    // Barriers that carry the sums (gridred.cuh) are slower here, 27 us: each of
+    // the 296 blocks polls the packets of all.
+    int w = 0, base = 0;
+    M g0[UA], g1[UA], g2[UA];
+    int cc[UA > U ? UA : U];
+    typename V4<M>::type gl[U];
+    const auto zero4 = mk4<M>(M(0), M(0), M(0), M(0));
+    auto slice_of = [&](int r) {
+        if (r >= n) return;
+        const int p0 = __ldg(a.sp + (r >> 5));
+        w = (__ldg(a.sp + (r >> 5) + 1) - p0) >> 5;
+        base = p0 + (r & (kSlice - 1));
+    };
+    auto first_a = [&](int r) {
+#pragma unroll
+        for (int u = 0; u < UA; ++u) {
+            const bool in = r < n && u < w;
+            const size_t pos = (size_t)base + kSlice * u;
+            g0[u] = in ? __ldcs(a.G + pos) : M(0);
+            g1[u] = in ? __ldcs(a.G + npad + pos) : M(0);
+            g2[u] = in ? __ldcs(a.G + 2 * npad + pos) : M(0);
+            if (!kRes) cc[u] = in ? __ldg(a.scol + pos) : r;  // resident columns are read at use
+        }
+    };
+    auto first_b = [&](int r) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = r < n && u < w;
+            const size_t pos = (size_t)base + kSlice * u;
+            gl[u] = in ? ldcs4(a.GL + pos) : zero4;
+            if (!kRes) cc[u] = in ? __ldg(a.scol + pos) : r;
+        }
+    };
+    slice_of(r0);
+    first_a(r0);
     const double norm0 = sqrt(*a.rr);
     double err = norm0 * norm0, errO = err;
     double eps = fmax(a.absTol, a.relTol * norm0);
@@ -631,25 +668,10 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
 #pragma unroll
         for (int f = 0; f < (NF > 0 ? NF : 1); ++f) wp[f] = 0.0;
         CgCols<kRes> cs{a.scol, cg_res, wbase, (int)(threadIdx.x & 31)};
-        for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        for (int r = r0; r < n; r += rstride) {
             double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-            const int s_ = r >> 5;
-            const int p0 = __ldg(a.sp + s_);
-            const int w = (__ldg(a.sp + s_ + 1) - p0) >> 5;
-            const int base = p0 + (r & (kSlice - 1));
-            // stage: G values and columns of U entries; the next stage is
+            // stage: G values and columns of UA entries; the next stage is
             // loaded before this stage's gathers
-            M g0[UA], g1[UA], g2[UA];
-            int cc[UA];
-#pragma unroll
-            for (int u = 0; u < UA; ++u) {
-                const bool in = u < w;
-                const size_t pos = (size_t)base + kSlice * u;
-                g0[u] = in ? __ldcs(a.G + pos) : M(0);
-                g1[u] = in ? __ldcs(a.G + npad + pos) : M(0);
-                g2[u] = in ? __ldcs(a.G + 2 * npad + pos) : M(0);
-                cc[u] = (!kRes && in) ? cs.col(r, base, u) : r;  // resident columns are read at use
-            }
             for (int k0 = 0; k0 < w; k0 += UA) {
                 M n0[UA], n1[UA], n2[UA];
                 int nc[UA];
@@ -677,10 +699,14 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
                     g0[u] = n0[u];
                     g1[u] = n1[u];
                     g2[u] = n2[u];
-                    cc[u] = nc[u];
+                    if (!kRes) cc[u] = nc[u];
                 }
             }
             cs.next_row(w);
+            if (r + rstride < n) {
+                slice_of(r + rstride);
+                first_a(r + rstride);
+            }
             const double2 rr = a.recA[r];
             const double pr = first ? rr.x : rr.x + beta * rr.y;
             a.recB[r] = mk4<M>((M)a0, (M)a1, (M)a2, (M)pr);
@@ -696,6 +722,8 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
                 if (threadIdx.x == 0) partA[(size_t)blockIdx.x * kCgPartStride + f] = t;
             }
         }
+        slice_of(r0);
+        first_b(r0);
         grid.sync();
         double cS[NF > 0 ? NF : 1];
 #pragma unroll
@@ -703,20 +731,8 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
         // ---- phase B: SP = L P - Gt GP - sum_f cS_f z_f ; <P, SP> ----
         double dsum = 0.0;
         CgCols<kRes> cb{a.scol, cg_res, wbase, (int)(threadIdx.x & 31)};
-        for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        for (int r = r0; r < n; r += rstride) {
             double lp = 0.0, gg = 0.0;
-            const auto zero4 = mk4<M>(M(0), M(0), M(0), M(0));
-            const int s_ = r >> 5;
-            const int p0 = __ldg(a.sp + s_);
-            const int w = (__ldg(a.sp + s_ + 1) - p0) >> 5;
-            const int base = p0 + (r & (kSlice - 1));
-            int cc[U];
-            typename V4<M>::type gl[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                cc[u] = (!kRes && u < w) ? cb.col(r, base, u) : r;
-                gl[u] = (u < w) ? ldcs4(a.GL + base + kSlice * u) : zero4;
-            }
             for (int k0 = 0; k0 < w; k0 += U) {
                 int ccn[U];  // next stage
                 typename V4<M>::type gln[U];
@@ -737,11 +753,15 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    cc[u] = ccn[u];
+                    if (!kRes) cc[u] = ccn[u];
                     gl[u] = gln[u];
                 }
             }
             cb.next_row(w);
+            if (r + rstride < n) {
+                slice_of(r + rstride);
+                first_b(r + rstride);
+            }
 #pragma unroll
             for (int f = 0; f < NF; ++f)
                 if (f < a.nface) gg += cS[f] * a.z[(size_t)f * n + r];
@@ -765,6 +785,8 @@ __global__ void __launch_bounds__(kCgThreads, 2) k_cg_persistent(CgArgs<M> a) {
         }
         rs = block_sum(rs, sm);
         if (threadIdx.x == 0) partC[(size_t)blockIdx.x * kCgPartStride] = rs;
+        slice_of(r0);
+        first_a(r0);
         grid.sync();
         const double e2 = sqrt(sum_partials(partC, 0, sm));
         err = e2 * e2;
