@@ -443,8 +443,9 @@ __global__ void __launch_bounds__(128) k_adj_asiq(const int4* __restrict__ ien, 
 // records grec, when there are).
 __global__ void __launch_bounds__(256) k_adj_node(const int* __restrict__ diag, const int* __restrict__ soff,
                                                   const int* __restrict__ slist, const double* __restrict__ erec,
-                                                  const double* __restrict__ grec, int nshg, double4* __restrict__ ybar,
-                                                  double4* __restrict__ abar) {
+                                                  const double* __restrict__ grec, int nshg, double* __restrict__ ybar,
+                                                  double* __restrict__ abar) {
+    static_assert(kAdjLanes == 4, "a node's lanes write its four components");
     constexpr int NPW = 32 / kAdjLanes;
     const int lane = threadIdx.x & 31, sub = lane % kAdjLanes;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -476,9 +477,10 @@ __global__ void __launch_bounds__(256) k_adj_node(const int* __restrict__ diag, 
         }
 #pragma unroll
         for (int k = 0; k < 7; ++k) v[k] = adj_lanes_sum(v[k]);
-        if (!valid || sub != 0) continue;
-        ybar[i] = make_double4(v[0], v[1], v[2], v[3]);
-        abar[i] = make_double4(v[4], v[5], v[6], 0.0);
+        if (!valid) continue;
+        // lane sub writes component sub: the caller's arrays, 8-byte aligned
+        ybar[4 * (size_t)i + sub] = sub == 0 ? v[0] : (sub == 1 ? v[1] : (sub == 2 ? v[2] : v[3]));
+        abar[4 * (size_t)i + sub] = sub == 0 ? v[4] : (sub == 1 ? v[5] : (sub == 2 ? v[6] : 0.0));
     }
 }
 
@@ -677,8 +679,8 @@ int elmgmr_vjp(crimson_ctx* c, const double* d_y, const double* d_ac, const doub
         np += ge;
     }
     launch(k_adj_node, gn, 256, 0, s, (const int*)c->diag.p, (const int*)c->soff.p, (const int*)c->slist.p,
-           (const double*)c->erec.p, p.idiff == 1 ? (const double*)c->qrec.p : nullptr, n,
-           reinterpret_cast<double4*>(d_ybar), reinterpret_cast<double4*>(d_abar));
+           (const double*)c->erec.p, p.idiff == 1 ? (const double*)c->qrec.p : nullptr, n, d_ybar,
+           d_abar);
     if (c->nface > 0) {
         launch(k_adj_faces, gf, 128, 0, s, (const int4*)c->ienb.p, (const int*)c->iBCB.p, x4, y4, l4,
                 c->nface, C, P, p.mu, d_ybar, mupart + np);
