@@ -1332,7 +1332,7 @@ int elmgmr_device(crimson_ctx* c, const double* d_y, const double* d_ac, const d
     cudaStream_t s = c->stream;
     // every pass below reads the pattern's contribution lists
     if (c->nnz == 0) CR_CHECK(build_pattern(c));
-    if (!c->diag.p || !c->soff.p || !c->slist.p) return CRIMSON_ERR_STATE;
+    if (!c->diag.p || !c->soff.p || !c->slist.p || !c->trans.p || (c->nedge > 0 && !c->uslot.p)) return CRIMSON_ERR_STATE;
     CR_CHECK(upload_elm_consts(s));
     const ElmParams P = elm_params(c->p);
     const double4* y4 = reinterpret_cast<const double4*>(d_y);

@@ -105,6 +105,8 @@ __global__ void k_to_one_based(const int* __restrict__ in, int* __restrict__ out
     for (; t < n; t += (long long)gridDim.x * blockDim.x) out[t] = in[t] + 1;
 }
 
+// c->nnz and c->nedge are set last: a call that fails part-way leaves the
+// pattern marked as not built, and the next one builds it again.
 int build_pattern(crimson_ctx* c) {
     cudaStream_t s = c->stream;
     const long long npair = (long long)c->nelem * 16;
@@ -145,7 +147,6 @@ int build_pattern(crimson_ctx* c) {
     int hnnz = 0;
     CR_CUDA(cudaMemcpyAsync(&hnnz, dcount.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     CR_CUDA(cudaStreamSynchronize(s));
-    c->nnz = hnnz;
     CR_CHECK(c->rowptr.alloc((size_t)c->nshg + 1));
     CR_CHECK(c->col.alloc((size_t)hnnz));
     CR_CHECK(c->diag.alloc((size_t)c->nshg));
@@ -170,9 +171,9 @@ int build_pattern(crimson_ctx* c) {
         return CRIMSON_ERR_PATTERN;
     }
     // the pattern is symmetric with its diagonal: half of the rest lies above
-    c->nedge = (c->nnz - c->nshg) / 2;
-    CR_CHECK(c->uslot.alloc((size_t)c->nedge));
-    if (c->nedge > 0) {
+    const long long nedge = ((long long)hnnz - c->nshg) / 2;
+    CR_CHECK(c->uslot.alloc((size_t)nedge));
+    if (nedge > 0) {
         // counts is no longer needed and holds npair + 1 >= nshg + 1 entries
         launch(k_upper_count, grid_for(c->nshg + 1, 256), 256, 0, s, c->rowptr.p, c->diag.p, c->nshg, vals.p);
         CR_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb_scan, vals.p, counts.p, c->nshg + 1, s));
@@ -181,6 +182,8 @@ int build_pattern(crimson_ctx* c) {
         CR_CUDA(cudaStreamSynchronize(s));
     }
     CR_CUDA(cudaGetLastError());
+    c->nedge = nedge;
+    c->nnz = hnnz;
     return CRIMSON_OK;
 }
 
