@@ -2712,16 +2712,17 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
     int gm_ok = 0;
     if (ls->GM.sD >= 1 && ls->GM.sD <= kGmMaxSD) CR_CHECK(gm_faces_prepare(L, &gm_ok));
     // One GMRES solve K X = R: k_gmres, whose statistics wait in slot g, or
-    // the launch-per-step form
+    // the form driven by the host (which also sets X = 0 where no cycle may run)
+    const bool gm_one = gm_ok && !kept && ls->GM.mItr >= 1;
     auto gmres_any = [&](const double* R_, double* X_, int g) -> int {
-        if (!gm_ok || kept) return gmres<M, B>(C, ls->GM, (const M*)Ks, R_, X_, gm_ok != 0);
+        if (!gm_one) return gmres<M, B>(C, ls->GM, (const M*)Ks, R_, X_, gm_ok != 0);
         CR_CUDA(cudaEventRecord(L->ev_gm[2 * g], s));
         CR_CHECK((gmres_launch<M, B>(C, ls->GM, (const M*)Ks, R_, X_, kSlotGm + 8 * g)));
         CR_CUDA(cudaEventRecord(L->ev_gm[2 * g + 1], s));
         return CRIMSON_OK;
     };
     auto gmres_stats = [&](int g) -> int {
-        if (!gm_ok || kept) return CRIMSON_OK;
+        if (!gm_one) return CRIMSON_OK;
         float ms = 0.f;
         CR_CUDA(cudaEventElapsedTime(&ms, L->ev_gm[2 * g], L->ev_gm[2 * g + 1]));
         return gmres_finish(C, ls->GM, kSlotGm + 8 * g, 1e-3 * ms);
