@@ -816,7 +816,8 @@ int crimson_memls_bc_create(crimson_lhs* L, int faIn, int nNo, int dof, int BC_t
     f.dof = dof;
     f.bGrp = BC_type;
     f.created = true;
-    L->gm_map_ok = -1;   // GMRES's map of the coupled faces' nodes is built anew
+    for (int k : L->gm_faces)
+        if (k == faIn - 1) L->gm_map_ok = -1;   // GMRES's map of the coupled faces' nodes is built anew
     std::vector<int> g(nNo);
     for (int a = 0; a < nNo; ++a) {
         g[a] = gNodes[a] - 1;
