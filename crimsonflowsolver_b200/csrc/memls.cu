@@ -2246,7 +2246,9 @@ static int cg_resident_bytes(crimson_lhs* L, size_t* bytes) {
     const int n = L->nNo;
     CR_CHECK(L->cg_tmp.alloc(1));
     CR_CUDA(cudaMemsetAsync(L->cg_tmp.p, 0, sizeof(int), s));
-    launch(k_max_offset, grid_for(n, 256), 256, 0, s, (const int*)L->rowptr, (const int*)L->col, n, L->cg_tmp.p);
+    // (an explicit operator's 2-ring offsets fit 16 bits, so these do)
+    if (L->s2_state != 1)
+        launch(k_max_offset, grid_for(n, 256), 256, 0, s, (const int*)L->rowptr, (const int*)L->col, n, L->cg_tmp.p);
     int maxoff = 0;
     CR_CUDA(cudaMemcpyAsync(&maxoff, L->cg_tmp.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     std::vector<int> sp((size_t)L->nslice + 1);
@@ -2268,7 +2270,8 @@ static int cg_resident_bytes(crimson_lhs* L, size_t* bytes) {
 }
 
 // Launch form of the two-product CG kernel on this lhs (kernel family and
-// grid), decided once per precision.
+// grid), decided at the first CGRAD of a precision, whichever operator that
+// takes: crimson_memls_cg_layout reports it.
 template <typename M>
 static int cg_layout(crimson_lhs* L, size_t* rbytes_out) {
     const void* kres[3] = {(const void*)k_cg_persistent<0, M, true>, (const void*)k_cg_persistent<1, M, true>,
@@ -2310,18 +2313,6 @@ static int cg_layout(crimson_lhs* L, size_t* rbytes_out) {
     return CRIMSON_OK;
 }
 
-// Diagnostics: what cg_layout decides for the precisions CGRAD has run in.
-int memls_cg_layout(crimson_lhs* L, int* resident64, int* resident32, long long* smem_bytes) {
-    if (!L->cg_used64 && !L->cg_used32) return CRIMSON_ERR_STATE;
-    size_t rb = 0;
-    if (L->cg_used64) CR_CHECK(cg_layout<double>(L, &rb));
-    if (L->cg_used32) CR_CHECK(cg_layout<float>(L, &rb));
-    if (resident64) *resident64 = L->cg_used64 ? L->cg_res64 : 0;
-    if (resident32) *resident32 = L->cg_used32 ? L->cg_res32 : 0;
-    if (smem_bytes) *smem_bytes = L->cg_res_bytes;
-    return CRIMSON_OK;
-}
-
 // CGRAD (memLS.f90:367-430) on the Schur-like operator L P - Gt G P; R in/out (n).
 // use_s2: on the explicit operator (schur.cu), else with two products on
 // Gs / GLs, the sliced G and {Gt, L} of this NSSOLVER call.  Launches only;
@@ -2332,7 +2323,8 @@ static int cgrad_launch(Ctx& C, const crimson_subls& ls, const M* Gs, const type
     crimson_lhs* L = C.L;
     cudaStream_t s = C.s;
     const int n = L->nNo;
-    (std::is_same<M, float>::value ? L->cg_used32 : L->cg_used64) = true;
+    size_t rbytes = 0;
+    CR_CHECK(cg_layout<M>(L, &rbytes));
     if (use_s2) {
         CR_CUDA(cudaEventRecord(L->ev0, s));
         CR_CHECK(cg_schur_launch<M>(L, R, nface, coef, ls.relTol, ls.absTol, ls.mItr, C.sc(kSlotCg)));
@@ -2340,8 +2332,6 @@ static int cgrad_launch(Ctx& C, const crimson_subls& ls, const M* Gs, const type
         return CRIMSON_OK;
     }
     C.dot((const double*)R, (const double*)R, n, kSlotErr);
-    size_t rbytes = 0;
-    CR_CHECK(cg_layout<M>(L, &rbytes));
     const int grid = std::is_same<M, float>::value ? L->cg_grid32 : L->cg_grid;
     const int mode = std::is_same<M, float>::value ? L->cg_res32 : L->cg_res64;
     const int fi = nface == 0 ? 0 : (nface == 1 ? 1 : 2);

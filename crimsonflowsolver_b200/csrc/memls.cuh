@@ -30,7 +30,6 @@ int schur_faces(crimson_lhs* L, int nface);
 template <typename M>
 int cg_schur_launch(crimson_lhs* L, double* R, int nface, const double* coef, double relTol, double absTol, int mItr,
                     double* out);
-int memls_cg_layout(crimson_lhs* L, int* resident64, int* resident32, long long* smem_bytes);
 
 }  // namespace crimson
 
@@ -71,7 +70,6 @@ struct crimson_lhs {
     DBuf<int> sell_ptr, sell_col;
     DBuf<double> Ks64, Gs64, GLs64;
     DBuf<float> Ks32, Gs32, GLs32;
-    bool cg_used64 = false, cg_used32 = false;   // a CGRAD ran in this precision
     int cg_grid = 0, cg_grid32 = 0;
     int cg_res64 = 0, cg_res32 = 0;    // CG kernel with block-resident columns (per matrix type)
     long long cg_res_bytes = -1;       // its shared memory per block (0: offsets exceed 16 bits); -1 unknown

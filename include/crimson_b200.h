@@ -531,9 +531,10 @@ int crimson_pvsq_noalloc(int nsurf, const int* surf_offsets, const int* d_nodes,
  * Valid after a solve on the lhs. */
 int crimson_memls_kernel_time(crimson_lhs* lhs, int which, int reps, double* ms);
 
-/* Diagnostics: column layout of the two-product CG kernel on this lhs (the
- * form CGRAD takes where the explicit operator does not apply), for the
- * precisions it has been solved in.
+/* Diagnostics: column layout of the two-product CG kernel on this lhs, for the
+ * precisions it has been solved in.  It is decided at the first CGRAD of a
+ * precision, also where CGRAD takes the explicit operator and the kernel does
+ * not run.
  * resident64 / resident32 = 1 when the kernel with FP64 / FP32 matrices keeps
  * every block's column indices in shared memory for the whole launch (16-bit
  * offsets col - row; chosen when the offsets fit and two blocks per SM fit
