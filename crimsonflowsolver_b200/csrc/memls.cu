@@ -2269,6 +2269,10 @@ static int cg_resident_bytes(crimson_lhs* L, size_t* bytes) {
     return CRIMSON_OK;
 }
 
+// Half of an SM's 228 KB less the 1 KB the driver reserves per block: more
+// never fits twice.
+constexpr size_t kCgResidentMax = 113 * 1024;
+
 // Launch form of the two-product CG kernel on this lhs (kernel family and
 // grid), decided at the first CGRAD of a precision, whichever operator that
 // takes: crimson_memls_cg_layout reports it.
@@ -2283,13 +2287,16 @@ static int cg_layout(crimson_lhs* L, size_t* rbytes_out) {
     size_t rbytes = 0;
     CR_CHECK(cg_resident_bytes(L, &rbytes));
     if (grid == 0) {
-        // block-resident columns when two blocks per SM fit with them
+        // block-resident columns when two blocks per SM fit with them; the
+        // kernels' limit is the same for every lhs (a smaller one's own size
+        // would make the launches of a larger one fail)
         mode = 0;
-        if (rbytes > 0) {
+        if (rbytes > 0 && rbytes <= kCgResidentMax) {
             int ok = 1;
             for (const void* f : kres) {
                 int nb = 0;
-                if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rbytes) != cudaSuccess ||
+                if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgResidentMax) !=
+                        cudaSuccess ||
                     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, kCgThreads, rbytes) != cudaSuccess || nb < 2)
                     ok = 0;
             }
