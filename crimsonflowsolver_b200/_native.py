@@ -18,6 +18,8 @@ c_dbl_p = ctypes.POINTER(ctypes.c_double)
 c_void_p = ctypes.c_void_p
 
 OK = 0
+# crimson_memls_cg_form's values
+CG_FORMS = ["none", "schur", "schur_resident", "products", "products_resident"]
 ERRORS = {1: "ARG", 2: "UNSUPPORTED", 3: "CUDA", 4: "OOM", 5: "PATTERN", 6: "SINGULAR", 7: "NONFINITE", 8: "STATE"}
 
 
@@ -81,6 +83,8 @@ SIGNATURES = {
     "crimson_memls_ls_set_precision": (ctypes.c_int, [c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_double]),
     "crimson_memls_refine_info": (ctypes.c_int, [c_void_p, ctypes.POINTER(ctypes.c_int), c_dbl_p]),
     "crimson_memls_ls_set_schur": (ctypes.c_int, [c_void_p, ctypes.c_int]),
+    "crimson_memls_ls_set_two_products": (ctypes.c_int, [c_void_p, ctypes.c_int]),
+    "crimson_memls_cg_form": (ctypes.c_int, [c_void_p, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]),
     "crimson_memls_schur_info": (ctypes.c_int, [c_void_p, ctypes.POINTER(ctypes.c_int),
                                                 ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong),
                                                 c_dbl_p]),

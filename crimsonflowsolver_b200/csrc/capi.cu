@@ -706,6 +706,19 @@ int crimson_memls_ls_set_schur(crimson_ls* ls, int explicit_schur) {
     return CRIMSON_OK;
 }
 
+int crimson_memls_ls_set_two_products(crimson_ls* ls, int on) {
+    if (!ls || on < 0 || on > 1) return CRIMSON_ERR_ARG;
+    ls->two_products = on;
+    return CRIMSON_OK;
+}
+
+int crimson_memls_cg_form(const crimson_lhs* L, int* form64, int* form32) {
+    if (!L) return CRIMSON_ERR_ARG;
+    if (form64) *form64 = L->cg_form64;
+    if (form32) *form32 = L->cg_form32;
+    return CRIMSON_OK;
+}
+
 int crimson_memls_schur_info(const crimson_lhs* L, int* state, long long* nnz, long long* npad, double* form_ms) {
     if (!L) return CRIMSON_ERR_ARG;
     if (state) *state = L->s2_asked ? L->s2_state : 0;

@@ -2348,6 +2348,8 @@ static int cgrad_launch(Ctx& C, const crimson_subls& ls, const M* Gs, const type
                                (const void*)k_cg_persistent<kMaxCoupled, M, true>}};
     const void* kfn = kfns[mode ? 1 : 0][fi];
     const size_t dyn = mode ? rbytes : 0;
+    (std::is_same<M, float>::value ? L->cg_form32 : L->cg_form64) =
+        mode ? CRIMSON_CG_PRODUCTS_RESIDENT : CRIMSON_CG_PRODUCTS;
     CR_CHECK(L->cgPart.alloc(3 * (size_t)kCgPartStride * std::max(L->cg_grid, L->cg_grid32)));
     CR_CHECK(L->cgRecA.alloc(2 * (size_t)n));
     CR_CHECK(L->cgRecB.alloc(4 * (size_t)n));
@@ -2693,9 +2695,9 @@ static int nssolver(crimson_lhs* L, crimson_ls* ls, const double* mK, const doub
     typename V4<M>::type* GLs = nullptr;
     // the FP32-tangent mode keeps the summation orders of its results (k_gmres_cycle)
     const bool kept = ls->precision == CRIMSON_MIXED_F32_TANGENT;
-    // CGRAD's operator: formed explicitly where the pattern allows (schur.cu);
-    // in the FP32-tangent mode only on request
-    const bool want_s2 = !kept || ls->schur;
+    // CGRAD's operator: formed explicitly where the pattern allows (schur.cu)
+    // and two products were not asked for; in the FP32-tangent mode only on request
+    const bool want_s2 = !ls->two_products && (!kept || ls->schur);
     if (want_s2) CR_CHECK(schur_pattern(L));
     const bool use_s2 = want_s2 && L->s2_state == 1;
     if (ls->schur) L->s2_asked = true;

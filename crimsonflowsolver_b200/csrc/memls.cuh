@@ -70,6 +70,7 @@ struct crimson_lhs {
     DBuf<int> sell_ptr, sell_col;
     DBuf<double> Ks64, Gs64, GLs64;
     DBuf<float> Ks32, Gs32, GLs32;
+    int cg_form64 = 0, cg_form32 = 0;   // CRIMSON_CG_*: what the last CGRAD of a precision ran
     int cg_grid = 0, cg_grid32 = 0;
     int cg_res64 = 0, cg_res32 = 0;    // CG kernel with block-resident columns (per matrix type)
     long long cg_res_bytes = -1;       // its shared memory per block (0: offsets exceed 16 bits); -1 unknown
@@ -131,6 +132,7 @@ struct crimson_ls {
     int max_refine = 4;            // FP64 refinement sweeps of the mixed solve
     double refine_tol = 0.0;       // target |R - A x| / |R|; <= 0: RI.relTol
     int schur = 0;                 // 1: report the explicit Schur operator; FP32-tangent mode: run the CG on it
+    int two_products = 0;          // 1: CGRAD never forms the explicit operator
     std::string log_path;          // per-solve log (memLS_NS.log format); empty: off
 };
 

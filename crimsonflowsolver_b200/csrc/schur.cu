@@ -860,6 +860,7 @@ int cg_schur_launch(crimson_lhs* L, double* R, int nface, const double* coef, do
     if (res && fixed + nvec * vec1 + own > budget) nvec = 3;
     if (!res && fixed + ring + 2 * vec1 > (size_t)160 * 1024) nvec = 0;
     const size_t smem = fixed + nvec * vec1 + (res ? own : ring);
+    (sizeof(M) == 4 ? L->cg_form32 : L->cg_form64) = res ? CRIMSON_CG_SCHUR_RESIDENT : CRIMSON_CG_SCHUR;
     const void* kfn = res ? (const void*)k_cg_schur<M, true> : (const void*)k_cg_schur<M, false>;
     // the same value for every lhs: host threads that launch side by side set it alike
     CR_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));

@@ -146,6 +146,9 @@ class FlowParams:
     # (crimson_memls_ls_set_schur); "fp64" and "mixed" use it where the pattern
     # allows.
     explicit_schur: int = 0
+    # True: the inner CG multiplies by L and Gt G as two products in every
+    # precision, as memLS does (crimson_memls_ls_set_two_products).
+    two_products: bool = False
 
     def outlets(self) -> list:
         """Coupled outlet surfaces in srflist order: the RCRs, the netlists,

@@ -192,6 +192,7 @@ class MemLS:
         N.check(L.crimson_memls_ls_set_precision(ls, PRECISIONS[P.precision], P.max_refine, P.refine_tol),
                 "crimson_memls_ls_set_precision")
         N.check(L.crimson_memls_ls_set_schur(ls, int(P.explicit_schur)), "crimson_memls_ls_set_schur")
+        N.check(L.crimson_memls_ls_set_two_products(ls, int(P.two_products)), "crimson_memls_ls_set_two_products")
         lhs = ctypes.c_void_p()
         self._ctx = ctx   # an lhs made from a context must be freed before it
         if ctx is not None:
@@ -248,6 +249,12 @@ class MemLS:
         N.check(N.lib().crimson_memls_schur_info(self.lhs, ctypes.byref(st), ctypes.byref(nnz), ctypes.byref(npad),
                                                  ctypes.byref(fm)), "crimson_memls_schur_info")
         return st.value, nnz.value, npad.value, fm.value
+
+    def cg_form(self):
+        """(FP64, FP32) kernels of the last inner CG on this lhs: names of _native.CG_FORMS."""
+        f64, f32 = ctypes.c_int(), ctypes.c_int()
+        N.check(N.lib().crimson_memls_cg_form(self.lhs, ctypes.byref(f64), ctypes.byref(f32)), "crimson_memls_cg_form")
+        return N.CG_FORMS[f64.value], N.CG_FORMS[f32.value]
 
     def refine_info(self):
         """(sweeps, relative FP64 defect) of the last mixed-precision solve."""

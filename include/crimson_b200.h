@@ -174,6 +174,10 @@ int crimson_memls_ls_set_precision(crimson_ls* ls, int precision, int max_refine
  * operator's state for this ls, and CRIMSON_MIXED_F32_TANGENT solves, which
  * otherwise multiply by two FP32 products, use it too. */
 int crimson_memls_ls_set_schur(crimson_ls* ls, int explicit_schur);
+/* on = 1: CGRAD multiplies by L and Gt G as two products in every precision
+ * and forms no operator, whatever crimson_memls_ls_set_schur says; 0 (the
+ * default): as described there. */
+int crimson_memls_ls_set_two_products(crimson_ls* ls, int on);
 /* Per-solve log in the format of memLS's memLS_NS.log (LOGFILE,
  * flowsolver/src/memLS.f90:1720-1757), appended to path after every solve
  * with this ls; path = "memLS_NS.log" gives the reference's file.  NULL or ""
@@ -534,7 +538,7 @@ int crimson_memls_kernel_time(crimson_lhs* lhs, int which, int reps, double* ms)
 /* Diagnostics: column layout of the two-product CG kernel on this lhs, for the
  * precisions it has been solved in.  It is decided at the first CGRAD of a
  * precision, also where CGRAD takes the explicit operator and the kernel does
- * not run.
+ * not run (crimson_memls_cg_form says what runs).
  * resident64 / resident32 = 1 when the kernel with FP64 / FP32 matrices keeps
  * every block's column indices in shared memory for the whole launch (16-bit
  * offsets col - row; chosen when the offsets fit and two blocks per SM fit
@@ -542,6 +546,14 @@ int crimson_memls_kernel_time(crimson_lhs* lhs, int which, int reps, double* ms)
  * smem_bytes = shared memory per block of the resident layout (0: offsets
  * exceed 16 bits).  Valid after a solve on the lhs. */
 int crimson_memls_cg_layout(const crimson_lhs* lhs, int* resident64, int* resident32, long long* smem_bytes);
+/* Diagnostics: the kernel that the last CGRAD with FP64 / FP32 matrices on
+ * this lhs ran (CRIMSON_CG_NONE: there was none). */
+#define CRIMSON_CG_NONE 0
+#define CRIMSON_CG_SCHUR 1               /* explicit operator, streamed */
+#define CRIMSON_CG_SCHUR_RESIDENT 2      /* explicit operator in shared memory */
+#define CRIMSON_CG_PRODUCTS 3            /* two products, columns streamed */
+#define CRIMSON_CG_PRODUCTS_RESIDENT 4   /* two products, columns in shared memory */
+int crimson_memls_cg_form(const crimson_lhs* lhs, int* form64, int* form32);
 
 /* Diagnostics of the explicit Schur operator on this lhs: state 1 = built and
  * used by CGRAD, -1 = the pattern does not allow it, 0 = no solve whose ls
