@@ -361,6 +361,28 @@ def cg_schur_iter_bytes(nnz2: int, n: int, nface: int, mbytes: int) -> int:
     return nnz2 * (mbytes + 2) + n * (24 + 48 + 16 + 24 * nface)
 
 
+# What each CG kernel (MemLS.cg_form) does in an iteration, and where its column indices are.
+CG_KERNELS = {
+    "schur": ("k_cg_schur<{}> (one CGRAD iteration on the explicit Schur operator: S R, coupled-face term, updates)",
+              "int16 offsets streamed with the values"),
+    "schur_resident": ("k_cg_schur<{}> (one CGRAD iteration on the explicit Schur operator in shared memory: S R, "
+                       "coupled-face term, updates)", "in shared memory with the values"),
+    "products": ("k_cg_persistent<{}> (one CGRAD iteration: G P, L P - Gt G P, updates)", "read per phase"),
+    "products_resident": ("k_cg_persistent<{}> (one CGRAD iteration: G P, L P - Gt G P, updates)",
+                          "block-resident in shared memory"),
+}
+
+
+def cg_iter_model(form: str, nnz: int, nnz2: int, n: int, nface: int, mbytes: int):
+    """(kernel, columns, algorithmic HBM bytes of one iteration) of the CG kernel that ran."""
+    kernel, columns = CG_KERNELS[form]
+    if form.startswith("schur"):
+        byt = cg_schur_iter_bytes(0 if form == "schur_resident" else nnz2, n, nface, mbytes)
+    else:
+        byt = cg_iter_bytes(nnz, n, mbytes, nface, form == "products_resident")
+    return kernel.format("float" if mbytes == 4 else "double"), columns, byt
+
+
 def run_ours(args):
     import ctypes
 
@@ -471,24 +493,14 @@ def run_ours(args):
         kt[name] = ms.value if rc == 0 else None
     peaks = _peaks()
     nface = len(P.rcr)
-    res64, res32, rbytes = ctypes.c_int(), ctypes.c_int(), ctypes.c_longlong()
-    N.check(L.crimson_memls_cg_layout(F64.memls.lhs, ctypes.byref(res64), None, None), "crimson_memls_cg_layout")
-    N.check(L.crimson_memls_cg_layout(FM.memls.lhs, None, ctypes.byref(res32), ctypes.byref(rbytes)), "crimson_memls_cg_layout")
     s2_nnz, s2_npad, s2_form_ms = FM.memls.schur_info()[1:]
-    if s2_nnz:
-        cg_bytes = cg_schur_iter_bytes(s2_nnz, n, nface, 4)
-        cg_kernel = ("k_cg_schur<float> (one CGRAD iteration on the explicit FP32 Schur operator: S R, "
-                     "coupled-face term, updates)")
-    else:
-        cg_bytes = cg_iter_bytes(nnz, n, 4, nface, bool(res32.value))
-        cg_kernel = "k_cg_persistent<float> (one CGRAD iteration: G P, L P - Gt G P, updates)"
-    s2_nnz64 = F64.memls.schur_info()[1]
-    cg_bytes64 = (cg_schur_iter_bytes(s2_nnz64, n, nface, 8) if s2_nnz64 else
-                  cg_iter_bytes(nnz, n, 8, nface, bool(res64.value)))
+    form32, form64 = FM.memls.cg_form()[1], F64.memls.cg_form()[0]
+    cg_kernel, cg_columns, cg_bytes = cg_iter_model(form32, nnz, s2_nnz, n, nface, 4)
+    _, _, cg_bytes64 = cg_iter_model(form64, nnz, F64.memls.schur_info()[1], n, nface, 8)
     achieved = cg_bytes / (kt["cg_iter_f32"] / 1e3) / 1e9 if kt["cg_iter_f32"] else None
     achieved64 = cg_bytes64 / (kt["cg_iter_f64"] / 1e3) / 1e9 if kt["cg_iter_f64"] else None
-    traffic_f32 = TRAFFIC_PER_ALG_S2 if s2_nnz else TRAFFIC_PER_ALG_F32
-    traffic_f64 = TRAFFIC_PER_ALG_S2_F64 if s2_nnz64 else TRAFFIC_PER_ALG_F64
+    traffic_f32 = TRAFFIC_PER_ALG_S2 if form32.startswith("schur") else TRAFFIC_PER_ALG_F32
+    traffic_f64 = TRAFFIC_PER_ALG_S2_F64 if form64.startswith("schur") else TRAFFIC_PER_ALG_F64
     line = {
         "metric": METRIC, "value": value, "unit": "s/timestep", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": tm_ms / args.steps, "higher_is_better": False, "scaling": "weak",
@@ -514,12 +526,11 @@ def run_ours(args):
                      "bound": "hbm", "achieved": achieved, "peak": peaks[0], "unit": "GB/s",
                      "frac": achieved / peaks[0] if achieved else None,
                      "traffic": traffic_f32 * cg_bytes,
-                     "traffic_source": TRAFFIC_SOURCE_S2 if s2_nnz else TRAFFIC_SOURCE,
+                     "traffic_source": TRAFFIC_SOURCE_S2 if form32.startswith("schur") else TRAFFIC_SOURCE,
                      "algorithmic_bytes_per_iter": cg_bytes, "peak_source": peaks[1],
                      "schur_operator": {"nnz": s2_nnz, "sliced_positions": s2_npad,
                                         "formation_ms": s2_form_ms},
-                     "columns": ("int16 offsets streamed with the FP32 values" if s2_nnz else
-                                 ("block-resident in shared memory" if res32.value else "read per phase")),
+                     "columns": cg_columns,
                      "fp64_kernel": {"achieved": achieved64, "frac": achieved64 / peaks[0] if achieved64 else None,
                                      "algorithmic_bytes_per_iter": cg_bytes64,
                                      "traffic": traffic_f64 * cg_bytes64}},
@@ -768,8 +779,8 @@ def run_scale(args):
     """Large-mesh run, one arm at a time (both at once would not fit beyond
     ~45M tets): mesh from --ncross / --naxial (170 x 290 gives 39.5M tets),
     one warm-up step and one timed step per arm, device memory of each arm,
-    the CG iteration time against its algorithmic bytes (columns streamed
-    when they do not fit in shared memory), mixed vs FP64."""
+    the CG iteration time against the algorithmic bytes of the kernel that
+    ran, mixed vs FP64."""
     import ctypes
 
     import torch
@@ -802,17 +813,14 @@ def run_scale(args):
         free1, _ = torch.cuda.mem_get_info()
         ms = ctypes.c_double()
         N.check(L.crimson_memls_kernel_time(F.memls.lhs, 1 if prec == "fp64" else 4, 1, ctypes.byref(ms)), "kt")
-        r64, r32, rb = ctypes.c_int(), ctypes.c_int(), ctypes.c_longlong()
-        N.check(L.crimson_memls_cg_layout(F.memls.lhs, ctypes.byref(r64), ctypes.byref(r32), ctypes.byref(rb)),
-                "cg_layout")
-        resident = bool(r64.value if prec == "fp64" else r32.value)
-        nnz = F.elm._nnz()
-        byt = cg_iter_bytes(nnz, m.nshg, 8 if prec == "fp64" else 4, len(P.rcr), resident)
+        mbytes = 8 if prec == "fp64" else 4
+        form = F.memls.cg_form()[0 if prec == "fp64" else 1]
+        kernel, columns, byt = cg_iter_model(form, F.elm._nnz(), F.memls.schur_info()[1], m.nshg, len(P.rcr), mbytes)
         y, _ = F.state()
         if y64 is None:
             y64 = y
         out[prec] = {"step_s": e0.elapsed_time(e1) / 1e3, "device_memory_used_gb": (free0 - free1) / 1e9,
-                     "cg_iter_ms": ms.value, "cg_columns_resident": resident,
+                     "cg_iter_ms": ms.value, "cg_kernel": kernel, "cg_columns": columns,
                      "cg_algorithmic_bytes_per_iter": byt, "cg_achieved_gbs": byt / ms.value / 1e6,
                      "cg_frac": byt / ms.value / 1e6 / peaks[0],
                      "iters_per_solve": [(st.ri_itr[i], st.gm_itr[i], st.cg_itr[i]) for i in range(st.nsolves)],
