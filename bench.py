@@ -66,10 +66,11 @@ TRAFFIC_PER_ALG_F32 = 0.765
 TRAFFIC_PER_ALG_F64 = 0.850
 TRAFFIC_SOURCE = "ncu --set full, k_cg_persistent, 2.07M-tet cylinder, 50 iterations/launch, scaled by blocks"
 # The same ratio for the CG on the explicit Schur operator (k_cg_schur), from
-# captures of the same case: FP32 142.7 MB per iteration of 158.0 algorithmic,
-# FP64 236 MB of 249.
-TRAFFIC_PER_ALG_S2 = 0.90
-TRAFFIC_PER_ALG_S2_F64 = 0.95
+# captures on a 2.11M-tet cylinder (23.0M entries of S): FP32 142.6 MB per
+# iteration of 179.5 algorithmic, FP64 243.1 MB of 271.5 (most of the vectors
+# stay in the L2).
+TRAFFIC_PER_ALG_S2 = 0.794
+TRAFFIC_PER_ALG_S2_F64 = 0.896
 TRAFFIC_SOURCE_S2 = "ncu, k_cg_schur, 2.11M-tet cylinder, 50 iterations/launch, scaled by entries"
 
 

@@ -221,7 +221,7 @@ struct crimson_ctx {
     crimson::DBuf<double> rmass;    // (nshg) 1 / lumped mass (geometry only)
     bool rmass_ready = false;       // rmass holds the inverse lumped mass
     crimson::DBuf<double> qrec;     // (nelem, 8) AsIq element records {W, q11,q12,q13,q22,q23,q33, 0}
-    crimson::DBuf<double> erec;     // (nelem, 48) element records of the residual and tangent
+    crimson::DBuf<double> erec;     // (nelem, 52) element records of the residual and tangent
     crimson::DBuf<double> y4, ac4, res4;   // (4, nshg) staging for host-pointer calls
     crimson::DBuf<double> lhsK, lhsP;      // (9, nnz), (4, nnz)
     crimson::DBuf<float> lhs32;            // (16, nnz) FP32 tangent records (mixed precision)

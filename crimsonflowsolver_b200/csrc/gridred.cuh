@@ -7,10 +7,11 @@
 // {value, epoch} and waits until the packets of all blocks carry the epoch,
 // so the values arrive with the barrier itself.  Every block sums the packets
 // in block order: the result is the same bits in every block and on every
-// run.  Measured on 148 blocks of 768 threads: 1.3 us for one value without
-// data (gr_publish / gr_collect), 2.3 us when each block's global writes are
-// ordered before it (fence, 0.6 us, and acquire); cooperative_groups'
-// grid.sync takes 1.2 us and reading and summing the partials after it 1.3.
+// run.  Measured (768 threads per block; one sum, without and with the blocks'
+// global writes ordered before it): 1.2 / 2.0 us on 20 blocks, 1.4 / 2.3 on
+// 74, 2.6 / 3.9 on 148, where every block's polls of all packets meet in the
+// L2.  cooperative_groups' grid.sync takes 1.2 us on any of them, and with the
+// writes before it and the partials read and summed after it 2.2-2.3.
 //
 // Packets of two consecutive epochs live in alternating regions: a block can
 // be at most one epoch ahead of the slowest one, which is still reading the
@@ -100,8 +101,8 @@ __device__ __forceinline__ void gr_acquire() { asm volatile("fence.acq_rel.gpu;"
 // every thread.  Value 0 comes from every block and is the barrier itself;
 // values 1 + 2 f and 2 + 2 f (f < nface) come only from the blocks whose
 // own_faces has bit f -- the others' are zero -- and fpend[32 f + lane] says
-// which these are (as gr_all_blocks).  Measured on 148 blocks: three values
-// from every block take 3.0 us where one takes 1.3.  pk: two regions of kvals
+// which these are (as gr_all_blocks).  Three values from every block take no
+// longer than one (2.5 us on 148 blocks).  pk: two regions of kvals
 // packets per block.  data: the block's global writes before the call are
 // visible to all blocks after it.  Returns whether a thread of the block gave
 // up a wait, in this call or before it (failed).

@@ -18,9 +18,11 @@
 // grid reduction whose last block sums the per-block partials in a fixed
 // order (deterministic).  CGRAD runs as one persistent cooperative kernel per
 // call: on the explicitly formed Schur operator (schur.cu) where the pattern
-// allows, else on the two-product kernel below.  The Krylov control flow (Givens rotations, back substitution, the
-// 2i x 2i Gram system solved by GE) runs on the host in FP64 on scalars
-// copied back per step, as the reference's serial code does.
+// allows, else on the two-product kernel below; GMRES as one per call, with
+// its restarts, Givens rotations and back substitution, or, in the FP32-tangent
+// mode, one per restart cycle.  The 2i x 2i Gram system (GE) and the outer
+// iteration run on the host in FP64 on scalars copied back once per outer
+// iteration.
 //
 // Modified Gram-Schmidt is fused: kernel j subtracts h(j-1) u_{j-1} from w and
 // accumulates <w, u_j> in the same pass.
@@ -2921,7 +2923,10 @@ static int precond_faces(crimson_lhs* L, bool after_scale) {
 // a header "gnNo nTasks nCoupledFaces" when the file is new, then the
 // success code (100 RI + 10 GM + CG), RI / GM / CG iterations, the time
 // split other / GM / CG in percent, the initial norm, the relative final
-// norm, the wall time, Resm, Resc and dB.
+// norm, the wall time, Resm, Resc and dB.  The solve's time is the host's wall
+// clock as in memLS; the shares of GM and CG are the device times of their
+// kernels (the host does not wait for each), for GMRES driven by the host its
+// wall clock.
 static void log_solve(const crimson_lhs* L, const crimson_ls* ls) {
     if (ls->log_path.empty()) return;
     FILE* probe = std::fopen(ls->log_path.c_str(), "r");

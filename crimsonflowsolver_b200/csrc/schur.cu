@@ -32,14 +32,21 @@
 //   * resident: where the block's chunks fit in shared memory (meshes up to
 //     about 300,000 tets in FP64, 500,000 in FP32) they are loaded once per
 //     call and no iteration touches the operator in memory again; bound by
-//     the two barriers (1.3 and 2.3 us) and one gather latency;
+//     the two barriers (1.2 and 2.0 us on 20 blocks, 2.6 and 3.9 on 148) and
+//     one gather latency: 108k tets, 148 blocks, barrier stalls 28.6 per issue
+//     of 38;
 //   * streaming: every warp runs its chunks through a ring of two
 //     shared-memory stages filled by cp.async.bulk, so the stream does not
-//     stop at slice ends, barriers or iteration ends; bound by HBM (the
-//     product phase reads 6.7 TB/s in FP64, 5.8 in FP32).
+//     stop at slice ends, barriers or iteration ends; bound by HBM, the
+//     gathers' latency and the barriers together (2.1M tets: 46 us per FP64
+//     iteration, 5.3 TB/s, DRAM 64% busy; 35 us FP32, 4.1 TB/s, 50%).
 // Per iteration, before (two-product kernel) and now, B200: 4M-tet cylinder
 // 118 / 80 us FP64, 74 / 57 FP32; 452k-tet bifurcation 24.6 / 16 FP32;
 // 108k-tet cylinder 20 / 9.2 FP64; 1152 tets 15 / 5.5 FP64.
+// S is formed in every NSSOLVER call, 2.2 ms on 4M tets: the time that 60 FP64
+// or 130 FP32 iterations gain.  Solves at loose tolerances (0.4 / 0.01 / 0.2)
+// take 111-290 there: whole steps 90 -> 71 ms FP64, 65 -> 58 mixed; 41-111 on
+// 108k tets: 10 -> 5 ms and 8.9 -> 5.2.
 //
 // Iteration.  S P is kept by the recurrence S P = S R + beta S P_prev, so the
 // product gathers only R (8 B per entry) and does not wait for P:

@@ -76,7 +76,9 @@ typedef struct {
 } crimson_params;
 
 /* memLS statistics, field for field memLS_subLsType
- * (flowsolver/src/memLS.f90:159-188). */
+ * (flowsolver/src/memLS.f90:159-188).  callD in seconds: RI's is the host's
+ * wall clock; CG's, and GM's where GMRES is one kernel per call, is the device
+ * time of the kernels. */
 typedef struct {
     double absTol, relTol, iNorm, fNorm, dB, callD;
     int suc, mItr, sD, itr, cM, cN, cD, reserve;
@@ -161,7 +163,9 @@ int crimson_memls_ls_free(crimson_ls* ls);
  * converged solution is unchanged, but with a fixed number of nonlinear
  * iterations per step the iterates follow a slightly different Newton path
  * (on a small cylinder after 2 steps of 3 iterations: 1e-6 velocity, 4e-5
- * pressure relative to the FP64 tangent). */
+ * pressure relative to the FP64 tangent).  It keeps the two-product CG and the
+ * order of its sums, and CRIMSON_MIXED is both faster and closer to FP64 (4M
+ * tets: 0.59 and 0.48 s per step). */
 int crimson_memls_ls_set_precision(crimson_ls* ls, int precision, int max_refine, double refine_tol);
 /* Form of the inner CG's operator (no counterpart in the reference).  CGRAD
  * multiplies by S = L - Gt G.  Where the pattern allows (every |col - row| of
@@ -172,7 +176,9 @@ int crimson_memls_ls_set_precision(crimson_ls* ls, int precision, int max_refine
  * multiplies by L and Gt G as two products, as memLS does.
  * explicit_schur = 1 (default 0): crimson_memls_schur_info reports the
  * operator's state for this ls, and CRIMSON_MIXED_F32_TANGENT solves, which
- * otherwise multiply by two FP32 products, use it too. */
+ * otherwise multiply by two FP32 products, use it too.  It does not select the
+ * form of the other modes: crimson_memls_ls_set_two_products does, and
+ * crimson_memls_cg_form says what ran. */
 int crimson_memls_ls_set_schur(crimson_ls* ls, int explicit_schur);
 /* on = 1: CGRAD multiplies by L and Gt G as two products in every precision
  * and forms no operator, whatever crimson_memls_ls_set_schur says; 0 (the
@@ -262,7 +268,11 @@ int crimson_solflow_device_transposed(crimson_ctx* ctx, crimson_lhs* lhs, crimso
  * d_res (optional) receives res itself.  Unlike the assembled tangent (the
  * reference's approximate Jacobian), this differentiates tauM, tauC, tauBar,
  * uBar and the flux projection as well.  Returns CRIMSON_ERR_UNSUPPORTED when
- * some node has one or two prescribed velocity components. */
+ * some node has one or two prescribed velocity components.  d_y, d_ac
+ * and d_res are 16-byte aligned, d_lambda, d_ybar and d_acbar need 8.  Everything is summed
+ * in a fixed order but the boundary faces' and outlets' terms of d_ybar, which
+ * are added with atomics: those of boundary nodes may differ in the last bits
+ * from call to call. */
 int crimson_elmgmr_vjp(crimson_ctx* ctx, const double* d_y, const double* d_ac, const double* coef1,
                        const double* coef2, const double* d_lambda, double* d_res, double* d_ybar, double* d_acbar,
                        double* mubar, double* coef1bar, double* coef2bar);
