@@ -2246,13 +2246,13 @@ static int cg_resident_bytes(crimson_lhs* L, size_t* bytes) {
     }
     cudaStream_t s = L->stream;
     const int n = L->nNo;
-    CR_CHECK(L->cg_tmp.alloc(1));
-    CR_CUDA(cudaMemsetAsync(L->cg_tmp.p, 0, sizeof(int), s));
-    // (an explicit operator's 2-ring offsets fit 16 bits, so these do)
-    if (L->s2_state != 1)
-        launch(k_max_offset, grid_for(n, 256), 256, 0, s, (const int*)L->rowptr, (const int*)L->col, n, L->cg_tmp.p);
     int maxoff = 0;
-    CR_CUDA(cudaMemcpyAsync(&maxoff, L->cg_tmp.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (L->s2_state != 1) {   // an explicit operator's 2-ring offsets fit 16 bits, so these do
+        CR_CHECK(L->cg_tmp.alloc(1));
+        CR_CUDA(cudaMemsetAsync(L->cg_tmp.p, 0, sizeof(int), s));
+        launch(k_max_offset, grid_for(n, 256), 256, 0, s, (const int*)L->rowptr, (const int*)L->col, n, L->cg_tmp.p);
+        CR_CUDA(cudaMemcpyAsync(&maxoff, L->cg_tmp.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    }
     std::vector<int> sp((size_t)L->nslice + 1);
     CR_CUDA(cudaMemcpyAsync(sp.data(), L->sell_ptr.p, sizeof(int) * sp.size(), cudaMemcpyDeviceToHost, s));
     CR_CUDA(cudaStreamSynchronize(s));
