@@ -18,9 +18,10 @@
 // previous region.  Epochs grow monotonically over the launches that share a
 // packet buffer, so the buffer is cleared once, at its allocation.
 //
-// Every wait is bounded; a block whose wait runs out reports it to its
-// threads, which leave the kernel's loop, and the other blocks follow when
-// their own waits run out.
+// Every wait is bounded.  A block whose wait runs out reports it to its threads
+// and waits for nothing more: they pass the barriers that are left in the
+// kernel's loops and leave them, and the other blocks follow when their own
+// waits run out.
 #pragma once
 
 #include "common.cuh"
@@ -29,7 +30,10 @@ namespace crimson {
 
 constexpr int kGrMaxBlocks = 160;              // blocks of a grid that reduces this way
 constexpr int kGrPolls = kGrMaxBlocks / 32;    // packets per lane and value
-constexpr long long kGrWaitClocks = 1LL << 32;  // SM clocks before a wait gives up (about two seconds)
+#ifndef CRIMSON_GR_WAIT_CLOCKS
+#define CRIMSON_GR_WAIT_CLOCKS (1LL << 32)
+#endif
+constexpr long long kGrWaitClocks = CRIMSON_GR_WAIT_CLOCKS;  // SM clocks before a wait gives up (about two seconds)
 
 __device__ __forceinline__ void gr_publish(ulonglong2* p, double v, unsigned long long epoch) {
     asm volatile(
@@ -59,10 +63,10 @@ __device__ __forceinline__ unsigned gr_all_blocks() {
 
 // Sum over a warp of the packets of the blocks in pend (per lane, as
 // gr_all_blocks), every lane receiving it; waits until all of them carry the
-// epoch.
-__device__ __forceinline__ double gr_collect(const ulonglong2* pk, unsigned pend, unsigned long long epoch, bool* fail) {
+// epoch or the limit since t0 (0: the first poll) has passed.
+__device__ __forceinline__ double gr_collect(const ulonglong2* pk, unsigned pend, unsigned long long epoch, bool* fail,
+                                             long long t0) {
     const int lane = threadIdx.x & 31;
-    long long t0 = 0;
     double v[kGrPolls];
 #pragma unroll
     for (int j = 0; j < kGrPolls; ++j) v[j] = 0.0;
@@ -112,6 +116,8 @@ static __device__ __noinline__ bool grid_reduce(ulonglong2* pk, int kvals, const
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, nv = 1 + 2 * nface;
     pk += (size_t)(ep & 1) * kvals * gridDim.x;
     bool fail = failed;
+    // after a wait that ran out: one poll
+    const long long t0 = failed ? -(1LL << 62) : 0;
     __syncthreads();
     for (int k = wid; k < nv; k += nw)
         if (k == 0 || ((own_faces >> ((k - 1) / 2)) & 1)) {
@@ -123,7 +129,7 @@ static __device__ __noinline__ bool grid_reduce(ulonglong2* pk, int kvals, const
         }
     for (int k = wid; k < nv; k += nw) {
         const unsigned pend = k == 0 ? gr_all_blocks() : fpend[32 * ((k - 1) / 2) + lane];
-        const double v = gr_collect(pk + (size_t)k * gridDim.x, pend, ep, &fail);
+        const double v = gr_collect(pk + (size_t)k * gridDim.x, pend, ep, &fail, t0);
         if (data) gr_acquire();
         if (lane == 0) tot[k] = v;
     }

@@ -502,9 +502,11 @@ __device__ __forceinline__ bool s2_try_wait(unsigned bar, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait for a stage's copy.
-__device__ __forceinline__ bool s2_wait(unsigned bar, unsigned parity) {
+// Bounded wait for a stage's copy; without patience (a copy has timed out
+// before) one try.
+__device__ __forceinline__ bool s2_wait(unsigned bar, unsigned parity, bool patience) {
     if (s2_try_wait(bar, parity)) return true;
+    if (!patience) return false;
     const long long t0 = clock64();
     while (clock64() - t0 < kGrWaitClocks)
         if (s2_try_wait(bar, parity)) return true;
@@ -703,7 +705,7 @@ __global__ void __launch_bounds__(32 * kS2CgWarps, 1) k_cg_schur(const __grid_co
                 d = e.y;
                 p = (e.x - (unsigned)c0) * COL;
             } else {
-                if (!s2_wait(s2_smem_u32(bars + gs), parity)) ok = false;
+                if (!s2_wait(s2_smem_u32(bars + gs), parity, ok)) ok = false;
                 d = sdesc[gs];
                 p = ring + gs * CB;
             }
@@ -818,9 +820,9 @@ __global__ void __launch_bounds__(32 * kS2CgWarps, 1) k_cg_schur(const __grid_co
         }
         __syncthreads();
     }
-    // the copies still under way, one per stage
-    for (int q = 0; q < nload && ok; ++q) {
-        ok = s2_wait(s2_smem_u32(bars + gs), parity);
+    // the copies still under way, one per stage (also after a wait that ran out)
+    for (int q = 0; q < nload; ++q) {
+        s2_wait(s2_smem_u32(bars + gs), parity, true);
         if (++gs == nload) {
             gs = 0;
             parity ^= 1u;
