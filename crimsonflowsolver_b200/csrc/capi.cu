@@ -898,7 +898,7 @@ int crimson_spmv4_prepare(crimson_ctx* c, int precision, const void* d_val) {
 
 int crimson_spmv4_apply(crimson_ctx* c, const void* d_u, void* d_ku) {
     if (!c || !d_u || !d_ku) return CRIMSON_ERR_ARG;
-    if (!c->s4_ptr.p) return CRIMSON_ERR_STATE;
+    if (c->s4_npad == 0) return CRIMSON_ERR_STATE;
     return spmv4_apply(c, d_u, d_ku);
 }
 

@@ -1838,9 +1838,9 @@ static int gm_face_map(crimson_lhs* L, int* ok) {
         return CRIMSON_OK;
     }
     L->gm_faces = cur;
-    L->gm_map_ok = 0;
+    L->gm_map_ok = (int)cur.size() > kMaxCoupled ? 0 : -1;   // -1 until all of it is built
     *ok = 0;
-    if ((int)cur.size() > kMaxCoupled) return CRIMSON_OK;
+    if (L->gm_map_ok == 0) return CRIMSON_OK;
     cudaStream_t s = L->stream;
     const int n = L->nNo;
     std::vector<int> node_of, fface;
@@ -1850,7 +1850,10 @@ static int gm_face_map(crimson_lhs* L, int* ok) {
         CR_CUDA(cudaMemcpyAsync(g.data(), f.glob.p, sizeof(int) * g.size(), cudaMemcpyDeviceToHost, s));
         CR_CUDA(cudaStreamSynchronize(s));
         for (int a = 0; a < f.nNo; ++a) {
-            if (g[a] < 0 || g[a] >= n) return CRIMSON_OK;
+            if (g[a] < 0 || g[a] >= n) {
+                L->gm_map_ok = 0;
+                return CRIMSON_OK;
+            }
             node_of.push_back(g[a]);
             fface.push_back(q);
         }
@@ -2590,7 +2593,8 @@ static int sell_mats(crimson_lhs* L, float** K, float** G, float4** GL, bool two
 
 // Sliced pattern of a CSR pattern (rowptr, col on the device): slice widths
 // from the row lengths (host), columns (device).  The column array carries
-// kSlice * kSellUnroll zero entries past npad.
+// kSlice * kSellUnroll zero entries past npad.  *npad_out is set last: 0 means
+// not built.
 int sell_build(const int* rowptr, const int* col, int n, cudaStream_t s, DBuf<int>& sell_ptr, DBuf<int>& sell_col,
                long long* npad_out, int* nslice_out) {
     std::vector<int> rp((size_t)n + 1);
@@ -2621,7 +2625,7 @@ int sell_build(const int* rowptr, const int* col, int n, cudaStream_t s, DBuf<in
 }
 
 static int sell_pattern(crimson_lhs* L) {
-    if (L->sell_ptr.p) return CRIMSON_OK;
+    if (L->npad > 0) return CRIMSON_OK;
     CR_CHECK(sell_build(L->rowptr, L->col, L->nNo, L->stream, L->sell_ptr, L->sell_col, &L->npad, &L->nslice));
     return CRIMSON_OK;
 }
@@ -2873,16 +2877,14 @@ static int lhs_work_alloc(crimson_lhs* L, const crimson_ls* ls) {
     CR_CHECK(L->basis.alloc(3 * (size_t)nNo * (sD + 1)));
     CR_CHECK(L->w3.alloc(3 * (size_t)nNo));
     CR_CHECK(sell_pattern(L));
-    if (!L->scal.p) {
-        CR_CHECK(L->scal.alloc(kScalTotal));
-        CR_CHECK(L->red.init());
-        CR_CUDA(cudaMallocHost(&L->hscal, sizeof(double) * kScalTotal));
-        CR_CUDA(cudaEventCreate(&L->ev0));
-        CR_CUDA(cudaEventCreate(&L->ev1));
-        for (cudaEvent_t& e : L->ev_gm) CR_CUDA(cudaEventCreate(&e));
-        CR_CUDA(cudaEventCreate(&L->s2_ev0));
-        CR_CUDA(cudaEventCreate(&L->s2_ev1));
-    }
+    // each on its own: a call that failed part-way is made up for by the next
+    CR_CHECK(L->scal.alloc(kScalTotal));
+    if (!L->red.ticket.p) CR_CHECK(L->red.init());
+    if (!L->hscal) CR_CUDA(cudaMallocHost(&L->hscal, sizeof(double) * kScalTotal));
+    cudaEvent_t* const ev[] = {&L->ev0,       &L->ev1,       &L->ev_gm[0],  &L->ev_gm[1],
+                               &L->ev_gm[2],  &L->ev_gm[3],  &L->s2_ev0,    &L->s2_ev1};
+    for (cudaEvent_t* e : ev)
+        if (!*e) CR_CUDA(cudaEventCreate(e));
     return CRIMSON_OK;
 }
 

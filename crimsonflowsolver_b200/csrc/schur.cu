@@ -198,9 +198,9 @@ __global__ void __launch_bounds__(256) k_s2_offsets(const int* __restrict__ rowp
 }
 
 // Per lhs, once: row lengths, slices, chunks, the blocks' slice ranges.
-// s2_state 1: usable, -1: the pattern does not qualify.
-int schur_pattern(crimson_lhs* L) {
-    if (L->s2_state != 0) return CRIMSON_OK;
+// s2_state 1: usable, -1: the pattern does not qualify (0: not built; a call
+// that fails leaves that).
+static int s2_build(crimson_lhs* L) {
     cudaStream_t s = L->stream;
     const int n = L->nNo;
     L->s2_state = -1;   // unusable unless every step below succeeds
@@ -305,6 +305,12 @@ int schur_pattern(crimson_lhs* L) {
     L->s2_nslice = ns;
     L->s2_state = 1;
     return CRIMSON_OK;
+}
+int schur_pattern(crimson_lhs* L) {
+    if (L->s2_state != 0) return CRIMSON_OK;
+    const int rc = s2_build(L);
+    if (rc != CRIMSON_OK) L->s2_state = 0;
+    return rc;
 }
 
 // The operator's buffer in storage type M with its column offsets, on the

@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(256) k_spmv4(const int* __restrict__ sp, const
 
 int spmv4_prepare(crimson_ctx* c, int precision, const void* d_val) {
     cudaStream_t s = c->stream;
-    if (!c->s4_ptr.p) CR_CHECK(sell_build(c->rowptr.p, c->col.p, c->nshg, s, c->s4_ptr, c->s4_col, &c->s4_npad,
-                                          &c->s4_nslice));
+    if (c->s4_npad == 0) CR_CHECK(sell_build(c->rowptr.p, c->col.p, c->nshg, s, c->s4_ptr, c->s4_col, &c->s4_npad,
+                                             &c->s4_nslice));
     const size_t np = (size_t)c->s4_npad + (size_t)kS4Slice * 8;
     c->s4_prec = precision;
     if (precision == CRIMSON_FP64) {
